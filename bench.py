@@ -345,8 +345,8 @@ def rk3_legs(dev, flush, steps_col=COLUMN512["steps"], steps_batch=1000, warmup=
         "steps_per_s": steps_batch / (ms / 1e3), "ms_per_step": ms / steps_batch, "steps": steps_batch,
         "column_steps_per_s": BATCH_NCOL * steps_batch / (ms / 1e3), "cell_updates_per_s": cells * steps_batch / (ms / 1e3),
         "threads": th, "tri_cap": cap, "autotune_ms_per_step": trial,
-        "autotune": "lica_boiling1d_b200.autotune: CTA width 64/128/256 x Thomas arrays in shared memory or "
-                    "scratch, timed on a copy of the batch, cached per GPU",
+        "autotune": "lica_boiling1d_b200.autotune: CTA width 32/64/128/256, timed on a copy of the batch, "
+                    "cached per GPU",
         "gpu_launches": launches,
         "ranks": world, "sharding": "contiguous column blocks balanced by cells, strong scaling of the fixed batch",
         "gathered_columns": len(hist)}

@@ -399,9 +399,9 @@ int lica_gpu_column_batch_destroy(lica_col_batch* batch);
 int lica_gpu_column_batch_layout(const lica_col_batch* batch, int64_t* offsets, int64_t* totals);
 int lica_gpu_column_batch_steps_device(const lica_col_batch* batch, const lica_col_state* st, int32_t nsteps,
                                        int32_t threads, void* scratch, int32_t* status, void* stream);
-/* The same with a limit on the column length whose Thomas arrays live in shared memory
- * (tri_cap < 0: as large as the CTAs per SM allow, the default; 0: all in scratch; the arithmetic
- * and results are the same either way) -- the launch autotuner's second axis. */
+/* The same with tri_cap, once a limit on the column length whose Thomas arrays live in shared
+ * memory: accepted and without effect, since the solves now stage every column's rows through
+ * shared memory of a fixed size. */
 int lica_gpu_column_batch_steps_ex_device(const lica_col_batch* batch, const lica_col_state* st, int32_t nsteps,
                                           int32_t threads, int32_t tri_cap, void* scratch, int32_t* status,
                                           void* stream);

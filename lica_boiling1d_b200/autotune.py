@@ -1,15 +1,11 @@
 """Launch-shape autotuner of the batched column step (lica_gpu_column_batch_steps_ex_device).
 
-The step kernel runs one CTA per column, persistent over all the steps of a launch.  A
-launch shape has two axes:
-  * the CTA width -- 32, 64, 128 or 256 threads -- which also fixes how many columns share an
-    SM (the 32- and 64-thread forms are bounded for 8 and 5 CTAs per SM, the wider ones run one
-    or two; a one-warp CTA runs TEMP_EXTP's two phases one after the other);
-  * the shared-memory cap of the Thomas arrays: as long a column as the CTAs per SM leave room
-    for (the default), or none (every column's arrays in the L2-resident scratch).  Results
-    are identical either way; the speed is not.
-Which shape is fastest depends on the batch: many short columns favour narrow CTAs and more
-columns per SM, a few long ones wide CTAs that finish each column sooner.
+The step kernel runs one CTA per column, persistent over all the steps of a launch.  The
+launch shape is the CTA width -- 32, 64, 128 or 256 threads -- which also fixes how many columns
+share an SM (the 32- and 64-thread forms are bounded for 8 and 5 CTAs per SM, the wider ones run one
+or two; a one-warp CTA runs TEMP_EXTP's two phases one after the other).  Results are identical;
+the speed is not: many short columns favour narrow CTAs and more columns per SM, a few long
+ones wide CTAs that finish each column sooner.
 
 ``tune(batch)`` times one warm-up step and ``trial_steps`` steps of each shape on a copy of
 the batch's device state (the batch itself does not advance), keeps the fastest, and
@@ -21,8 +17,9 @@ import json
 import os
 import threading
 
-# (threads, tri_cap): tri_cap -1 = the largest the CTAs per SM allow, 0 = no shared arrays
-SHAPES = ((32, -1), (64, -1), (128, -1), (256, -1), (32, 0), (64, 0), (128, 0), (256, 0))
+# (threads, tri_cap): tri_cap has no effect any more; cache entries of the shapes that had one
+# (tri_cap 0) are still read
+SHAPES = ((32, -1), (64, -1), (128, -1), (256, -1))
 
 
 def _name(shape):
@@ -35,7 +32,9 @@ def _shape(entry):
         sh = (int(entry["threads"]), int(entry.get("tri_cap", -1)))
     except (KeyError, TypeError, ValueError):
         return None
-    return sh if sh in SHAPES else None
+    return sh if sh in SHAPES or (sh[0], -1 - sh[1]) in SHAPES else None
+
+
 _lock = threading.Lock()
 _memo = {}
 

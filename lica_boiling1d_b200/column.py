@@ -314,9 +314,9 @@ class ColumnBatch:
     def steps(self, nsteps, threads=0, stream=None, scratch=None, tri_cap=-1):
         """nsteps time steps of every column (device state).  threads: the CTA width (64,
         128 or 256), or 0 for the autotuner's launch shape for this batch on this GPU (timed
-        once on a copy of the state, then cached; see autotune.py); tri_cap: the longest
-        column whose Thomas arrays live in shared memory (-1: as the CTAs per SM allow, 0:
-        none).  Returns the per-column status."""
+        once on a copy of the state, then cached; see autotune.py); tri_cap: accepted and
+        without effect (the solves stage every column through shared memory of a fixed size).
+        Returns the per-column status."""
         import torch
         if threads == 0:
             from . import autotune

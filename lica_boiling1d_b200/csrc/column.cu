@@ -7,7 +7,8 @@
 // Parallel structure: one CTA per column; the CTA loops over the time steps without
 // returning to the host.  Per-cell work is spread over the CTA's threads with a barrier
 // between phases; the three tridiagonal solves per substep (LHSPS, LHSW, POISSON) run as
-// the Thomas algorithm on one thread, in the reference's order; the band work (TEMP_GRAD's
+// the Thomas algorithm on one warp, in the reference's order of operations (solve_line,
+// solve_pressure); the band work (TEMP_GRAD's
 // interface pieces, TEMP_EXTP's narrow extension region, TRANSPORT) runs on warp 0 with the
 // band window of lvs_device.cuh in shared memory.  Columns of a batch are independent.
 //
@@ -19,6 +20,7 @@
 //
 // Every floating-point expression keeps the reference's operation order; with the
 // library's -fmad=false the results agree bit for bit with the CPU restatement.
+#include "fp64_rn.cuh"
 #include "lvs_device.cuh"
 
 #include <algorithm>
@@ -49,7 +51,7 @@ __constant__ double c_ro[4] = {0.0, 0.0, -17.0 / 60.0, -5.0 / 12.0};
 // scratch array indices (each n+2 doubles)
 enum {
     S_DFZ, S_VFZ, S_PSIZ, S_DFC, S_PSIC, S_DENFZ, S_DENFZI, S_DENFC, S_RHS1, S_RK3ZO, S_RHSPS, S_DIVG,
-    S_AK, S_BK, S_CK, S_GK, S_GAM, S_VZD, S_VZV, S_VCD, S_TEMP0, S_TEMP1, S_NPHI, S_PSIH, S_PSITMP, S_SPARE0,
+    S_AK, S_BK, S_CK, S_GK, S_GAM, S_VZD, S_VZV, S_VCD, S_TEMP0, S_TEMP1, S_NPHI, S_PSIH, S_PSITMP, S_SOL,
     S_SPARE1, S_SPARE2, S_SPARE3, S_SPARE4
 };
 
@@ -75,8 +77,6 @@ struct Args {
     long long* prof;   // optional per-phase cycle totals (PH_COUNT per column) or null
     double* hist;      // optional interface history (HIST_REC doubles per column and step) or null
     int hist_cap;      // steps of one launch the history holds per column
-    int tri_smem;      // 1: the tridiagonal arrays of columns with n <= tri_cap live in dynamic shared memory
-    int tri_cap;       // longest column whose arrays fit the dynamic shared memory (longer ones use scratch)
     int has_geo;       // 1: every column is the stretched column geo describes (device arrays)
     col::ColGeoDev geo;
 };
@@ -142,13 +142,33 @@ struct XPhase {
     double tm[XR], dt[XR], dtrk[XR], to[XR], trk[XR], nw[XR];
 };
 
+// Row panels of the pressure line: two in flight, the rows of one filled and checked by the
+// other warps while warp 0 walks the other's chain.
+constexpr int PANEL = 64;
+struct Panel {
+    double a[PANEL], b[PANEL], c[PANEL], r[PANEL], y[PANEL];
+    double g[PANEL + 1], u[PANEL + 1];   // g[i], u[i]: the state row i starts from
+};
+
+// Segments of the implicit diffusion lines: 32 pieces of at most 17 rows.
+constexpr int PIECE = 17, SEG = 512, SEGP = 32 * PIECE;
+
 struct Shared {
-    lvs::Win win;
+    // the band work and the tridiagonal solves alternate and keep nothing here between them
+    union {
+        struct {
+            lvs::Win win;
+            // flow cells xk0 .. xk0+XR-1 around the band (xk0 = the band window's flow
+            // origin): NPHI, PSIH and PSI_CN of TEMP_GRAD, and the two phases' extension arrays
+            double x_nphi[XR], x_psih[XR], x_pcn[XR];
+            XPhase xp[2];
+        };
+        struct {
+            double sa[SEGP], sb[SEGP], sc[SEGP], sr[SEGP], sg[SEGP], su[SEGP];
+        };
+        Panel panel[2];
+    };
     double red[32];
-    // flow cells xk0 .. xk0+XR-1 around the band (xk0 = the band window's flow origin):
-    // NPHI, PSIH and PSI_CN of TEMP_GRAD, and the two phases' extension arrays
-    double x_nphi[XR], x_psih[XR], x_pcn[XR];
-    XPhase xp[2];
     int ibuf[8];
     double dbuf[8];
 };
@@ -174,59 +194,367 @@ __device__ __forceinline__ double block_min(double v, Shared& sh) {
     return r;
 }
 
+#define FOR_K(lo, hi) for (int k = (lo) + (int)threadIdx.x; k <= (hi); k += (int)blockDim.x)
+
 // Thomas algorithm of TRDIAG3 (1d.f:3783-3811) on one line, unknowns l1..l2; r becomes the
-// solution.  One thread.
-// The coefficients are read in blocks of PF ahead of the dependent recurrence, so the
-// memory latency overlaps instead of adding to every step of the chain.
-constexpr int PF = 4;
-__device__ void thomas(const double* a, const double* b, const double* c, double* r, double* gam, int l1, int l2) {
+// solution.  One thread; the forms below fall back to it where a pivot is extreme.
+__device__ __noinline__ void thomas(const double* a, const double* b, const double* c, double* r, double* gam, int l1,
+                                    int l2) {
     double bet = 1.0 / b[l1];
     double u = r[l1] * bet;
     r[l1] = u;
-    double cprev = c[l1];
-    for (int j0 = l1 + 1; j0 <= l2; j0 += PF) {
-        double A[PF], B[PF], Cc[PF], R[PF];
-#pragma unroll
-        for (int q = 0; q < PF; ++q) {
-            const int j = min(j0 + q, l2);
-            A[q] = a[j];
-            B[q] = b[j];
-            Cc[q] = c[j];
-            R[q] = r[j];
-        }
-#pragma unroll
-        for (int q = 0; q < PF; ++q) {
-            const int j = j0 + q;
-            if (j <= l2) {
-                const double gm = cprev * bet;
-                gam[j] = gm;
-                bet = 1.0 / (B[q] - A[q] * gm);
-                u = (R[q] - A[q] * u) * bet;
-                r[j] = u;
-                cprev = Cc[q];
+    for (int j = l1 + 1; j <= l2; ++j) {
+        gam[j] = c[j - 1] * bet;
+        bet = 1.0 / (b[j] - a[j] * gam[j]);
+        u = (r[j] - a[j] * u) * bet;
+        r[j] = u;
+    }
+    for (int j = l2 - 1; j >= l1; --j) {
+        u = r[j] - gam[j + 1] * u;
+        r[j] = u;
+    }
+}
+
+__device__ __forceinline__ bool same_bits(double x, double y) {
+    return __double_as_longlong(x) == __double_as_longlong(y);
+}
+
+// Forward elimination of a segment of cnt rows (sh.sa .. sr) on one warp, each row's
+// operations those of thomas() and in its order; g, u: the state the first row starts from on
+// entry, the state after the last row on return (all lanes).  The segment is cut into 32
+// pieces, a lane each.  Every lane runs its piece from an approximate starting state, then
+// again from the state the piece below it left, until no starting state changes: a piece is a
+// function of its starting state alone, so what unchanged states leave is what the serial
+// algorithm leaves, bit for bit (piece k starts right after k rounds at the latest).  Returns
+// whether every pivot was ordinary.
+__device__ bool pieces_forward(Shared& sh, int cnt, double& g0, double& u0) {
+    const int lane = threadIdx.x & 31;
+    const int m = ((cnt + 31) / 32) | 1;   // odd: the lanes' rows lie in different banks
+    const int s0 = lane * m, s1 = min(s0 + m, cnt);
+    const bool own = s0 < cnt;
+    const int last = (cnt - 1) / m;
+    bool ok = true;
+    double g = g0, u = u0;
+    if (own && lane > 0) {
+        const double y = rn::recip(sh.sb[s0 - 1]);
+        g = sh.sc[s0 - 1] * y;
+        u = sh.sr[s0 - 1] * y;
+    }
+    double ge = g, ue = u;
+    for (int round = 0; round < 32; ++round) {
+        ge = g;
+        ue = u;
+        if (own) {
+            double A = sh.sa[s0], B = sh.sb[s0], C = sh.sc[s0], R = sh.sr[s0];
+            for (int j = s0; j < s1; ++j) {
+                const int jn = min(j + 1, s1 - 1);
+                const double An = sh.sa[jn], Bn = sh.sb[jn], Cn = sh.sc[jn], Rn = sh.sr[jn];
+                sh.sg[j] = ge;
+                const double d = B - A * ge;
+                const double y = rn::recip(d);
+                ok = ok && rn::ordinary(d);
+                ue = (R - A * ue) * y;
+                sh.su[j] = ue;
+                ge = C * y;
+                A = An;
+                B = Bn;
+                C = Cn;
+                R = Rn;
             }
+        }
+        double gn = __shfl_up_sync(0xffffffffu, ge, 1), un = __shfl_up_sync(0xffffffffu, ue, 1);
+        if (lane == 0) {
+            gn = g0;
+            un = u0;
+        }
+        const bool moved = own && !(same_bits(gn, g) && same_bits(un, u));
+        g = gn;
+        u = un;
+        if (!__any_sync(0xffffffffu, moved)) break;
+    }
+    g0 = __shfl_sync(0xffffffffu, ge, last);
+    u0 = __shfl_sync(0xffffffffu, ue, last);
+    __syncwarp();
+    return __all_sync(0xffffffffu, ok);
+}
+
+// Back substitution of a segment from sg[0..cnt] (GAM, the row above the segment's included;
+// 0 above the line's last row) and su (the forward results): sr[i] = the solution; x0: the
+// solution above the last row on entry, of the first row on return.
+__device__ void pieces_back(Shared& sh, int cnt, double& x0) {
+    const int lane = threadIdx.x & 31;
+    const int m = ((cnt + 31) / 32) | 1;
+    const int s0 = lane * m, s1 = min(s0 + m, cnt);
+    const bool own = s0 < cnt;
+    const int last = (cnt - 1) / m;
+    double x = (lane == last) ? x0 : (own ? sh.su[s1] : 0.0);
+    double xe = x;
+    for (int round = 0; round < 32; ++round) {
+        xe = x;
+        if (own) {
+            double G = sh.sg[s1], S = sh.su[s1 - 1];
+            for (int j = s1 - 1; j >= s0; --j) {
+                const int jn = max(j - 1, s0);
+                const double Gn = sh.sg[jn + 1], Sn = sh.su[jn];
+                xe = S - G * xe;
+                sh.sr[j] = xe;
+                G = Gn;
+                S = Sn;
+            }
+        }
+        double xn = __shfl_down_sync(0xffffffffu, xe, 1);
+        if (lane >= last) xn = x0;
+        const bool moved = own && !same_bits(xn, x);
+        x = xn;
+        if (!__any_sync(0xffffffffu, moved)) break;
+    }
+    x0 = __shfl_sync(0xffffffffu, xe, 0);
+    __syncwarp();
+}
+
+// The tridiagonal line of rows l1..l2: row(k, a, b, c, r) gives row k's coefficients and
+// apply(k, x) takes its solution; all threads of the CTA.  For the implicit diffusion lines
+// (LHSPS, LHSW), which are diagonally dominant: a wrong starting state of a piece is forgotten
+// within some rows, so that a few rounds over n/32 rows take the place of a chain of n rows,
+// each a reciprocal and five operations.  512 rows, a 256-thread CTA, coefficients and update
+// included: 122 k cycles with one thread's chain, 12 k so.  Columns longer than SEG go
+// segment by segment, GAM and the forward results kept in scratch meanwhile (the segments take
+// no more shared memory than the band work, so the length of a column does not change how many
+// CTAs an SM holds).
+template <typename Row, typename Apply>
+__device__ __forceinline__ void solve_line(Col& c, Shared& sh, int l1, int l2, Row row, Apply apply) {
+    const int tid = threadIdx.x, nt = blockDim.x;
+    const int nrow = l2 - l1 + 1;
+    const int nseg = (nrow + SEG - 1) / SEG, len = (nrow + nseg - 1) / nseg;
+    double *gam = c.a[S_GAM], *sol = c.a[S_SOL];
+    double g = 0.0, u = 0.0;
+    bool ok = true;
+    for (int q = 0; q < nseg; ++q) {
+        const int k0 = l1 + q * len, cnt = min(len, l2 + 1 - k0);
+        for (int i = tid; i < cnt; i += nt) row(k0 + i, sh.sa[i], sh.sb[i], sh.sc[i], sh.sr[i]);
+        __syncthreads();
+        if (tid < 32) ok = pieces_forward(sh, cnt, g, u) && ok;
+        __syncthreads();
+        if (nseg > 1) {
+            for (int i = tid; i < cnt; i += nt) {
+                gam[k0 + i] = sh.sg[i];
+                sol[k0 + i] = sh.su[i];
+            }
+            __syncthreads();
         }
     }
-    for (int j0 = l2 - 1; j0 >= l1; j0 -= PF) {
-        double G[PF], R[PF];
+    if (__syncthreads_or(!ok)) {   // a pivot out of the ordinary range: the plain chain
+        double *ak = c.a[S_AK], *bk = c.a[S_BK], *ck = c.a[S_CK], *gk = c.a[S_GK];
+        FOR_K(l1, l2) row(k, ak[k], bk[k], ck[k], gk[k]);
+        __syncthreads();
+        if (tid == 0) thomas(ak, bk, ck, gk, gam, l1, l2);
+        __syncthreads();
+        FOR_K(l1, l2) apply(k, gk[k]);
+        __syncthreads();
+        return;
+    }
+    double x = 0.0;
+    for (int q = nseg - 1; q >= 0; --q) {
+        const int k0 = l1 + q * len, cnt = min(len, l2 + 1 - k0);
+        if (nseg > 1)
+            for (int i = tid; i < cnt; i += nt) {
+                sh.sg[i] = gam[k0 + i];
+                sh.su[i] = sol[k0 + i];
+            }
+        if (tid == 0) sh.sg[cnt] = (q == nseg - 1) ? 0.0 : gam[k0 + cnt];
+        __syncthreads();
+        if (tid < 32) pieces_back(sh, cnt, x);
+        __syncthreads();
+        for (int i = tid; i < cnt; i += nt) apply(k0 + i, sh.sr[i]);
+        __syncthreads();
+    }
+}
+
+// One panel of the pressure line's forward elimination, every lane alike.  The reciprocal of
+// row i's pivot comes from the seed y[i] by one Newton step; check_panel tells whether it is
+// the correctly rounded one.
+template <int ROWS>
+__device__ __forceinline__ void panel_rows(const Panel& P, int j, double (&A)[ROWS], double (&B)[ROWS],
+                                           double (&C)[ROWS], double (&R)[ROWS], double (&Y)[ROWS]) {
 #pragma unroll
-        for (int q = 0; q < PF; ++q) {
-            const int j = max(j0 - q, l1);
-            G[q] = gam[j + 1];
-            R[q] = r[j];
+    for (int q = 0; q < ROWS; ++q) {
+        A[q] = P.a[j + q];
+        B[q] = P.b[j + q];
+        C[q] = P.c[j + q];
+        R[q] = P.r[j + q];
+        Y[q] = P.y[j + q];
+    }
+}
+template <int ROWS>
+__device__ __forceinline__ void panel_chain(Panel& P, int j, const double (&A)[ROWS], const double (&B)[ROWS],
+                                            const double (&C)[ROWS], const double (&R)[ROWS], const double (&Y)[ROWS],
+                                            double& g, double& u, bool first) {
+#pragma unroll
+    for (int q = 0; q < ROWS; ++q) {
+        const double d = B[q] - A[q] * g;
+        const double y = __fma_rn(Y[q], __fma_rn(-d, Y[q], 1.0), Y[q]);
+        u = (R[q] - A[q] * u) * y;
+        g = C[q] * y;
+        if (first) {
+            P.g[j + q + 1] = g;
+            P.u[j + q + 1] = u;
+        }
+    }
+}
+__device__ void panel_forward(Panel& P, int rows, double& g, double& u) {
+    const bool first = (threadIdx.x & 31) == 0;
+    if (first) {
+        P.g[0] = g;
+        P.u[0] = u;
+    }
+    double A0[4], B0[4], C0[4], R0[4], Y0[4], A1[4], B1[4], C1[4], R1[4], Y1[4];
+    panel_rows(P, 0, A0, B0, C0, R0, Y0);
+#pragma unroll 1
+    for (int j = 0; j < rows; j += 8) {
+        panel_rows(P, j + 4, A1, B1, C1, R1, Y1);
+        panel_chain(P, j, A0, B0, C0, R0, Y0, g, u, first);
+        panel_rows(P, min(j + 8, PANEL - 4), A0, B0, C0, R0, Y0);
+        panel_chain(P, j + 4, A1, B1, C1, R1, Y1, g, u, first);
+    }
+}
+
+// Back substitution of a panel of rows in falling order, every lane alike: a = the GAM of the
+// row above, b = the forward result; c = the solution.
+__device__ void panel_back(Panel& P, int rows, double& x) {
+    const bool first = (threadIdx.x & 31) == 0;
+    double G0[4], S0[4], G1[4], S1[4];
+#pragma unroll
+    for (int q = 0; q < 4; ++q) {
+        G0[q] = P.a[q];
+        S0[q] = P.b[q];
+    }
+#pragma unroll 1
+    for (int j = 0; j < rows; j += 8) {
+#pragma unroll
+        for (int q = 0; q < 4; ++q) {
+            G1[q] = P.a[j + 4 + q];
+            S1[q] = P.b[j + 4 + q];
         }
 #pragma unroll
-        for (int q = 0; q < PF; ++q) {
-            const int j = j0 - q;
-            if (j >= l1) {
-                u = R[q] - G[q] * u;
-                r[j] = u;
-            }
+        for (int q = 0; q < 4; ++q) {
+            x = S0[q] - G0[q] * x;
+            if (first) P.c[j + q] = x;
+        }
+        const int jn = min(j + 8, PANEL - 4);
+#pragma unroll
+        for (int q = 0; q < 4; ++q) {
+            G0[q] = P.a[jn + q];
+            S0[q] = P.b[jn + q];
+        }
+#pragma unroll
+        for (int q = 0; q < 4; ++q) {
+            x = S1[q] - G1[q] * x;
+            if (first) P.c[j + 4 + q] = x;
         }
     }
 }
 
-#define FOR_K(lo, hi) for (int k = (lo) + (int)threadIdx.x; k <= (hi); k += (int)blockDim.x)
+// The pressure line of rows 1..n (POISSON's Thomas solve): row(k, a, b, c, r) gives row k's
+// coefficients, the solution goes to p[1..n].  A Laplacian forgets nothing, so pieces would not
+// help: the rows stay one chain, on warp 0, and everything else is taken off it.  With the
+// bottom wall's Neumann row the pivots are -c up to rounding, which gives a reciprocal seed to
+// a few units in the last place ahead of the chain: a row of the chain is five dependent
+// operations (c*bet, a*gam, b-, and one Newton step) instead of three and a division.  The
+// other warps fill the next panel's rows and seeds and check the last panel's: every row's
+// division is redone there with the plain operator, and the whole line falls back to thomas()
+// where one does not agree.  PRESSURE_CORRECTION of 512 rows, a 256-thread CTA: 155 k cycles
+// with one thread's chain, 52 k so; 1500 rows and 64 threads: 231 k.
+template <typename Row>
+__device__ __forceinline__ void solve_pressure(Col& c, Shared& sh, int n, Row row, double* p) {
+    const int tid = threadIdx.x, nt = blockDim.x;
+    const bool solo = nt == 32;
+    const int ht = solo ? tid : tid - 32, hn = solo ? nt : nt - 32;   // the helpers' threads
+    const bool walker = tid < 32, helper = solo || !walker;
+    const int np = (n + PANEL - 1) / PANEL;
+    double *gam = c.a[S_GAM], *sol = c.a[S_SOL];
+    bool bad = false;
+    auto fill = [&](int q, int t, int step) {
+        Panel& P = sh.panel[q & 1];
+        for (int i = t; i < PANEL; i += step) {
+            const int k = 1 + q * PANEL + i;
+            if (k <= n) {
+                double a, b, cc, r;
+                row(k, a, b, cc, r);
+                P.a[i] = a;
+                P.b[i] = b;
+                P.c[i] = cc;
+                P.r[i] = r;
+                P.y[i] = -1.0 / cc;
+            } else {
+                P.a[i] = P.c[i] = P.r[i] = 0.0;
+                P.b[i] = P.y[i] = 1.0;
+            }
+        }
+    };
+    auto check = [&](int q, int t, int step) {
+        const Panel& P = sh.panel[q & 1];
+        for (int i = t; i < PANEL; i += step) {
+            const int k = 1 + q * PANEL + i;
+            if (k > n) break;
+            const double y = 1.0 / (P.b[i] - P.a[i] * P.g[i]);
+            bad |= !(P.g[i + 1] == P.c[i] * y) || !(P.u[i + 1] == (P.r[i] - P.a[i] * P.u[i]) * y);
+            gam[k] = P.g[i];
+            sol[k] = P.u[i + 1];
+        }
+    };
+    double g = 0.0, u = 0.0;
+    fill(0, tid, nt);
+    __syncthreads();
+    for (int q = 0; q < np; ++q) {
+        if (walker) panel_forward(sh.panel[q & 1], min(PANEL, n - q * PANEL), g, u);
+        if (helper) {
+            if (q > 0) check(q - 1, ht, hn);
+            if (q + 1 < np) fill(q + 1, ht, hn);
+        }
+        __syncthreads();
+    }
+    check(np - 1, tid, nt);
+    if (__syncthreads_or(bad)) {
+        double *ak = c.a[S_AK], *bk = c.a[S_BK], *ck = c.a[S_CK], *gk = c.a[S_GK];
+        FOR_K(1, n) row(k, ak[k], bk[k], ck[k], gk[k]);
+        __syncthreads();
+        if (tid == 0) thomas(ak, bk, ck, gk, gam, 1, n);
+        __syncthreads();
+        FOR_K(1, n) p[k] = gk[k];
+        __syncthreads();
+        return;
+    }
+    // rows n .. 1, panel q holding rows n - q PANEL downwards
+    auto fill_back = [&](int q, int t, int step) {
+        Panel& P = sh.panel[q & 1];
+        for (int i = t; i < PANEL; i += step) {
+            const int k = n - q * PANEL - i;
+            P.a[i] = (k >= 1 && k < n) ? gam[k + 1] : 0.0;
+            P.b[i] = (k >= 1) ? sol[k] : 0.0;
+        }
+    };
+    auto store = [&](int q, int t, int step) {
+        const Panel& P = sh.panel[q & 1];
+        for (int i = t; i < PANEL; i += step) {
+            const int k = n - q * PANEL - i;
+            if (k >= 1) p[k] = P.c[i];
+        }
+    };
+    double x = 0.0;
+    fill_back(0, tid, nt);
+    __syncthreads();
+    for (int q = 0; q < np; ++q) {
+        if (walker) panel_back(sh.panel[q & 1], min(PANEL, n - q * PANEL), x);
+        if (helper) {
+            if (q > 0) store(q - 1, ht, hn);
+            if (q + 1 < np) fill_back(q + 1, ht, hn);
+        }
+        __syncthreads();
+    }
+    store(np - 1, tid, nt);
+    __syncthreads();
+}
+
 
 // REGION (1d.f:2038-2056), evaluated per cell: 2 within two cells of a PSI_CN jump, else 1
 // in liquid, else 0 (the serial loop's final state).
@@ -409,14 +737,13 @@ __device__ void cal_cont_bc(const Geo& g, const Phys& ph, Col& c) {
 }
 
 // LHSPS, 1d.f:4380-4497.
-__device__ void lhsps(const Geo& g, const Phys& ph, Col& c, double alpha, double dt) {
+__device__ void lhsps(const Geo& g, const Phys& ph, Col& c, Shared& sh, double alpha, double dt) {
     const int n = g.n;
     const double den_diffi = (ph.den_diff == 0.0) ? 1.0 : 1.0 / ph.den_diff;
     const double acops = alpha * dt / (ph.re * ph.prm);
-    double *ak = c.a[S_AK], *bk = c.a[S_BK], *ck = c.a[S_CK], *gk = c.a[S_GK];
     const double *psi_c = c.a[S_PSIC], *df_c = c.a[S_DFC];
     double* rhsps = c.a[S_RHSPS];
-    FOR_K(1, n) {
+    auto row = [&](int k, double& ak, double& bk, double& ck, double& gk) {
         const double denscf = ph.denscm + ph.densc_diff * psi_c[k];
         const double coef = acops / denscf;
         double psi_tmp = (df_c[k - 1] - ph.denm) * den_diffi;
@@ -425,24 +752,20 @@ __device__ void lhsps(const Geo& g, const Phys& ph, Col& c, double alpha, double
         const double tct = ph.tcm + ph.tc_diff * psi_tmp;
         double a = coef * tcb * g.akuv(k);
         double cc = coef * tct * g.ckuv(k);
-        bk[k] = 1.0 - (a + cc);
-        gk[k] = rhsps[k];
+        bk = 1.0 - (a + cc);
+        gk = rhsps[k];
         const double pc = c.psi_cn[k];
         if (fabs(pc - 0.5) != 0.5) {
             if (pc <= 0.5) cc = 0.0;
             else if (pc > 0.5) a = 0.0;
         }
-        ak[k] = a;
-        ck[k] = cc;
-    }
-    __syncthreads();
-    if (threadIdx.x == 0) thomas(ak, bk, ck, gk, c.a[S_GAM], 1, n);
-    __syncthreads();
-    FOR_K(1, n) {
-        rhsps[k] = gk[k];
-        c.t[k] = gk[k] + c.t[k];
-    }
-    __syncthreads();
+        ak = a;
+        ck = cc;
+    };
+    solve_line(c, sh, 1, n, row, [&](int k, double x) {
+        rhsps[k] = x;
+        c.t[k] = x + c.t[k];
+    });
     if (threadIdx.x == 0) {
         c.t[0] = 0.0;
         c.t[n] = 1.0;
@@ -1078,7 +1401,7 @@ __device__ int rhsnlhs(const Geo& g, const Phys& ph, Col& c, Shared& sh, double 
             rhsps[k] = ((densc - denscf) * c.t[k] + r) / denscf;
         }
         __syncthreads();
-        lhsps(g, ph, c, alpha, dt);   // substitute for the undefined LHSPS2
+        lhsps(g, ph, c, sh, alpha, dt);   // substitute for the undefined LHSPS2
         c.mark(PH_ENERGY);
         iters = temp_grad(g, ph, c, sh, L, dtconst);
         if (iters < 0) return iters;
@@ -1102,7 +1425,7 @@ __device__ int rhsnlhs(const Geo& g, const Phys& ph, Col& c, Shared& sh, double 
             rhsps[k] = ((densc - denscf) * c.t[k] + r) / denscf;
         }
         __syncthreads();
-        lhsps(g, ph, c, alpha, dt);
+        lhsps(g, ph, c, sh, alpha, dt);
         c.mark(PH_ENERGY);
     }
     // RHSZ (1d.f:1603-1745) and RHS1 = RHS1 / rho - W (1564-1568)
@@ -1138,22 +1461,17 @@ __device__ int rhsnlhs(const Geo& g, const Phys& ph, Col& c, Shared& sh, double 
     }
     // LHSW (1d.f:1749-1809)
     {
-        double *ak = c.a[S_AK], *bk = c.a[S_BK], *ck = c.a[S_CK], *gk = c.a[S_GK];
         const double* vf_z = c.a[S_VFZ];
-        FOR_K(2, n) {
+        auto row = [&](int k, double& ak, double& bk, double& ck, double& gk) {
             const double dk1 = 2. * acoef * denf_zi[k] * vf_z[k - 1] * g.akw(k);
             const double dk3 = 2. * acoef * denf_zi[k] * vf_z[k] * g.ckw(k);
             const double dk2 = -dk1 - dk3;
-            ak[k] = dk1;
-            ck[k] = dk3;
-            bk[k] = 1. + dk2;
-            gk[k] = rhs1[k];
-        }
-        __syncthreads();
-        if (threadIdx.x == 0) thomas(ak, bk, ck, gk, c.a[S_GAM], 2, n);
-        __syncthreads();
-        FOR_K(2, n) c.w[k] = gk[k] + c.w[k];
-        __syncthreads();
+            ak = dk1;
+            ck = dk3;
+            bk = 1. + dk2;
+            gk = rhs1[k];
+        };
+        solve_line(c, sh, 2, n, row, [&](int k, double x) { c.w[k] = x + c.w[k]; });
         c.mark(PH_LHSW);
     }
     // BC + BC_FLUX (1d.f:1812-1923)
@@ -1195,20 +1513,15 @@ __device__ void pressure_correction(const Geo& g, const Phys& ph, Col& c, Shared
         }
         __syncthreads();
         // POISSON (1d.f:3492-3578)
-        double *ak = c.a[S_AK], *bk = c.a[S_BK], *ck = c.a[S_CK], *gk = c.a[S_GK];
-        FOR_K(1, n) {
+        auto row = [&](int k, double& ak, double& bk, double& ck, double& gk) {
             const double fixkl = (k == 1) ? 1.0 : 0.0;
-            const double a = g.vvdz(k) * g.ssdz(k) * denf_zi[k] * (1.0 - fixkl);
-            const double cc = g.vvdz(k + 1) * g.ssdz(k) * denf_zi[k + 1];
-            ak[k] = a;
-            ck[k] = cc;
-            bk[k] = -(a + cc);
-            gk[k] = divg[k];
-        }
-        __syncthreads();
+            ak = g.vvdz(k) * g.ssdz(k) * denf_zi[k] * (1.0 - fixkl);
+            ck = g.vvdz(k + 1) * g.ssdz(k) * denf_zi[k + 1];
+            bk = -(ak + ck);
+            gk = divg[k];
+        };
+        solve_pressure(c, sh, n, row, c.p);
         if (threadIdx.x == 0) {
-            thomas(ak, bk, ck, gk, c.a[S_GAM], 1, n);
-            for (int k = 1; k <= n; ++k) c.p[k] = gk[k];
             c.p[0] = c.p[1];
             c.p[n + 1] = c.p[n];
         }
@@ -1338,7 +1651,6 @@ template <int NTH>
 // columns gain more from columns in flight than they lose to a few spilled registers.
 __global__ void __launch_bounds__(NTH, NTH == 32 ? 8 : (NTH == 64 ? 5 : 1)) k_column_steps(const __grid_constant__ Args A) {
     __shared__ Shared sh;
-    extern __shared__ double dsm[];   // 5 (n+2) doubles when A.tri_smem
     if ((int)blockIdx.x >= A.ncol) return;
     const int col = A.order ? A.order[blockIdx.x] : (int)blockIdx.x;
     int n;
@@ -1388,15 +1700,6 @@ __global__ void __launch_bounds__(NTH, NTH == 32 ? 8 : (NTH == 64 ? 5 : 1)) k_co
     double* d = A.dscr + od;
     for (int q = 0; q < NFLOW; ++q) c.a[q] = d + q * sf;
     c.psif_mtp = d + NFLOW * sf;
-    if (A.tri_smem && n <= A.tri_cap) {
-        // the Thomas coefficient, right-hand-side and elimination arrays: thread 0 walks
-        // them sequentially, so they are kept at shared-memory latency
-        c.a[S_AK] = dsm;
-        c.a[S_BK] = dsm + sf;
-        c.a[S_CK] = dsm + 2 * sf;
-        c.a[S_GK] = dsm + 3 * sf;
-        c.a[S_GAM] = dsm + 4 * sf;
-    }
     share_scratch(c);
     c.region = A.iscr + oi;
     c.prof = A.prof ? A.prof + (size_t)col * PH_COUNT : nullptr;
@@ -1780,15 +2083,6 @@ bool state_ok(const lica_col_state* st) {
            st->mflvs && st->sfgas && st->sfgas2 && st->imask && st->scal && st->stats;
 }
 
-// Launch A over A.ncol CTAs of `threads` threads; nmax = the largest column, which sizes
-// the shared-memory tridiagonal arrays.
-template <int NTH>
-int column_ctas_by_registers() {
-    int occ = 1;
-    cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ, colk::k_column_steps<NTH>, NTH, 0);
-    return std::max(occ, 1);
-}
-
 // The CTA width when the caller leaves it open: 256 threads while the batch has at most one
 // column per SM (each column is a latency chain, and a wider CTA finishes its phases sooner),
 // 64 beyond that (five columns per SM; on the 4096-column batch 64 threads take 25.6-25.8 ms
@@ -1804,53 +2098,13 @@ int default_width(int ncol) {
     return ncol <= sms ? 256 : 64;
 }
 
-int launch_columns(colk::Args& A, int nmax, int threads, void* stream, int cap_limit = -1) {
+int launch_columns(const colk::Args& A, int threads, void* stream) {
     const int nth = (threads == 32 || threads == 64 || threads == 128 || threads == 256) ? threads
                                                                                           : default_width(A.ncol);
-    // Shared-memory tridiagonal arrays for columns up to tri_cap cells, sized so that the
-    // CTAs the registers allow per SM still fit (longer columns keep them in scratch; the
-    // arithmetic is the same either way).
-    const int ctas = nth == 32    ? column_ctas_by_registers<32>()
-                     : nth == 64  ? column_ctas_by_registers<64>()
-                     : nth == 128 ? column_ctas_by_registers<128>()
-                                  : column_ctas_by_registers<256>();
-    const long budget = (long)(228 * 1024) / ctas - (long)sizeof(colk::Shared) - 2048;
-    long cap = std::min<long>(nmax, budget / (5 * (long)sizeof(double)) - 2);
-    if (cap_limit >= 0) cap = std::min<long>(cap, cap_limit);   // a caller's (autotuner's) limit
-    A.tri_cap = cap >= 64 ? (int)cap : 0;
-    A.tri_smem = A.tri_cap > 0 ? 1 : 0;
-    const size_t dyn = A.tri_smem ? 5 * ((size_t)A.tri_cap + 2) * sizeof(double) : 0;
-    {
-        // the attribute is the current device's: kept per device
-        static std::mutex mu;
-        static size_t set_bytes[kMaxDevices][4] = {};
-        std::lock_guard<std::mutex> lk(mu);
-        const int dev = current_device();
-        if (dev >= kMaxDevices) {
-            lica_set_last_error("launch_columns", "device ordinal above 63", __FILE__, __LINE__);
-            return LICA_BAD_ARG;
-        }
-        const int slot = nth == 64 ? 0 : (nth == 128 ? 1 : (nth == 256 ? 2 : 3));
-        if (dyn > set_bytes[dev][slot]) {
-            cudaError_t e = cudaSuccess;
-            if (nth == 32)
-                e = cudaFuncSetAttribute(colk::k_column_steps<32>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)dyn);
-            else if (nth == 64)
-                e = cudaFuncSetAttribute(colk::k_column_steps<64>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)dyn);
-            else if (nth == 128)
-                e = cudaFuncSetAttribute(colk::k_column_steps<128>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                         (int)dyn);
-            else
-                e = cudaFuncSetAttribute(colk::k_column_steps<256>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                         (int)dyn);
-            LICA_CUDA_TRY(e);
-            set_bytes[dev][slot] = dyn;
-        }
-    }
-    if (nth == 32) colk::k_column_steps<32><<<A.ncol, 32, dyn, (cudaStream_t)stream>>>(A);
-    else if (nth == 64) colk::k_column_steps<64><<<A.ncol, 64, dyn, (cudaStream_t)stream>>>(A);
-    else if (nth == 128) colk::k_column_steps<128><<<A.ncol, 128, dyn, (cudaStream_t)stream>>>(A);
-    else colk::k_column_steps<256><<<A.ncol, 256, dyn, (cudaStream_t)stream>>>(A);
+    if (nth == 32) colk::k_column_steps<32><<<A.ncol, 32, 0, (cudaStream_t)stream>>>(A);
+    else if (nth == 64) colk::k_column_steps<64><<<A.ncol, 64, 0, (cudaStream_t)stream>>>(A);
+    else if (nth == 128) colk::k_column_steps<128><<<A.ncol, 128, 0, (cudaStream_t)stream>>>(A);
+    else colk::k_column_steps<256><<<A.ncol, 256, 0, (cudaStream_t)stream>>>(A);
     LICA_CUDA_TRY(cudaGetLastError());
     lica_count_launches(1);
     return LICA_OK;
@@ -1924,7 +2178,7 @@ int column_steps_device(int32_t ncol, int32_t n, double length, const lica_col_p
     const size_t sf = (size_t)n + 2, sq = 2 * (size_t)n + 2;
     A.dscr = (double*)scr;
     A.iscr = (int*)((char*)scr + (size_t)ncol * (colk::NFLOW * sf + sq) * sizeof(double));
-    return launch_columns(A, n, threads, stream);
+    return launch_columns(A, threads, stream);
 }
 
 }  // namespace
@@ -2110,7 +2364,7 @@ int lica_gpu_column_batch_steps_ex_device(const lica_col_batch* b, const lica_co
     }
     A.dscr = (double*)scr;
     A.iscr = (int*)((char*)scr + (size_t)b->tot[3] * sizeof(double));
-    return launch_columns(A, b->nmax, threads, stream, tri_cap);
+    return launch_columns(A, threads, stream);
 }
 
 }  // extern "C"
