@@ -825,132 +825,151 @@ __device__ __forceinline__ double warp_maxd(double v) {
 
 constexpr int kMaxHalvings = 40;
 
-struct ExtpLane {
-    int lane, R;
-    bool act, small;
-    double vv, psh, fmn, fmx;
-    int im;
-    // one TEMP_EXTP_RK3 step (chphase.f:806-956) of the cell this lane holds
-    __device__ __forceinline__ double sweep(double x, double hl, double hr, int nd, double dtn, double redtl) const {
-        double xm = __shfl_up_sync(0xffffffffu, x, 1);
-        double xp = __shfl_down_sync(0xffffffffu, x, 1);
-        if (lane == 0) xm = hl;
-        if (lane == R - 1) xp = hr;
-        double nv = x;
-        if (act) {
-            const double apzm = (x - xm) * vv;
-            const double apzp = (xp - x) * vv;
-            const double ax = 0.0, ay = 0.0;
-            const double az = fmn * apzp + fmx * apzm;
-            double drhs;
-            if (im == 1) {
-                drhs = (ax + ay + az) + nd * dtn;
-                nv = x - redtl * drhs * (1 - psh);
-            } else {
-                drhs = (ax + ay + az) - nd * dtn;
-                nv = x - redtl * drhs * psh;
-            }
-            if (nd == 0 && small) {
-                drhs = (ax + ay + az);
-                nv = x - redtl * drhs;
-            }
-        }
-        return nv;
+// Whether every cell's relative change of an iteration is below eps: fabs(x / old - 1.0) < eps
+// for the largest cell that counts, as the butterfly of fmax over the lanes has it, without the
+// divisions where the answer is clear: |x - old| is compared with eps |old| by a margin far
+// above the roundings of either form, and only a lane in between (or a lane that is not finite)
+// makes the warp evaluate the quotients.  zero_counts: a cell that was 0 counts as changed by 1
+// when it moved (TEMP_EXTP's first loop) or not at all (its second).
+__device__ __forceinline__ bool extp_settled(double x, double old, bool valid, bool zero_counts, double eps) {
+    const double dx = fabs(x - old), ref = eps * fabs(old);
+    const bool plain = fabs(old) > 1e-290;
+    const bool below = !valid || (plain ? dx < ref * (1.0 - 1e-9) : (old == 0.0 && (x == 0.0 || !zero_counts)));
+    const bool above = valid && (plain ? (dx > ref * (1.0 + 1e-9) && dx < 1e290) : (old == 0.0 && zero_counts && dx > 0.0));
+    if (__any_sync(0xffffffffu, above)) return false;
+    if (__all_sync(0xffffffffu, below)) return true;
+    double rat = 0.0;
+    if (valid) {
+        if (old != 0.0) rat = fabs(x / old - 1.0);
+        else if (zero_counts && x != 0.0) rat = fabs(old / x - 1.0);
     }
+    return fabs(warp_maxd(rat)) < eps;
+}
+
+// One pseudo-time loop of TEMP_EXTP (100 SSP-RK3 iterations per step size, the step halved
+// until an iteration changes no cell by eps) on cells held one a lane.  TEMP_EXTP_RK3 is
+// first-order upwind in the direction of the phase, so a cell's three stages read the cell
+// itself and the three next upwind: each lane fetches those once per iteration and steps the
+// two nearer ones along (the same operations as their own lanes do), instead of a shuffle
+// between the stages.  w0..w2: the factors of the cell and the two next (0: the cell does not
+// move, which leaves x - dt * f * 0 = x); d0..d2 the source of the second loop (0 in the
+// first); v0..v2 VVDZ; edge1..3: the cell so far upwind is the halo, which stays at `halo`.
+// Returns the iterations, or -1 when kMaxHalvings halvings did not converge.
+struct ExtpCells {
+    double w0, w1, w2, d0, d1, d2, v0, v1, v2, halo;
+    int up1, up2, up3;
+    bool edge1, edge2, edge3, valid;
 };
+__device__ __forceinline__ double extp_up(double x, double up, double v, double d, double w, double redtl) {
+    return x - redtl * ((x - up) * v + d) * w;
+}
+__device__ __forceinline__ double extp_iteration(const ExtpCells& L, double x, double redtl) {
+    double x1 = __shfl_sync(0xffffffffu, x, L.up1), x2 = __shfl_sync(0xffffffffu, x, L.up2),
+           x3 = __shfl_sync(0xffffffffu, x, L.up3);
+    if (L.edge1) x1 = L.halo;
+    if (L.edge2) x2 = L.halo;
+    if (L.edge3) x3 = L.halo;
+    const double a0 = extp_up(x, x1, L.v0, L.d0, L.w0, redtl), a1 = extp_up(x1, x2, L.v1, L.d1, L.w1, redtl),
+                 a2 = extp_up(x2, x3, L.v2, L.d2, L.w2, redtl);
+    const double b0 = extp_up(a0, a1, L.v0, L.d0, L.w0, redtl), b1 = extp_up(a1, a2, L.v1, L.d1, L.w1, redtl);
+    const double m0 = 0.75 * x + 0.25 * b0;
+    double m1 = 0.75 * x1 + 0.25 * b1;
+    if (L.edge1) m1 = L.halo;
+    return 1.0 / 3.0 * x + 2.0 / 3.0 * extp_up(m0, m1, L.v0, L.d0, L.w0, redtl);
+}
+__device__ int extp_loop(const ExtpCells& L, double& x, double redtl, bool zero_counts, double eps) {
+    int total = 0;
+    for (int halving = 0; halving <= kMaxHalvings; ++halving) {
+        // the next iteration is on its way while the votes of this one come in
+        double y = extp_iteration(L, x, redtl);
+        for (int it = 1; it <= 100; ++it) {
+            ++total;
+            const double z = extp_iteration(L, y, redtl);
+            const bool done = extp_settled(y, x, L.valid, zero_counts, eps);
+            x = y;
+            if (done) return total;
+            y = z;
+        }
+        redtl = 0.5 * redtl;
+    }
+    return -1;
+}
 
 // TEMP_EXTP's two pseudo-time loops for an extension range of at most 32 cells: lane i
-// holds cell xk0 + lo + i in registers, neighbours come by shuffle, the halo cells (one
-// each side, never updated) are constants.  Same operations and order as extp_sweep.
-// Returns the iteration count, or -1 when kMaxHalvings halvings did not converge.
+// holds cell xk0 + lo + i in registers.  Same operations as extp_sweep on each cell; of its
+// sum fmin(nz, 0) * (downwind difference) + fmax(nz, 0) * (upwind difference) only the upwind
+// term is formed, the other being 0 for finite values.  512-cell column, about 515 iterations a
+// phase and step: 549 k cycles with three shuffles, a division and a butterfly of maxima an
+// iteration, 209 k so.  Returns the iteration count, -1 when
+// kMaxHalvings halvings did not converge, or -2, nothing done, where a value is not of
+// ordinary size (the general form then keeps the reference's Inf and NaN).
 __device__ int extp_registers(const Geo& g, const Shared& sh, XPhase& X, int xk0, int lo, int hi, int im,
                               double eps) {
     const int lane = threadIdx.x & 31;
-    ExtpLane L;
-    L.lane = lane;
-    L.R = hi - lo + 1;
-    L.im = im;
-    const bool valid = lane < L.R;
-    const int xi = valid ? lo + lane : lo;
-    const int k = xk0 + xi;
+    const int R = hi - lo + 1, dir = im == 1 ? 1 : -1;
+    const bool valid = lane < R;
     const double sm_grid = fmin(fmin(1.0, 1.0), 2.0 * g.hf);
-    const double nph = sh.x_nphi[xi];
-    L.act = false;
-    if (valid && nph != 0.0) {
+    // cell lane + q * dir: factor of both loops (f1 in the first, f2 in the second), VVDZ
+    auto cell = [&](int q, double& f1, double& f2, double& v) {
+        const int l = lane + q * dir;
+        f1 = f2 = v = 0.0;
+        if (!valid || l < 0 || l >= R) return;
+        const int xi = lo + l, k = xk0 + xi;
+        const double nph = sh.x_nphi[xi];
+        v = g.vvdz(k);
+        if (nph == 0.0) return;
         double dpz;
         if (sh.x_nphi[xi - 1] == 0.0) dpz = (sh.x_nphi[xi + 1] - nph) * g.vvdz(k + 1);
-        else if (sh.x_nphi[xi + 1] == 0.0) dpz = (nph - sh.x_nphi[xi - 1]) * g.vvdz(k);
-        else dpz = 0.5 * (sh.x_nphi[xi + 1] - sh.x_nphi[xi - 1]) * g.vvdz(k);
-        L.act = ((0.0 + 0.0) + dpz * dpz) != 0.0;
-    }
-    L.small = fabs(nph) <= sm_grid;
-    L.vv = g.vvdz(k);
-    L.psh = sh.x_psih[xi];
-    const double nz = (im == 1) ? (-1.0) * 1.0 : 1.0;
-    L.fmn = fmin(nz, 0.0);
-    L.fmx = fmax(nz, 0.0);
-    int total = 0;
-    // extension of the normal gradient (nd = 0); its halo values are 0
-    double x = X.dt[xi];
-    double redtl = 0.2 * sm_grid;
-    bool conv = false;
-    for (int halving = 0; halving <= kMaxHalvings && !conv; ++halving) {
-        for (int it = 1; it <= 100; ++it) {
-            ++total;
-            const double rk = x;
-            x = L.sweep(x, 0.0, 0.0, 0, x, redtl);
-            x = L.sweep(x, 0.0, 0.0, 0, x, redtl);
-            x = 0.75 * rk + 0.25 * x;
-            x = L.sweep(x, 0.0, 0.0, 0, x, redtl);
-            x = 1.0 / 3.0 * rk + 2.0 / 3.0 * x;
-            double rat = 0.0;
-            if (valid) {
-                if (rk != 0.0) rat = fabs(x / rk - 1.0);
-                else if (x != 0.0) rat = fabs(rk / x - 1.0);
-            }
-            rat = warp_maxd(rat);
-            if (fabs(rat) < eps) {
-                conv = true;
-                break;
-            }
-        }
-        if (!conv) redtl = 0.5 * redtl;
-    }
-    if (!conv) return -1;
-    const double dtn = x;
-    // extension of the phase temperature (nd = 1); halo = the unchanged neighbours
-    const double hl = X.tm[lo - 1], hr = X.tm[hi + 1];
-    double tm = X.tm[xi];
-    redtl = 0.2 * sm_grid;
-    conv = false;
-    for (int halving = 0; halving <= kMaxHalvings && !conv; ++halving) {
-        for (int it = 1; it <= 100; ++it) {
-            ++total;
-            const double rk = tm;
-            double to = tm;
-            to = L.sweep(to, hl, hr, 1, dtn, redtl);
-            to = L.sweep(to, hl, hr, 1, dtn, redtl);
-            to = 0.75 * rk + 0.25 * to;
-            to = L.sweep(to, hl, hr, 1, dtn, redtl);
-            to = 1.0 / 3.0 * rk + 2.0 / 3.0 * to;
-            tm = to;
-            double rat = 0.0;
-            if (valid && rk != 0.0) rat = fabs(tm / rk - 1.0);
-            rat = warp_maxd(rat);
-            if (fabs(rat) < eps) {
-                conv = true;
-                break;
-            }
-        }
-        if (!conv) redtl = 0.5 * redtl;
-    }
-    if (!conv) return -1;
+        else if (sh.x_nphi[xi + 1] == 0.0) dpz = (nph - sh.x_nphi[xi - 1]) * v;
+        else dpz = 0.5 * (sh.x_nphi[xi + 1] - sh.x_nphi[xi - 1]) * v;
+        if (((0.0 + 0.0) + dpz * dpz) == 0.0) return;
+        f2 = im == 1 ? 1 - sh.x_psih[xi] : sh.x_psih[xi];
+        f1 = fabs(nph) <= sm_grid ? 1.0 : f2;
+    };
+    ExtpCells L;
+    double f20, f21, f22;
+    cell(0, L.w0, f20, L.v0);
+    cell(1, L.w1, f21, L.v1);
+    cell(2, L.w2, f22, L.v2);
+    L.valid = valid;
+    L.up1 = (lane + dir) & 31;
+    L.up2 = (lane + 2 * dir) & 31;
+    L.up3 = (lane + 3 * dir) & 31;
+    auto outside = [&](int q) { const int l = lane + q * dir; return l < 0 || l >= R; };
+    L.edge1 = outside(1);
+    L.edge2 = outside(2);
+    L.edge3 = outside(3);
+    L.d0 = L.d1 = L.d2 = 0.0;
+    // the first loop's halo values are 0, the second's the unchanged upwind neighbour
+    const double t_halo = X.tm[im == 1 ? hi + 1 : lo - 1];
+    double x = valid ? X.dt[lo + lane] : 0.0;
+    double tm = valid ? X.tm[lo + lane] : 0.0;
+    const bool tame = fabs(x) < 1e100 && fabs(tm) < 1e100 && fabs(X.tm[lo - 1]) < 1e100 && fabs(X.tm[hi + 1]) < 1e100 &&
+                      fabs(L.v0) < 1e100 && fabs(f20) < 1e100;
+    if (!__all_sync(0xffffffffu, tame)) return -2;
+    // extension of the normal gradient (nd = 0)
+    L.halo = 0.0;
+    const int n1 = extp_loop(L, x, 0.2 * sm_grid, true, eps);
+    if (n1 < 0) return -1;
+    // extension of the phase temperature (nd = 1): the gradient is its source
+    L.w0 = f20;
+    L.w1 = f21;
+    L.w2 = f22;
+    const double src = im == 1 ? x : -x;
+    L.d0 = src;
+    L.d1 = __shfl_sync(0xffffffffu, src, L.up1);
+    L.d2 = __shfl_sync(0xffffffffu, src, L.up2);
+    if (L.edge1) L.d1 = 0.0;
+    if (L.edge2) L.d2 = 0.0;
+    L.halo = t_halo;
+    const int n2 = extp_loop(L, tm, 0.2 * sm_grid, false, eps);
+    if (n2 < 0) return -1;
     if (valid) {
-        X.dt[xi] = dtn;
-        X.tm[xi] = tm;
+        X.dt[lo + lane] = x;
+        X.tm[lo + lane] = tm;
     }
     __syncwarp();
-    return total;
+    return n1 + n2;
 }
 
 // TEMP_EXTP, chphase.f:467-805 (1-D), one phase (im = 0 vapour, 1 liquid) on one warp;
@@ -1002,10 +1021,10 @@ __device__ int temp_extp(const Geo& g, const Phys& ph, Shared& sh, int xk0, int 
         X.dt[i] = d;
     }
     __syncwarp();
-    if (hi - lo + 1 <= 32) {
-        const int it = extp_registers(g, sh, X, xk0, lo, hi, im, eps);
-        if (it < 0) return -1;
-        total += it;
+    const int quick = hi - lo + 1 <= 32 ? extp_registers(g, sh, X, xk0, lo, hi, im, eps) : -2;
+    if (quick != -2) {
+        if (quick < 0) return -1;
+        total += quick;
     } else {
         // extension of the normal gradient (nd = 0)
         double redtl = 0.2 * sm_grid;
