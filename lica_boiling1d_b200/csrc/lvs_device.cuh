@@ -4,6 +4,7 @@
 #pragma once
 #include "common.cuh"
 #include "column_geom.cuh"
+#include "fp64_rn.cuh"
 
 #include <cmath>
 
@@ -26,7 +27,6 @@ struct Win {
     double phi[WIN];
     double rk3[WIN];
     double alphio[WIN];
-    double dp[WIN];
     double nv[WIN];
     double wf[WIN];
     double start[WIN];   // phi at TRANSPORT entry: the phase test of the source, :1470
@@ -268,75 +268,149 @@ __device__ inline int band_generation(Ctx& c) {
     return __shfl_sync(0xffffffffu, ovf, 0);
 }
 
-// HJWENO, two_phase.f:2477-2500.
+// HJWENO, two_phase.f:2477-2500.  Its five quotients share two chains: the smoothness terms'
+// reciprocals side by side, then the sum's, which both weights take (fp64_rn.cuh; as plain
+// operators the five take 115 cycles each, one after the other).
 __device__ __forceinline__ double hjweno(double a, double b, double cc, double dd) {
     const double eps = 1e-6;
     const double s1 = 13.0 * (a - b) * (a - b) + 3.0 * (a - 3.0 * b) * (a - 3.0 * b);
     const double s2 = 13.0 * (b - cc) * (b - cc) + 3.0 * (b + cc) * (b + cc);
     const double s3 = 13.0 * (cc - dd) * (cc - dd) + 3.0 * (3.0 * cc - dd) * (3.0 * cc - dd);
-    const double a1 = 1.0 / ((eps + s1) * (eps + s1));
-    const double a2 = 6.0 / ((eps + s2) * (eps + s2));
-    const double a3 = 3.0 / ((eps + s3) * (eps + s3));
-    const double w1 = a1 / (a1 + a2 + a3);
-    const double w3 = a3 / (a1 + a2 + a3);
+    const double e1 = (eps + s1) * (eps + s1), e2 = (eps + s2) * (eps + s2), e3 = (eps + s3) * (eps + s3);
+    const double r2 = rn::recip(e2), r3 = rn::recip(e3);
+    double a1 = rn::recip(e1), a2 = rn::quot(6.0, e2, r2), a3 = rn::quot(3.0, e3, r3);
+    double sum = a1 + a2 + a3;
+    const double rs = rn::recip(sum);
+    double w1 = rn::quot(a1, sum, rs), w3 = rn::quot(a3, sum, rs);
+    if (!(rn::ordinary(e1) && rn::ordinary(e2) && rn::ordinary(e3) && rn::ordinary(sum))) {
+        a1 = 1.0 / e1;
+        a2 = 6.0 / e2;
+        a3 = 3.0 / e3;
+        sum = a1 + a2 + a3;
+        w1 = a1 / sum;
+        w3 = a3 / sum;
+    }
     return 1.0 / 3.0 * w1 * (a - 2.0 * b + cc) + 1.0 / 6.0 * (w3 - 0.5) * (b - 2.0 * cc + dd);
 }
 
-// face differences dp(i) = (phi(i+1) - phi(i)) * SSDZF over the window
-__device__ inline void face_diff(Ctx& c) {
-    Win* s = c.s;
-    // the WENO stencils of band cells read dp over [blo-3, bhi+2]
-    for (int i = max(0, c.blo - 3) + c.lane; i <= min(WIN - 1, c.bhi + 3); i += 32) {
-        const double b = (i + 1 < WIN) ? s->phi[i + 1] : 0.0;
-        s->dp[i] = (b - s->phi[i]) * c.ssdzf;
-    }
-    __syncwarp();
+// One-sided WENO5 derivative at window cell i (two_phase.f:1170-1290, z part) from the face
+// differences dp(j) = (phi(j+1) - phi(j)) * SSDZF: of the lower side (DM, from dp(i-3..i+1)) or
+// the upper (DP, from dp(i+2..i-2)).  Walking the cells towards i from its own side, the upper
+// one is the lower one's expression with every sign turned, but for the order of the sum; a
+// change of sign is exact throughout.  A band cell has three window cells on either side.
+__device__ __forceinline__ double weno_side(const Win* s, int i, double ssdzf, bool upper) {
+    const int j = upper ? i + 3 : i - 3, d = upper ? -1 : 1;
+    const double p0 = s->phi[j], p1 = s->phi[j + d], p2 = s->phi[j + 2 * d], p3 = s->phi[j + 3 * d],
+                 p4 = s->phi[j + 4 * d], p5 = s->phi[j + 5 * d];
+    const double v1 = (p1 - p0) * ssdzf, v2 = (p2 - p1) * ssdzf, v3 = (p3 - p2) * ssdzf, v4 = (p4 - p3) * ssdzf,
+                 v5 = (p5 - p4) * ssdzf;
+    const double w = hjweno(v2 - v1, v3 - v2, v4 - v3, v5 - v4);
+    const double t0 = upper ? v5 : v2, t1 = upper ? v4 : v3, t2 = upper ? v3 : v4, t3 = upper ? v2 : v5;
+    const double r = 1.0 / 12.0 * (-t0 + 7.0 * t1 + 7.0 * t2 - t3) - w;
+    return upper ? -r : r;
 }
 
-// one-sided WENO5 derivatives at window cell i (two_phase.f:1170-1290, z part)
-__device__ __forceinline__ void weno_z(const Win* s, int i, double& dm, double& dpl) {
-    {
-        const double v1 = s->dp[i - 3], v2 = s->dp[i - 2], v3 = s->dp[i - 1], v4 = s->dp[i], v5 = s->dp[i + 1];
-        const double w = hjweno(v2 - v1, v3 - v2, v4 - v3, v5 - v4);
-        dm = 1.0 / 12.0 * (-v2 + 7.0 * v3 + 7.0 * v4 - v5) - w;
-    }
-    {
-        const double v1 = s->dp[i + 2], v2 = s->dp[i + 1], v3 = s->dp[i], v4 = s->dp[i - 1], v5 = s->dp[i - 2];
-        const double w = hjweno(v1 - v2, v2 - v3, v3 - v4, v4 - v5);
-        dpl = 1.0 / 12.0 * (-v5 + 7.0 * v4 + 7.0 * v3 - v2) + w;
-    }
+// The usual band: at most 16 cells on layers 1..NN1 (WENO cells) and 32 on layers 1..NN2, as
+// every band of one interface has (two cells a layer).  The stages then run on registers:
+// lane e < c10 holds list cell e and its phi, and the two sides of WENO cell e are evaluated by
+// lanes e and e + 16 at once.  Phi in the window is what the neighbours read.
+struct Compact {
+    bool on;
+    int c8, c10, i, wi;   // this lane's cell (lane < c10), the WENO cell of its side (lane % 16 < c8)
+};
+__device__ __forceinline__ Compact compact_band(const Ctx& c) {
+    Compact b;
+    b.c8 = c.s->lstart[NN1 + 1];
+    b.c10 = c.s->lstart[NN2 + 1];
+    b.on = b.c8 <= 16 && b.c10 <= 32;
+    b.i = (b.on && c.lane < b.c10) ? c.s->lst[c.lane] : 0;
+    b.wi = (b.on && (c.lane & 15) < b.c8) ? c.s->lst[c.lane & 15] : 0;
+    return b;
+}
+// dm, dpl of this lane's cell (lanes < c8)
+__device__ __forceinline__ void compact_weno(const Ctx& c, const Compact& b, double& dm, double& dpl) {
+    double v = 0.0;
+    if ((c.lane & 15) < b.c8) v = weno_side(c.s, b.wi, c.ssdzf, c.lane >= 16);
+    dm = __shfl_sync(0xffffffffu, v, c.lane & 15);
+    dpl = __shfl_sync(0xffffffffu, v, (c.lane & 15) + 16);
 }
 
-// TRANSPORT_RK3, two_phase.f:1133-1495 (1-D): one upwind/LLF stage on layers 1..NN1 plus
-// the phase-change source, liquid side divided by DENR (:1466-1477).
+// TRANSPORT_RK3, two_phase.f:1133-1495 (1-D), of one cell: the upwind/LLF flux of layers
+// 1..NN1; src: the phase-change source times the step, divided by DENR on the liquid side
+// (:1466-1477).
+__device__ __forceinline__ double transport_cell(double phi, double uu1, double uu2, double dm, double dpl,
+                                                 double dtlvs, int iphs, double src) {
+    const double uu3 = 0.5 * (uu1 + uu2);
+    double az;
+    if (uu1 >= 0.0 && uu2 >= 0.0 && uu3 >= 0.0) {
+        az = uu3 * dm;
+    } else if (uu1 <= 0.0 && uu2 <= 0.0 && uu3 <= 0.0) {
+        az = uu3 * dpl;
+    } else {
+        const double umax = fmax(fmax(fabs(uu1), fabs(uu2)), fabs(uu3));
+        az = 0.5 * (uu3 * (dpl + dm) - umax * (dpl - dm));
+    }
+    double pn = phi - dtlvs * ((0.0 + 0.0) + az);
+    if (iphs == 1) pn = pn - src;
+    return pn;
+}
+__device__ __forceinline__ double transport_source(const Win* s, int i, double dtlvs, int iphs, double denr) {
+    if (iphs != 1) return 0.0;
+    return s->start[i] > 0.0 ? dtlvs * s->mf[i] / denr : dtlvs * s->mf[i];
+}
+
 __device__ inline void transport_rk3(Ctx& c, double dtlvs, int iphs, double denr) {
     Win* s = c.s;
-    face_diff(c);
     for (int i = c.blo + c.lane; i <= c.bhi; i += 32) {
         const int m = s->layer[i];
         if (m < 1 || m > NN1) continue;
-        const double uu1 = s->wf[i], uu2 = s->wf[i + 1], uu3 = 0.5 * (uu1 + uu2);
-        double dm, dpl, az;
-        weno_z(s, i, dm, dpl);
-        if (uu1 >= 0.0 && uu2 >= 0.0 && uu3 >= 0.0) {
-            az = uu3 * dm;
-        } else if (uu1 <= 0.0 && uu2 <= 0.0 && uu3 <= 0.0) {
-            az = uu3 * dpl;
-        } else {
-            const double umax = fmax(fmax(fabs(uu1), fabs(uu2)), fabs(uu3));
-            az = 0.5 * (uu3 * (dpl + dm) - umax * (dpl - dm));
-        }
-        double pn = s->phi[i] - dtlvs * ((0.0 + 0.0) + az);
-        if (iphs == 1) {
-            if (s->start[i] > 0.0) pn = pn - dtlvs * s->mf[i] / denr;
-            else pn = pn - dtlvs * s->mf[i];
-        }
-        s->nv[i] = pn;
+        const double dm = weno_side(s, i, c.ssdzf, false), dpl = weno_side(s, i, c.ssdzf, true);
+        s->nv[i] = transport_cell(s->phi[i], s->wf[i], s->wf[i + 1], dm, dpl, dtlvs, iphs,
+                                  transport_source(s, i, dtlvs, iphs, denr));
     }
     __syncwarp();
     for (int i = c.blo + c.lane; i <= c.bhi; i += 32) {
         const int m = s->layer[i];
         if (m >= 1 && m <= NN1) s->phi[i] = s->nv[i];
+    }
+    __syncwarp();
+}
+
+// The three stages of one TRANSPORT substep on layers 1..NN1 (two_phase.f:855-905).
+__device__ inline void transport_substep(Ctx& c, double dtlvs, int iphs, double denr) {
+    Win* s = c.s;
+    const Compact b = compact_band(c);
+    if (b.on) {
+        const bool mine = c.lane < b.c8;
+        const double p0 = mine ? s->phi[b.i] : 0.0, u1 = s->wf[b.i], u2 = s->wf[b.i + 1];
+        const double src = mine ? transport_source(s, b.i, dtlvs, iphs, denr) : 0.0;
+        double p = p0, dm, dpl;
+        for (int st = 0; st < 3; ++st) {
+            compact_weno(c, b, dm, dpl);
+            if (mine) {
+                p = transport_cell(p, u1, u2, dm, dpl, dtlvs, iphs, src);
+                if (st == 1) p = 0.75 * p0 + 0.25 * p;
+                if (st == 2) p = 1.0 / 3.0 * p0 + 2.0 / 3.0 * p;
+            }
+            __syncwarp();
+            if (mine) s->phi[b.i] = p;
+            __syncwarp();
+        }
+        return;
+    }
+    for (int i = c.blo + c.lane; i <= c.bhi; i += 32) s->rk3[i] = s->phi[i];
+    __syncwarp();
+    transport_rk3(c, dtlvs, iphs, denr);
+    transport_rk3(c, dtlvs, iphs, denr);
+    for (int i = c.blo + c.lane; i <= c.bhi; i += 32) {
+        const int m = s->layer[i];
+        if (m >= 1 && m <= NN1) s->phi[i] = 0.75 * s->rk3[i] + 0.25 * s->phi[i];
+    }
+    __syncwarp();
+    transport_rk3(c, dtlvs, iphs, denr);
+    for (int i = c.blo + c.lane; i <= c.bhi; i += 32) {
+        const int m = s->layer[i];
+        if (m >= 1 && m <= NN1) s->phi[i] = 1.0 / 3.0 * s->rk3[i] + 2.0 / 3.0 * s->phi[i];
     }
     __syncwarp();
 }
@@ -351,30 +425,39 @@ __device__ __forceinline__ double godunov(double sg, double ap, double am) {
     return ap;
 }
 
-// REINITIALIZATION_RK3, two_phase.f:2174-2445 (1-D): WENO on layers 1..NN1, first-order
-// one-sided differences on NN1+1..NN2, Peng's smoothed sign with eps = min(h)^2.
+// REINITIALIZATION_RK3, two_phase.f:2174-2445 (1-D), of one cell: dz its central difference,
+// a0 its phi at entry; Peng's smoothed sign with eps = min(h)^2.  The x and y parts of GODUNOV
+// are 0, and the root of a square is the value itself wherever the square neither over- nor
+// underflows (a square and its root each rounded to nearest).
+__device__ __forceinline__ double reinit_cell(double phi, double a0, double dz, double dm, double dpl, double eps,
+                                              double redtl) {
+    const double dal = (0.0 + 0.0) + dz * dz;
+    const double den = sqrt(a0 * a0 + dal * eps);
+    double sg = rn::quot(a0, den, rn::recip(den));
+    if (!(rn::ordinary(a0) && rn::ordinary(den))) sg = a0 / den;
+    const double az = godunov(sg, dpl, dm);
+    double root = fabs(az);
+    if (!rn::ordinary(az) && az != 0.0) root = sqrt(az * az);
+    const double drhs = sg * (1.0 - root);
+    return phi + redtl * drhs;
+}
+
 __device__ inline void reinit_rk3(Ctx& c, double redtl) {
     Win* s = c.s;
     const double eps = c.hf * c.hf;
-    face_diff(c);
     for (int i = c.blo + c.lane; i <= c.bhi; i += 32) {
         const int m = s->layer[i];
         if (m < 1 || m > NN2) continue;
         const double dz = 0.5 * (s->phi[i + 1] - s->phi[i - 1]) * c.ssdzf;
-        const double dal = (0.0 + 0.0) + dz * dz;
-        const double a0 = s->alphio[i];
-        const double sg = a0 / sqrt(a0 * a0 + dal * eps);
         double dm, dpl;
         if (m <= NN1) {
-            weno_z(s, i, dm, dpl);
+            dm = weno_side(s, i, c.ssdzf, false);
+            dpl = weno_side(s, i, c.ssdzf, true);
         } else {
             dm = (s->phi[i] - s->phi[i - 1]) * c.ssdzf;
             dpl = (s->phi[i + 1] - s->phi[i]) * c.ssdzf;
         }
-        const double ax = godunov(sg, 0.0, 0.0), ay = godunov(sg, 0.0, 0.0);
-        const double az = godunov(sg, dpl, dm);
-        const double drhs = sg * (1.0 - sqrt(ax * ax + ay * ay + az * az));
-        s->nv[i] = s->phi[i] + redtl * drhs;
+        s->nv[i] = reinit_cell(s->phi[i], s->alphio[i], dz, dm, dpl, eps, redtl);
     }
     __syncwarp();
     for (int i = c.blo + c.lane; i <= c.bhi; i += 32) {
@@ -384,12 +467,43 @@ __device__ inline void reinit_rk3(Ctx& c, double redtl) {
     __syncwarp();
 }
 
-// REINITIALIZATION, two_phase.f:2033-2170: ILIMIT pseudo-time SSP-RK3 steps, dtau = h/2.
+// REINITIALIZATION, two_phase.f:2033-2170: ILIMIT pseudo-time SSP-RK3 steps, dtau = h/2: WENO on
+// layers 1..NN1, first-order one-sided differences on NN1+1..NN2.  Ten iterations of the usual
+// band: 88 k cycles with ten dependent divisions and two roots a stage, NEW_REINIT k so.
 __device__ inline void reinitialization(Ctx& c, int ilimit) {
     Win* s = c.s;
+    const double redtl = 0.5 * c.hf;
+    const Compact b = compact_band(c);
+    if (b.on) {
+        const double eps = c.hf * c.hf;
+        const bool mine = c.lane < b.c10;
+        const double a0 = mine ? s->phi[b.i] : 0.0;
+        double p = a0;
+        for (int it = 0; it < ilimit; ++it) {
+            const double rk = p;
+            for (int st = 0; st < 3; ++st) {
+                double dm, dpl;
+                compact_weno(c, b, dm, dpl);
+                if (mine) {
+                    const double pm = s->phi[b.i - 1], pp = s->phi[b.i + 1];
+                    const double dz = 0.5 * (pp - pm) * c.ssdzf;
+                    if (c.lane >= b.c8) {
+                        dm = (p - pm) * c.ssdzf;
+                        dpl = (pp - p) * c.ssdzf;
+                    }
+                    p = reinit_cell(p, a0, dz, dm, dpl, eps, redtl);
+                    if (st == 1) p = 0.75 * rk + 0.25 * p;
+                    if (st == 2) p = 1.0 / 3.0 * rk + 2.0 / 3.0 * p;
+                }
+                __syncwarp();
+                if (mine) s->phi[b.i] = p;
+                __syncwarp();
+            }
+        }
+        return;
+    }
     for (int i = c.blo + c.lane; i <= c.bhi; i += 32) s->alphio[i] = s->phi[i];
     __syncwarp();
-    const double redtl = 0.5 * c.hf;
     for (int it = 0; it < ilimit; ++it) {
         for (int i = c.blo + c.lane; i <= c.bhi; i += 32) s->rk3[i] = s->phi[i];
         __syncwarp();
@@ -730,21 +844,7 @@ __device__ inline int transport_column(Win* s, int lane, int n, double length, d
         }
         if (time_tran + dtlvs >= P.dtconst) dtlvs = P.dtconst - time_tran;
         time_tran = time_tran + dtlvs;
-        for (int i = c.blo + lane; i <= c.bhi; i += 32) s->rk3[i] = s->phi[i];
-        __syncwarp();
-        transport_rk3(c, dtlvs, P.iphs, P.denr);
-        transport_rk3(c, dtlvs, P.iphs, P.denr);
-        for (int i = c.blo + lane; i <= c.bhi; i += 32) {
-            const int m = s->layer[i];
-            if (m >= 1 && m <= NN1) s->phi[i] = 0.75 * s->rk3[i] + 0.25 * s->phi[i];
-        }
-        __syncwarp();
-        transport_rk3(c, dtlvs, P.iphs, P.denr);
-        for (int i = c.blo + lane; i <= c.bhi; i += 32) {
-            const int m = s->layer[i];
-            if (m >= 1 && m <= NN1) s->phi[i] = 1.0 / 3.0 * s->rk3[i] + 2.0 / 3.0 * s->phi[i];
-        }
-        __syncwarp();
+        transport_substep(c, dtlvs, P.iphs, P.denr);
         rein_trigger(c, dmax, dmin);
         imass = (dmax > 2.0 || dmin < 1e-4) ? 1 : 0;
         if (P.iphs == 1) {
