@@ -1,6 +1,6 @@
-// Correctly rounded FP64 reciprocals and quotients without a branch.
+// Correctly rounded FP64 reciprocals, quotients and square roots without a branch.
 //
-// `a / b` and `1.0 / b` carry a test for extreme operands and a call behind it, so two
+// `a / b`, `1.0 / b` and `sqrt` carry a test for extreme operands and a call behind it, so two
 // independent divisions of one thread do not overlap: measured on a B200, 64 cycles for 1/b,
 // 115 for a/b, and 123 for two independent 1/b.  These forms are straight-line FMA chains
 // that do overlap, and the test for extreme operands (`ordinary`) is apart, to be made once
@@ -12,7 +12,10 @@
 // for every b but a mantissa of all ones; the quotient by Markstein's correction of a
 // quotient within a unit in the last place (P. W. Markstein, "Computation of elementary
 // functions on the IBM RISC System/6000 processor", IBM J. Res. Dev. 34, 1990).  A first
-// correction brings a * (1/b), up to 1.5 units off, to within one.
+// correction brings a * (1/b), up to 1.5 units off, to within one.  The square root by two
+// coupled Newton steps (Goldschmidt) from the hardware's seed and a last correction, the
+// rounding then checked by the remainder's size (Tuckerman's test): g is the rounded root of x
+// exactly if -g ulp(g) < x - g^2 <= g ulp(g).
 #pragma once
 
 namespace lica {
@@ -40,6 +43,25 @@ __device__ __forceinline__ double quot(double a, double b, double y) {
     double q = a * y;
     q = __fma_rn(__fma_rn(-b, q, a), y, q);
     return __fma_rn(__fma_rn(-b, q, a), y, q);
+}
+
+// sqrt(x), x ordinary; ok is cleared where the result is not the correctly rounded root
+__device__ __forceinline__ double root(double x, bool& ok) {
+    double y;
+    asm("rsqrt.approx.ftz.f64 %0, %1;" : "=d"(y) : "d"(x));
+    double g = x * y, h = 0.5 * y;
+    double r = __fma_rn(-g, h, 0.5);
+    g = __fma_rn(g, r, g);
+    h = __fma_rn(h, r, h);
+    r = __fma_rn(-g, h, 0.5);
+    g = __fma_rn(g, r, g);
+    h = __fma_rn(h, r, h);
+    g = __fma_rn(__fma_rn(-g, g, x), h, g);
+    // ulp(g) = 2^(exponent - 52): g >= 2^-200 here
+    const double gu = g * __hiloint2double((__double2hiint(g) & 0x7ff00000) - (52 << 20), 0);
+    const double rem = __fma_rn(-g, g, x);
+    ok = ok && rem > -gu && rem <= gu;
+    return g;
 }
 
 }  // namespace rn

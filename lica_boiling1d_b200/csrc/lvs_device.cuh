@@ -268,28 +268,32 @@ __device__ inline int band_generation(Ctx& c) {
     return __shfl_sync(0xffffffffu, ovf, 0);
 }
 
-// HJWENO, two_phase.f:2477-2500.  Its five quotients share two chains: the smoothness terms'
-// reciprocals side by side, then the sum's, which both weights take (fp64_rn.cuh; as plain
-// operators the five take 115 cycles each, one after the other).
-__device__ __forceinline__ double hjweno(double a, double b, double cc, double dd) {
+// HJWENO, two_phase.f:2477-2500, with the plain operators.
+static __device__ __noinline__ double hjweno_plain(double a, double b, double cc, double dd) {
+    const double eps = 1e-6;
+    const double s1 = 13.0 * (a - b) * (a - b) + 3.0 * (a - 3.0 * b) * (a - 3.0 * b);
+    const double s2 = 13.0 * (b - cc) * (b - cc) + 3.0 * (b + cc) * (b + cc);
+    const double s3 = 13.0 * (cc - dd) * (cc - dd) + 3.0 * (3.0 * cc - dd) * (3.0 * cc - dd);
+    const double a1 = 1.0 / ((eps + s1) * (eps + s1));
+    const double a2 = 6.0 / ((eps + s2) * (eps + s2));
+    const double a3 = 3.0 / ((eps + s3) * (eps + s3));
+    const double w1 = a1 / (a1 + a2 + a3);
+    const double w3 = a3 / (a1 + a2 + a3);
+    return 1.0 / 3.0 * w1 * (a - 2.0 * b + cc) + 1.0 / 6.0 * (w3 - 0.5) * (b - 2.0 * cc + dd);
+}
+// The same, its five quotients on two branch-free chains: the smoothness terms' reciprocals side
+// by side, then the sum's, which both weights take (as plain operators the five take 115 cycles
+// each, one after the other).  ok is cleared where a term is out of the ordinary range.
+__device__ __forceinline__ double hjweno(double a, double b, double cc, double dd, bool& ok) {
     const double eps = 1e-6;
     const double s1 = 13.0 * (a - b) * (a - b) + 3.0 * (a - 3.0 * b) * (a - 3.0 * b);
     const double s2 = 13.0 * (b - cc) * (b - cc) + 3.0 * (b + cc) * (b + cc);
     const double s3 = 13.0 * (cc - dd) * (cc - dd) + 3.0 * (3.0 * cc - dd) * (3.0 * cc - dd);
     const double e1 = (eps + s1) * (eps + s1), e2 = (eps + s2) * (eps + s2), e3 = (eps + s3) * (eps + s3);
-    const double r2 = rn::recip(e2), r3 = rn::recip(e3);
-    double a1 = rn::recip(e1), a2 = rn::quot(6.0, e2, r2), a3 = rn::quot(3.0, e3, r3);
-    double sum = a1 + a2 + a3;
-    const double rs = rn::recip(sum);
-    double w1 = rn::quot(a1, sum, rs), w3 = rn::quot(a3, sum, rs);
-    if (!(rn::ordinary(e1) && rn::ordinary(e2) && rn::ordinary(e3) && rn::ordinary(sum))) {
-        a1 = 1.0 / e1;
-        a2 = 6.0 / e2;
-        a3 = 3.0 / e3;
-        sum = a1 + a2 + a3;
-        w1 = a1 / sum;
-        w3 = a3 / sum;
-    }
+    const double a1 = rn::recip(e1), a2 = rn::quot(6.0, e2, rn::recip(e2)), a3 = rn::quot(3.0, e3, rn::recip(e3));
+    const double sum = a1 + a2 + a3, rs = rn::recip(sum);
+    const double w1 = rn::quot(a1, sum, rs), w3 = rn::quot(a3, sum, rs);
+    ok = ok && rn::ordinary(e1) && rn::ordinary(e2) && rn::ordinary(e3) && rn::ordinary(sum);
     return 1.0 / 3.0 * w1 * (a - 2.0 * b + cc) + 1.0 / 6.0 * (w3 - 0.5) * (b - 2.0 * cc + dd);
 }
 
@@ -298,39 +302,48 @@ __device__ __forceinline__ double hjweno(double a, double b, double cc, double d
 // the upper (DP, from dp(i+2..i-2)).  Walking the cells towards i from its own side, the upper
 // one is the lower one's expression with every sign turned, but for the order of the sum; a
 // change of sign is exact throughout.  A band cell has three window cells on either side.
-__device__ __forceinline__ double weno_side(const Win* s, int i, double ssdzf, bool upper) {
+template <bool PLAIN>
+__device__ __forceinline__ double weno_side(const Win* s, int i, double ssdzf, bool upper, bool& ok) {
     const int j = upper ? i + 3 : i - 3, d = upper ? -1 : 1;
     const double p0 = s->phi[j], p1 = s->phi[j + d], p2 = s->phi[j + 2 * d], p3 = s->phi[j + 3 * d],
                  p4 = s->phi[j + 4 * d], p5 = s->phi[j + 5 * d];
     const double v1 = (p1 - p0) * ssdzf, v2 = (p2 - p1) * ssdzf, v3 = (p3 - p2) * ssdzf, v4 = (p4 - p3) * ssdzf,
                  v5 = (p5 - p4) * ssdzf;
-    const double w = hjweno(v2 - v1, v3 - v2, v4 - v3, v5 - v4);
+    const double w = PLAIN ? hjweno_plain(v2 - v1, v3 - v2, v4 - v3, v5 - v4)
+                           : hjweno(v2 - v1, v3 - v2, v4 - v3, v5 - v4, ok);
     const double t0 = upper ? v5 : v2, t1 = upper ? v4 : v3, t2 = upper ? v3 : v4, t3 = upper ? v2 : v5;
     const double r = 1.0 / 12.0 * (-t0 + 7.0 * t1 + 7.0 * t2 - t3) - w;
     return upper ? -r : r;
+}
+__device__ __forceinline__ double weno_plain(const Win* s, int i, double ssdzf, bool upper) {
+    bool ok = true;
+    return weno_side<true>(s, i, ssdzf, upper, ok);
 }
 
 // The usual band: at most 16 cells on layers 1..NN1 (WENO cells) and 32 on layers 1..NN2, as
 // every band of one interface has (two cells a layer).  The stages then run on registers:
 // lane e < c10 holds list cell e and its phi, and the two sides of WENO cell e are evaluated by
-// lanes e and e + 16 at once.  Phi in the window is what the neighbours read.
+// lanes e and e + 16 at once.  Phi in the window is what the neighbours read.  Lanes without a
+// cell compute on a cell of the band all the same and keep nothing, so a stage has no branch and
+// its chains (the weights, the smoothed sign) interleave; where an operand is out of the
+// ordinary range the stage is redone with the plain operators.
 struct Compact {
     bool on;
-    int c8, c10, i, wi;   // this lane's cell (lane < c10), the WENO cell of its side (lane % 16 < c8)
+    int c8, c10, i, wi;   // this lane's cell (its own for lane < c10), the WENO cell of its side
 };
 __device__ __forceinline__ Compact compact_band(const Ctx& c) {
     Compact b;
     b.c8 = c.s->lstart[NN1 + 1];
     b.c10 = c.s->lstart[NN2 + 1];
-    b.on = b.c8 <= 16 && b.c10 <= 32;
-    b.i = (b.on && c.lane < b.c10) ? c.s->lst[c.lane] : 0;
-    b.wi = (b.on && (c.lane & 15) < b.c8) ? c.s->lst[c.lane & 15] : 0;
+    b.on = b.c8 >= 1 && b.c8 <= 16 && b.c10 <= 32;
+    b.i = b.on ? c.s->lst[min(c.lane, b.c10 - 1)] : 0;
+    b.wi = b.on ? c.s->lst[min(c.lane & 15, b.c8 - 1)] : 0;
     return b;
 }
 // dm, dpl of this lane's cell (lanes < c8)
-__device__ __forceinline__ void compact_weno(const Ctx& c, const Compact& b, double& dm, double& dpl) {
-    double v = 0.0;
-    if ((c.lane & 15) < b.c8) v = weno_side(c.s, b.wi, c.ssdzf, c.lane >= 16);
+template <bool PLAIN>
+__device__ __forceinline__ void compact_weno(const Ctx& c, const Compact& b, double& dm, double& dpl, bool& ok) {
+    const double v = weno_side<PLAIN>(c.s, b.wi, c.ssdzf, c.lane >= 16, ok);
     dm = __shfl_sync(0xffffffffu, v, c.lane & 15);
     dpl = __shfl_sync(0xffffffffu, v, (c.lane & 15) + 16);
 }
@@ -364,7 +377,7 @@ __device__ inline void transport_rk3(Ctx& c, double dtlvs, int iphs, double denr
     for (int i = c.blo + c.lane; i <= c.bhi; i += 32) {
         const int m = s->layer[i];
         if (m < 1 || m > NN1) continue;
-        const double dm = weno_side(s, i, c.ssdzf, false), dpl = weno_side(s, i, c.ssdzf, true);
+        const double dm = weno_plain(s, i, c.ssdzf, false), dpl = weno_plain(s, i, c.ssdzf, true);
         s->nv[i] = transport_cell(s->phi[i], s->wf[i], s->wf[i + 1], dm, dpl, dtlvs, iphs,
                                   transport_source(s, i, dtlvs, iphs, denr));
     }
@@ -382,16 +395,16 @@ __device__ inline void transport_substep(Ctx& c, double dtlvs, int iphs, double 
     const Compact b = compact_band(c);
     if (b.on) {
         const bool mine = c.lane < b.c8;
-        const double p0 = mine ? s->phi[b.i] : 0.0, u1 = s->wf[b.i], u2 = s->wf[b.i + 1];
-        const double src = mine ? transport_source(s, b.i, dtlvs, iphs, denr) : 0.0;
+        const double p0 = s->phi[b.i], u1 = s->wf[b.i], u2 = s->wf[b.i + 1];
+        const double src = transport_source(s, b.i, dtlvs, iphs, denr);
         double p = p0, dm, dpl;
         for (int st = 0; st < 3; ++st) {
-            compact_weno(c, b, dm, dpl);
-            if (mine) {
-                p = transport_cell(p, u1, u2, dm, dpl, dtlvs, iphs, src);
-                if (st == 1) p = 0.75 * p0 + 0.25 * p;
-                if (st == 2) p = 1.0 / 3.0 * p0 + 2.0 / 3.0 * p;
-            }
+            bool ok = true;
+            compact_weno<false>(c, b, dm, dpl, ok);
+            if (!__all_sync(0xffffffffu, ok)) compact_weno<true>(c, b, dm, dpl, ok);
+            p = transport_cell(p, u1, u2, dm, dpl, dtlvs, iphs, src);
+            if (st == 1) p = 0.75 * p0 + 0.25 * p;
+            if (st == 2) p = 1.0 / 3.0 * p0 + 2.0 / 3.0 * p;
             __syncwarp();
             if (mine) s->phi[b.i] = p;
             __syncwarp();
@@ -415,30 +428,37 @@ __device__ inline void transport_substep(Ctx& c, double dtlvs, int iphs, double 
     __syncwarp();
 }
 
-// GODUNOV, two_phase.f:2448-2474.
+// GODUNOV, two_phase.f:2448-2474 (its tests in reverse, so that the first one decides).
 __device__ __forceinline__ double godunov(double sg, double ap, double am) {
     const double aplus = sg * ap, aminus = sg * am;
-    if (aplus >= 0.0 && aminus >= 0.0) return am;
-    if (aplus <= 0.0 && aminus <= 0.0) return ap;
-    if (aplus > 0.0 && aminus < 0.0) return 0.0;
-    if (aplus + aminus > 0.0) return am;
-    return ap;
+    double r = (aplus + aminus > 0.0) ? am : ap;
+    r = (aplus > 0.0 && aminus < 0.0) ? 0.0 : r;
+    r = (aplus <= 0.0 && aminus <= 0.0) ? ap : r;
+    return (aplus >= 0.0 && aminus >= 0.0) ? am : r;
 }
 
 // REINITIALIZATION_RK3, two_phase.f:2174-2445 (1-D), of one cell: dz its central difference,
 // a0 its phi at entry; Peng's smoothed sign with eps = min(h)^2.  The x and y parts of GODUNOV
 // are 0, and the root of a square is the value itself wherever the square neither over- nor
 // underflows (a square and its root each rounded to nearest).
+template <bool PLAIN>
 __device__ __forceinline__ double reinit_cell(double phi, double a0, double dz, double dm, double dpl, double eps,
-                                              double redtl) {
+                                              double redtl, bool& ok) {
     const double dal = (0.0 + 0.0) + dz * dz;
-    const double den = sqrt(a0 * a0 + dal * eps);
-    double sg = rn::quot(a0, den, rn::recip(den));
-    if (!(rn::ordinary(a0) && rn::ordinary(den))) sg = a0 / den;
+    const double sq = a0 * a0 + dal * eps;
+    double sg;
+    if (PLAIN) {
+        sg = a0 / sqrt(sq);
+    } else {
+        const double den = rn::root(sq, ok);
+        sg = rn::quot(a0, den, rn::recip(den));
+        ok = ok && rn::ordinary(sq) && rn::ordinary(a0) && rn::ordinary(den);
+    }
     const double az = godunov(sg, dpl, dm);
-    double root = fabs(az);
-    if (!rn::ordinary(az) && az != 0.0) root = sqrt(az * az);
-    const double drhs = sg * (1.0 - root);
+    double mod = fabs(az);
+    if (PLAIN) mod = sqrt(az * az);
+    else ok = ok && (rn::ordinary(az) || az == 0.0);
+    const double drhs = sg * (1.0 - mod);
     return phi + redtl * drhs;
 }
 
@@ -451,13 +471,14 @@ __device__ inline void reinit_rk3(Ctx& c, double redtl) {
         const double dz = 0.5 * (s->phi[i + 1] - s->phi[i - 1]) * c.ssdzf;
         double dm, dpl;
         if (m <= NN1) {
-            dm = weno_side(s, i, c.ssdzf, false);
-            dpl = weno_side(s, i, c.ssdzf, true);
+            dm = weno_plain(s, i, c.ssdzf, false);
+            dpl = weno_plain(s, i, c.ssdzf, true);
         } else {
             dm = (s->phi[i] - s->phi[i - 1]) * c.ssdzf;
             dpl = (s->phi[i + 1] - s->phi[i]) * c.ssdzf;
         }
-        s->nv[i] = reinit_cell(s->phi[i], s->alphio[i], dz, dm, dpl, eps, redtl);
+        bool ok = true;
+        s->nv[i] = reinit_cell<true>(s->phi[i], s->alphio[i], dz, dm, dpl, eps, redtl, ok);
     }
     __syncwarp();
     for (int i = c.blo + c.lane; i <= c.bhi; i += 32) {
@@ -477,24 +498,26 @@ __device__ inline void reinitialization(Ctx& c, int ilimit) {
     if (b.on) {
         const double eps = c.hf * c.hf;
         const bool mine = c.lane < b.c10;
-        const double a0 = mine ? s->phi[b.i] : 0.0;
+        const bool first_order = c.lane >= b.c8;
+        const double a0 = s->phi[b.i];
         double p = a0;
         for (int it = 0; it < ilimit; ++it) {
             const double rk = p;
             for (int st = 0; st < 3; ++st) {
+                const double pm = s->phi[b.i - 1], pp = s->phi[b.i + 1];
+                const double dz = 0.5 * (pp - pm) * c.ssdzf;
+                const double fm = (p - pm) * c.ssdzf, fp = (pp - p) * c.ssdzf;
                 double dm, dpl;
-                compact_weno(c, b, dm, dpl);
-                if (mine) {
-                    const double pm = s->phi[b.i - 1], pp = s->phi[b.i + 1];
-                    const double dz = 0.5 * (pp - pm) * c.ssdzf;
-                    if (c.lane >= b.c8) {
-                        dm = (p - pm) * c.ssdzf;
-                        dpl = (pp - p) * c.ssdzf;
-                    }
-                    p = reinit_cell(p, a0, dz, dm, dpl, eps, redtl);
-                    if (st == 1) p = 0.75 * rk + 0.25 * p;
-                    if (st == 2) p = 1.0 / 3.0 * rk + 2.0 / 3.0 * p;
+                bool ok = true;
+                compact_weno<false>(c, b, dm, dpl, ok);
+                double q = reinit_cell<false>(p, a0, dz, first_order ? fm : dm, first_order ? fp : dpl, eps, redtl, ok);
+                if (!__all_sync(0xffffffffu, ok)) {
+                    compact_weno<true>(c, b, dm, dpl, ok);
+                    q = reinit_cell<true>(p, a0, dz, first_order ? fm : dm, first_order ? fp : dpl, eps, redtl, ok);
                 }
+                if (st == 1) q = 0.75 * rk + 0.25 * q;
+                if (st == 2) q = 1.0 / 3.0 * rk + 2.0 / 3.0 * q;
+                p = q;
                 __syncwarp();
                 if (mine) s->phi[b.i] = p;
                 __syncwarp();
