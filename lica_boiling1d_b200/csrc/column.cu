@@ -972,6 +972,79 @@ __device__ int extp_registers(const Geo& g, const Shared& sh, XPhase& X, int xk0
     return n1 + n2;
 }
 
+// The two pseudo-time loops for any range, in passes over shared memory.
+__device__ __noinline__ int extp_general(const Geo g, Shared& sh, int xk0, int lo, int hi, int im) {
+    const int lane = threadIdx.x & 31;
+    const double sm_grid = fmin(fmin(2.0 * 0.5, 2.0 * 0.5), 2.0 * g.hf);
+    const double eps = 1e-4;
+    XPhase& X = sh.xp[im];
+    int total = 0;
+    // extension of the normal gradient (nd = 0)
+    double redtl = 0.2 * sm_grid;
+    bool conv = false;
+    for (int halving = 0; halving <= kMaxHalvings && !conv; ++halving) {
+        for (int it = 1; it <= 100; ++it) {
+            ++total;
+            for (int i = lo + lane; i <= hi; i += 32) X.dtrk[i] = X.dt[i];
+            __syncwarp();
+            extp_sweep(g, sh, X, xk0, lo, hi, X.dt, im, redtl, 0);
+            extp_sweep(g, sh, X, xk0, lo, hi, X.dt, im, redtl, 0);
+            for (int i = lo + lane; i <= hi; i += 32) X.dt[i] = 0.75 * X.dtrk[i] + 0.25 * X.dt[i];
+            __syncwarp();
+            extp_sweep(g, sh, X, xk0, lo, hi, X.dt, im, redtl, 0);
+            double rat = 0.0;
+            for (int i = lo + lane; i <= hi; i += 32) {
+                const double v = 1.0 / 3.0 * X.dtrk[i] + 2.0 / 3.0 * X.dt[i];
+                X.dt[i] = v;
+                if (X.dtrk[i] != 0.0) rat = fmax(fabs(v / X.dtrk[i] - 1.0), rat);
+                else if (v != 0.0) rat = fmax(fabs(X.dtrk[i] / v - 1.0), rat);
+            }
+            rat = warp_maxd(rat);
+            __syncwarp();
+            if (fabs(rat) < eps) {
+                conv = true;
+                break;
+            }
+        }
+        if (!conv) redtl = 0.5 * redtl;
+    }
+    if (!conv) return -1;
+    // extension of the phase temperature (nd = 1)
+    redtl = 0.2 * sm_grid;
+    conv = false;
+    for (int halving = 0; halving <= kMaxHalvings && !conv; ++halving) {
+        for (int it = 1; it <= 100; ++it) {
+            ++total;
+            for (int i = lo - 1 + lane; i <= hi + 1; i += 32) {
+                X.trk[i] = X.tm[i];
+                X.to[i] = X.tm[i];
+            }
+            __syncwarp();
+            extp_sweep(g, sh, X, xk0, lo, hi, X.to, im, redtl, 1);
+            extp_sweep(g, sh, X, xk0, lo, hi, X.to, im, redtl, 1);
+            for (int i = lo + lane; i <= hi; i += 32) X.to[i] = 0.75 * X.trk[i] + 0.25 * X.to[i];
+            __syncwarp();
+            extp_sweep(g, sh, X, xk0, lo, hi, X.to, im, redtl, 1);
+            double rat = 0.0;
+            for (int i = lo + lane; i <= hi; i += 32) {
+                const double v = 1.0 / 3.0 * X.trk[i] + 2.0 / 3.0 * X.to[i];
+                X.to[i] = v;
+                X.tm[i] = v;
+                if (X.trk[i] != 0.0) rat = fmax(fabs(v / X.trk[i] - 1.0), rat);
+            }
+            rat = warp_maxd(rat);
+            __syncwarp();
+            if (fabs(rat) < eps) {
+                conv = true;
+                break;
+            }
+        }
+        if (!conv) redtl = 0.5 * redtl;
+    }
+    if (!conv) return -1;
+    return total;
+}
+
 // TEMP_EXTP, chphase.f:467-805 (1-D), one phase (im = 0 vapour, 1 liquid) on one warp;
 // the two phases are independent and run on warps 0 and 1 at once.  Only cells with
 // NPHI != 0 change; they lie in [xk0+lo, xk0+hi], held with one halo cell each side in
@@ -1026,69 +1099,9 @@ __device__ int temp_extp(const Geo& g, const Phys& ph, Shared& sh, int xk0, int 
         if (quick < 0) return -1;
         total += quick;
     } else {
-        // extension of the normal gradient (nd = 0)
-        double redtl = 0.2 * sm_grid;
-        bool conv = false;
-        for (int halving = 0; halving <= kMaxHalvings && !conv; ++halving) {
-            for (int it = 1; it <= 100; ++it) {
-                ++total;
-                for (int i = lo + lane; i <= hi; i += 32) X.dtrk[i] = X.dt[i];
-                __syncwarp();
-                extp_sweep(g, sh, X, xk0, lo, hi, X.dt, im, redtl, 0);
-                extp_sweep(g, sh, X, xk0, lo, hi, X.dt, im, redtl, 0);
-                for (int i = lo + lane; i <= hi; i += 32) X.dt[i] = 0.75 * X.dtrk[i] + 0.25 * X.dt[i];
-                __syncwarp();
-                extp_sweep(g, sh, X, xk0, lo, hi, X.dt, im, redtl, 0);
-                double rat = 0.0;
-                for (int i = lo + lane; i <= hi; i += 32) {
-                    const double v = 1.0 / 3.0 * X.dtrk[i] + 2.0 / 3.0 * X.dt[i];
-                    X.dt[i] = v;
-                    if (X.dtrk[i] != 0.0) rat = fmax(fabs(v / X.dtrk[i] - 1.0), rat);
-                    else if (v != 0.0) rat = fmax(fabs(X.dtrk[i] / v - 1.0), rat);
-                }
-                rat = warp_maxd(rat);
-                __syncwarp();
-                if (fabs(rat) < eps) {
-                    conv = true;
-                    break;
-                }
-            }
-            if (!conv) redtl = 0.5 * redtl;
-        }
-        if (!conv) return -1;
-        // extension of the phase temperature (nd = 1)
-        redtl = 0.2 * sm_grid;
-        conv = false;
-        for (int halving = 0; halving <= kMaxHalvings && !conv; ++halving) {
-            for (int it = 1; it <= 100; ++it) {
-                ++total;
-                for (int i = lo - 1 + lane; i <= hi + 1; i += 32) {
-                    X.trk[i] = X.tm[i];
-                    X.to[i] = X.tm[i];
-                }
-                __syncwarp();
-                extp_sweep(g, sh, X, xk0, lo, hi, X.to, im, redtl, 1);
-                extp_sweep(g, sh, X, xk0, lo, hi, X.to, im, redtl, 1);
-                for (int i = lo + lane; i <= hi; i += 32) X.to[i] = 0.75 * X.trk[i] + 0.25 * X.to[i];
-                __syncwarp();
-                extp_sweep(g, sh, X, xk0, lo, hi, X.to, im, redtl, 1);
-                double rat = 0.0;
-                for (int i = lo + lane; i <= hi; i += 32) {
-                    const double v = 1.0 / 3.0 * X.trk[i] + 2.0 / 3.0 * X.to[i];
-                    X.to[i] = v;
-                    X.tm[i] = v;
-                    if (X.trk[i] != 0.0) rat = fmax(fabs(v / X.trk[i] - 1.0), rat);
-                }
-                rat = warp_maxd(rat);
-                __syncwarp();
-                if (fabs(rat) < eps) {
-                    conv = true;
-                    break;
-                }
-            }
-            if (!conv) redtl = 0.5 * redtl;
-        }
-        if (!conv) return -1;
+        const int it = extp_general(g, sh, xk0, lo, hi, im);
+        if (it < 0) return -1;
+        total += it;
     }
     for (int i = lo + lane; i <= hi; i += 32) temp_g[xk0 + i] = X.tm[i];
     __syncwarp();
@@ -1134,50 +1147,78 @@ __device__ int temp_grad(const Geo& g, const Phys& ph, Col& c, Shared& sh, doubl
     const int xk0 = cx.kw0;   // valid on warp 0; shared below through ibuf
     if (warp == 0) {
         // (1) NPHI / PSIH of the flow cells of the band (:147-211), in list order; every
-        // band cell's flow cell lies in [xk0+2, xk0+66]
-        if (lane == 0) {
-            int ic = 0;
-            for (int j = s->lstart[1]; j < s->lstart[lvs::NN2 + 1]; ++j) {
-                const int k = cx.w0 + s->lst[j];
-                const int kk = g.kcoump_vel(k);
-                const int x = kk - xk0;
-                if (sh.x_nphi[x] == 0.0) {
-                    const int k1 = g.kcou2(kk), k2 = g.kcoump2(kk);   // PHINSINTP's KCOU2(KO), KCOUMP2(KO)
-                    const double zd = (k1 == k2) ? 0.0 : (g.zp(kk) - g.zpf(k1)) / (g.zpf(k2) - g.zpf(k1));
-                    const double a1 = cx.p(k1), a2 = cx.p(k2);
-                    const double c00 = a1 * (1.0 - 0.5) + a1 * 0.5;
-                    const double c01 = a2 * (1.0 - 0.5) + a2 * 0.5;
-                    const double c0 = c00 * (1.0 - 0.5) + c00 * 0.5;
-                    const double c1 = c01 * (1.0 - 0.5) + c01 * 0.5;
-                    double nsphi = c0 * (1.0 - zd) + c1 * zd;
-                    if (nsphi > 0.0) ic = 1;
-                    if (nsphi < 0.0) ic = 0;
-                    if (a1 == 0.0 || a2 == 0.0) nsphi = 0.0;
-                    sh.x_nphi[x] = 1e-7;
-                    sh.x_nphi[x] = nsphi;
-                    if (fabs(sh.x_pcn[x] - 0.5) != 0.5) sh.x_psih[x] = (double)ic;
-                    else sh.x_psih[x] = sh.x_pcn[x];
-                }
-            }
-            for (int j = s->lstart[lvs::N_MAX]; j < s->lstart[lvs::N_MAX + 1]; ++j) {
-                const int k = cx.w0 + s->lst[j];
-                const int kk = g.kcoump_vel(k);
-                const int x = kk - xk0;
+        // band cell's flow cell lies in [xk0+2, xk0+66].  The interpolations are independent and
+        // run one list cell a lane; where none is zero (the reference skips a flow cell already
+        // set, and a zero leaves it unset) the first list cell of a flow cell decides it, and
+        // PHINSINTP's IC is its own sign; else the list is walked in order.  One lane doing
+        // both took 38 k cycles a substep, 7 k so.
+        const int j0 = s->lstart[1], j1 = s->lstart[lvs::NN2 + 1], j2 = s->lstart[lvs::N_MAX + 1];
+        double *ns = s->rk3, *zero = s->alphio;   // by list position
+        int *xs = s->lst2, *first = s->fmask;     // flow cell by list position; first position by flow cell
+        for (int x = lane; x < XR; x += 32) first[x] = 1 << 30;
+        __syncwarp();
+        bool clear = true;
+        for (int j = j0 + lane; j < j2; j += 32) {
+            const int k = cx.w0 + s->lst[j];
+            const int kk = g.kcoump_vel(k);
+            xs[j] = kk - xk0;
+            if (j < j1) {
+                const int k1 = g.kcou2(kk), k2 = g.kcoump2(kk);   // PHINSINTP's KCOU2(KO), KCOUMP2(KO)
+                const double zd = (k1 == k2) ? 0.0 : (g.zp(kk) - g.zpf(k1)) / (g.zpf(k2) - g.zpf(k1));
+                const double a1 = cx.p(k1), a2 = cx.p(k2);
+                const double c00 = a1 * (1.0 - 0.5) + a1 * 0.5;
+                const double c01 = a2 * (1.0 - 0.5) + a2 * 0.5;
+                const double c0 = c00 * (1.0 - 0.5) + c00 * 0.5;
+                const double c1 = c01 * (1.0 - 0.5) + c01 * 0.5;
+                const double nsphi = c0 * (1.0 - zd) + c1 * zd;
+                ns[j] = nsphi;
+                zero[j] = (a1 == 0.0 || a2 == 0.0) ? 1.0 : 0.0;
+                clear = clear && (nsphi > 0.0 || nsphi < 0.0) && a1 != 0.0 && a2 != 0.0;
+                atomicMin(&first[kk - xk0], j);
+            } else {
                 const double dx = 0.25, dy = 0.25;
                 const double dz = g.zpf(k) - g.zp(kk);
-                const double pre = s->phi[s->lst[j]] + sqrt(dx * dx + dy * dy + dz * dz);
-                sh.x_nphi[x] = fmin(sh.x_nphi[x], pre);
+                ns[j] = s->phi[s->lst[j]] + sqrt(dx * dx + dy * dy + dz * dz);
+            }
+        }
+        clear = __all_sync(0xffffffffu, clear);
+        __syncwarp();
+        if (clear) {
+            for (int j = j0 + lane; j < j1; j += 32) {
+                const int x = xs[j];
+                if (first[x] != j) continue;
+                sh.x_nphi[x] = ns[j];
+                sh.x_psih[x] = fabs(sh.x_pcn[x] - 0.5) != 0.5 ? (ns[j] > 0.0 ? 1.0 : 0.0) : sh.x_pcn[x];
+            }
+        } else if (lane == 0) {
+            int ic = 0;
+            for (int j = j0; j < j1; ++j) {
+                const int x = xs[j];
+                if (sh.x_nphi[x] != 0.0) continue;
+                if (ns[j] > 0.0) ic = 1;
+                if (ns[j] < 0.0) ic = 0;
+                sh.x_nphi[x] = zero[j] != 0.0 ? 0.0 : ns[j];
+                sh.x_psih[x] = fabs(sh.x_pcn[x] - 0.5) != 0.5 ? (double)ic : sh.x_pcn[x];
+            }
+        }
+        __syncwarp();
+        if (lane == 0)
+            for (int j = j1; j < j2; ++j) {
+                const int x = xs[j];
+                sh.x_nphi[x] = fmin(sh.x_nphi[x], ns[j]);
                 sh.x_psih[x] = sh.x_pcn[x];
             }
-            // extension range: the cells with NPHI != 0
-            int ka = n + 1, kb = 0;
-            for (int j = s->lstart[1]; j < s->lstart[lvs::N_MAX + 1]; ++j) {
-                const int kk = g.kcoump_vel(cx.w0 + s->lst[j]);
-                if (sh.x_nphi[kk - xk0] != 0.0) {
-                    ka = min(ka, kk);
-                    kb = max(kb, kk);
-                }
+        __syncwarp();
+        // extension range: the cells with NPHI != 0
+        int ka = n + 1, kb = 0;
+        for (int j = j0 + lane; j < j2; j += 32)
+            if (sh.x_nphi[xs[j]] != 0.0) {
+                ka = min(ka, xs[j] + xk0);
+                kb = max(kb, xs[j] + xk0);
             }
+        ka = __reduce_min_sync(0xffffffffu, ka);
+        kb = __reduce_max_sync(0xffffffffu, kb);
+        if (lane == 0) {
             sh.ibuf[1] = ka;
             sh.ibuf[2] = kb;
             sh.ibuf[7] = xk0;
@@ -1328,7 +1369,8 @@ __device__ int temp_grad(const Geo& g, const Phys& ph, Col& c, Shared& sh, doubl
             {
                 int ktop, kbot;
                 lvs::window_crossings(cx, ktop, kbot);
-                if (lane == 0) c.scal[4] = lvs::column_vapour_volume(cx, s->nv, ktop, kbot, 0.5 * 0.5 * g.hf);
+                const double vol = lvs::column_vapour_volume(cx, s->nv, ktop, kbot, 0.5 * 0.5 * g.hf);
+                if (lane == 0) c.scal[4] = vol;
             }
             for (int i = cx.blo + lane; i <= cx.bhi; i += 32) {
                 const int k = cx.w0 + i, m = s->layer[i];
@@ -1369,11 +1411,11 @@ __device__ void cal_continuity2(const Geo& g, const Phys& ph, Col& c) {
         if (k >= 2) {
             double v = psi_z[k];
             if (reg[k] == 2)
-                v = v - col::box_mean(c.sfgas2, nf, g.kcou2(k), g.kcou1(k + 1), g.zp(k - 1), g.zp(k), g.hf);
+                v = v - col::box_mean_sparse(c.sfgas2, nf, g.kcou2(k), g.kcou1(k + 1), g.zp(k - 1), g.zp(k), g.hf);
             psi_z[k] = (v > 1.0) ? 1.0 : (v < 0.0 ? 0.0 : v);
         }
         double v = psi_c[k];
-        if (reg[k] == 2) v = v - col::box_mean(c.sfgas2, nf, g.kcou2(k), g.kcou1(k + 1), g.z(k), g.z(k + 1), g.hf);
+        if (reg[k] == 2) v = v - col::box_mean_sparse(c.sfgas2, nf, g.kcou2(k), g.kcou1(k + 1), g.z(k), g.z(k + 1), g.hf);
         psi_c[k] = (v > 1.0) ? 1.0 : (v < 0.0 ? 0.0 : v);
     }
     __syncthreads();
@@ -1524,7 +1566,7 @@ __device__ void pressure_correction(const Geo& g, const Phys& ph, Col& c, Shared
         FOR_K(1, n) {
             double d = (k <= n - 1) ? (c.w[k + 1] - c.w[k]) * g.ssdz(k) : 0.0;
             if (ph.iphs == 1) {
-                const double ssum = col::box_mean(c.sfgas, g.nf, g.kcou2(k), g.kcou1(k + 1), g.z(k), g.z(k + 1), g.hf);
+                const double ssum = col::box_mean_sparse(c.sfgas, g.nf, g.kcou2(k), g.kcou1(k + 1), g.z(k), g.z(k + 1), g.hf);
                 d = d - ssum * (ph.den_diff / (ph.denp * ph.denm));
             }
             if (k >= 2) d = d * dtconsti;
@@ -1612,7 +1654,7 @@ __device__ int column_step(const Geo& g, const Phys& ph, Col& c, Shared& sh, dou
         FOR_K(1, n) {
             double d = (c.w[k + 1] - c.w[k]) * g.ssdz(k);
             if (ph.iphs == 1) {
-                const double ssum = col::box_mean(c.sfgas, g.nf, g.kcou2(k), g.kcou1(k + 1), g.z(k), g.z(k + 1), g.hf);
+                const double ssum = col::box_mean_sparse(c.sfgas, g.nf, g.kcou2(k), g.kcou1(k + 1), g.z(k), g.z(k + 1), g.hf);
                 d = d - ssum * (ph.den_diff / ph.denp);
             }
             dv = fmax(fabs(d), dv);

@@ -47,7 +47,7 @@ __device__ __forceinline__ int kcoump_vel(double h, double hf, int n, int k) {
 // k1..k2: the x/y ranges cover both refined replicas whole, so the z loop runs once per
 // (II,JJ) replica -- four times -- and the result is PSI_SUM/VOLF.  f is indexed [k],
 // k = 1..nf; indices outside that range read the nearest end value.
-__device__ __forceinline__ double box_mean(const double* f, int nf, int k1, int k2, double z1, double z2,
+static __device__ __noinline__ double box_mean(const double* f, int nf, int k1, int k2, double z1, double z2,
                                            double hf) {
     const double ssdzf = 1.0 / hf;
     double sum = 0.0, volf = 0.0;
@@ -74,6 +74,16 @@ __device__ __forceinline__ double box_mean(const double* f, int nf, int k1, int 
         }
     }
     return sum / volf;
+}
+
+// The same for fields that are zero away from the interface (SFGAS, SFGAS2): where every value
+// of the box is zero the mean is too, without the sums and divisions.  For boxes of some
+// extent inside the column, whose volume is not zero.
+__device__ __forceinline__ double box_mean_sparse(const double* f, int nf, int k1, int k2, double z1, double z2,
+                                                  double hf) {
+    bool any = false;
+    for (int kk = k1; kk <= k2; ++kk) any |= f[kk < 1 ? 1 : (kk > nf ? nf : kk)] != 0.0;
+    return any ? box_mean(f, nf, k1, k2, z1, z2, hf) : 0.0;
 }
 
 }  // namespace col

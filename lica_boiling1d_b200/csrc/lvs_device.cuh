@@ -372,7 +372,7 @@ __device__ __forceinline__ double transport_source(const Win* s, int i, double d
     return s->start[i] > 0.0 ? dtlvs * s->mf[i] / denr : dtlvs * s->mf[i];
 }
 
-__device__ inline void transport_rk3(Ctx& c, double dtlvs, int iphs, double denr) {
+__device__ __forceinline__ void transport_rk3(const Ctx& c, double dtlvs, int iphs, double denr) {
     Win* s = c.s;
     for (int i = c.blo + c.lane; i <= c.bhi; i += 32) {
         const int m = s->layer[i];
@@ -385,6 +385,25 @@ __device__ inline void transport_rk3(Ctx& c, double dtlvs, int iphs, double denr
     for (int i = c.blo + c.lane; i <= c.bhi; i += 32) {
         const int m = s->layer[i];
         if (m >= 1 && m <= NN1) s->phi[i] = s->nv[i];
+    }
+    __syncwarp();
+}
+
+static __device__ __noinline__ void transport_general(Ctx c, double dtlvs, int iphs, double denr) {
+    Win* s = c.s;
+    for (int i = c.blo + c.lane; i <= c.bhi; i += 32) s->rk3[i] = s->phi[i];
+    __syncwarp();
+    transport_rk3(c, dtlvs, iphs, denr);
+    transport_rk3(c, dtlvs, iphs, denr);
+    for (int i = c.blo + c.lane; i <= c.bhi; i += 32) {
+        const int m = s->layer[i];
+        if (m >= 1 && m <= NN1) s->phi[i] = 0.75 * s->rk3[i] + 0.25 * s->phi[i];
+    }
+    __syncwarp();
+    transport_rk3(c, dtlvs, iphs, denr);
+    for (int i = c.blo + c.lane; i <= c.bhi; i += 32) {
+        const int m = s->layer[i];
+        if (m >= 1 && m <= NN1) s->phi[i] = 1.0 / 3.0 * s->rk3[i] + 2.0 / 3.0 * s->phi[i];
     }
     __syncwarp();
 }
@@ -411,21 +430,7 @@ __device__ inline void transport_substep(Ctx& c, double dtlvs, int iphs, double 
         }
         return;
     }
-    for (int i = c.blo + c.lane; i <= c.bhi; i += 32) s->rk3[i] = s->phi[i];
-    __syncwarp();
-    transport_rk3(c, dtlvs, iphs, denr);
-    transport_rk3(c, dtlvs, iphs, denr);
-    for (int i = c.blo + c.lane; i <= c.bhi; i += 32) {
-        const int m = s->layer[i];
-        if (m >= 1 && m <= NN1) s->phi[i] = 0.75 * s->rk3[i] + 0.25 * s->phi[i];
-    }
-    __syncwarp();
-    transport_rk3(c, dtlvs, iphs, denr);
-    for (int i = c.blo + c.lane; i <= c.bhi; i += 32) {
-        const int m = s->layer[i];
-        if (m >= 1 && m <= NN1) s->phi[i] = 1.0 / 3.0 * s->rk3[i] + 2.0 / 3.0 * s->phi[i];
-    }
-    __syncwarp();
+    transport_general(c, dtlvs, iphs, denr);
 }
 
 // GODUNOV, two_phase.f:2448-2474 (its tests in reverse, so that the first one decides).
@@ -439,8 +444,8 @@ __device__ __forceinline__ double godunov(double sg, double ap, double am) {
 
 // REINITIALIZATION_RK3, two_phase.f:2174-2445 (1-D), of one cell: dz its central difference,
 // a0 its phi at entry; Peng's smoothed sign with eps = min(h)^2.  The x and y parts of GODUNOV
-// are 0, and the root of a square is the value itself wherever the square neither over- nor
-// underflows (a square and its root each rounded to nearest).
+// are 0, and the root of a square is the value itself where the square neither over- nor
+// underflows (a square and its root each rounded to nearest); below that 1 less it is 1 both ways.
 template <bool PLAIN>
 __device__ __forceinline__ double reinit_cell(double phi, double a0, double dz, double dm, double dpl, double eps,
                                               double redtl, bool& ok) {
@@ -457,12 +462,12 @@ __device__ __forceinline__ double reinit_cell(double phi, double a0, double dz, 
     const double az = godunov(sg, dpl, dm);
     double mod = fabs(az);
     if (PLAIN) mod = sqrt(az * az);
-    else ok = ok && (rn::ordinary(az) || az == 0.0);
+    else ok = ok && (__double2hiint(az) & 0x7fffffff) < 0x5f000000;   // below 2^496
     const double drhs = sg * (1.0 - mod);
     return phi + redtl * drhs;
 }
 
-__device__ inline void reinit_rk3(Ctx& c, double redtl) {
+__device__ __forceinline__ void reinit_rk3(const Ctx& c, double redtl) {
     Win* s = c.s;
     const double eps = c.hf * c.hf;
     for (int i = c.blo + c.lane; i <= c.bhi; i += 32) {
@@ -488,9 +493,48 @@ __device__ inline void reinit_rk3(Ctx& c, double redtl) {
     __syncwarp();
 }
 
+// One stage of the usual band's cell with the plain operators.
+static __device__ __noinline__ double reinit_stage_plain(const Win* s, int wi, bool first_order, double ssdzf, double p,
+                                                         double a0, double eps, double redtl, int i) {
+    const int lane = threadIdx.x & 31;
+    bool ok = true;
+    const double v = weno_side<true>(s, wi, ssdzf, lane >= 16, ok);
+    const double dm = __shfl_sync(0xffffffffu, v, lane & 15), dpl = __shfl_sync(0xffffffffu, v, (lane & 15) + 16);
+    const double pm = s->phi[i - 1], pp = s->phi[i + 1];
+    const double dz = 0.5 * (pp - pm) * ssdzf;
+    return reinit_cell<true>(p, a0, dz, first_order ? (p - pm) * ssdzf : dm, first_order ? (pp - p) * ssdzf : dpl, eps,
+                             redtl, ok);
+}
+
+// REINITIALIZATION of any band, in passes over the window.  Out of line, like the other rare
+// paths: the step's code is read once per launch of one step, and its length is part of the time.
+static __device__ __noinline__ void reinitialization_general(Ctx c, int ilimit) {
+    Win* s = c.s;
+    const double redtl = 0.5 * c.hf;
+    for (int i = c.blo + c.lane; i <= c.bhi; i += 32) s->alphio[i] = s->phi[i];
+    __syncwarp();
+    for (int it = 0; it < ilimit; ++it) {
+        for (int i = c.blo + c.lane; i <= c.bhi; i += 32) s->rk3[i] = s->phi[i];
+        __syncwarp();
+        reinit_rk3(c, redtl);
+        reinit_rk3(c, redtl);
+        for (int i = c.blo + c.lane; i <= c.bhi; i += 32) {
+            const int m = s->layer[i];
+            if (m >= 1 && m <= NN2) s->phi[i] = 0.75 * s->rk3[i] + 0.25 * s->phi[i];
+        }
+        __syncwarp();
+        reinit_rk3(c, redtl);
+        for (int i = c.blo + c.lane; i <= c.bhi; i += 32) {
+            const int m = s->layer[i];
+            if (m >= 1 && m <= NN2) s->phi[i] = 1.0 / 3.0 * s->rk3[i] + 2.0 / 3.0 * s->phi[i];
+        }
+        __syncwarp();
+    }
+}
+
 // REINITIALIZATION, two_phase.f:2033-2170: ILIMIT pseudo-time SSP-RK3 steps, dtau = h/2: WENO on
 // layers 1..NN1, first-order one-sided differences on NN1+1..NN2.  Ten iterations of the usual
-// band: 88 k cycles with ten dependent divisions and two roots a stage, NEW_REINIT k so.
+// band: 88 k cycles with ten dependent divisions and two roots a stage, 36 k so.
 __device__ inline void reinitialization(Ctx& c, int ilimit) {
     Win* s = c.s;
     const double redtl = 0.5 * c.hf;
@@ -511,10 +555,7 @@ __device__ inline void reinitialization(Ctx& c, int ilimit) {
                 bool ok = true;
                 compact_weno<false>(c, b, dm, dpl, ok);
                 double q = reinit_cell<false>(p, a0, dz, first_order ? fm : dm, first_order ? fp : dpl, eps, redtl, ok);
-                if (!__all_sync(0xffffffffu, ok)) {
-                    compact_weno<true>(c, b, dm, dpl, ok);
-                    q = reinit_cell<true>(p, a0, dz, first_order ? fm : dm, first_order ? fp : dpl, eps, redtl, ok);
-                }
+                if (!__all_sync(0xffffffffu, ok)) q = reinit_stage_plain(c.s, b.wi, first_order, c.ssdzf, p, a0, eps, redtl, b.i);
                 if (st == 1) q = 0.75 * rk + 0.25 * q;
                 if (st == 2) q = 1.0 / 3.0 * rk + 2.0 / 3.0 * q;
                 p = q;
@@ -525,25 +566,7 @@ __device__ inline void reinitialization(Ctx& c, int ilimit) {
         }
         return;
     }
-    for (int i = c.blo + c.lane; i <= c.bhi; i += 32) s->alphio[i] = s->phi[i];
-    __syncwarp();
-    for (int it = 0; it < ilimit; ++it) {
-        for (int i = c.blo + c.lane; i <= c.bhi; i += 32) s->rk3[i] = s->phi[i];
-        __syncwarp();
-        reinit_rk3(c, redtl);
-        reinit_rk3(c, redtl);
-        for (int i = c.blo + c.lane; i <= c.bhi; i += 32) {
-            const int m = s->layer[i];
-            if (m >= 1 && m <= NN2) s->phi[i] = 0.75 * s->rk3[i] + 0.25 * s->phi[i];
-        }
-        __syncwarp();
-        reinit_rk3(c, redtl);
-        for (int i = c.blo + c.lane; i <= c.bhi; i += 32) {
-            const int m = s->layer[i];
-            if (m >= 1 && m <= NN2) s->phi[i] = 1.0 / 3.0 * s->rk3[i] + 2.0 / 3.0 * s->phi[i];
-        }
-        __syncwarp();
-    }
+    reinitialization_general(c, ilimit);
 }
 
 // REIN_TRIGGER, two_phase.f:646-697: max and min of |grad phi| over layers 1..NN1.
@@ -665,11 +688,45 @@ __device__ inline void window_crossings(Ctx& c, int& ktop, int& kbot) {
     kbot = (top < 0) ? -1 : bot;
 }
 
+// v after d > 0 has been added to v >= 0 n times, one rounded addition after the other.  Inside
+// one binade of v every addition moves v by the same multiple of its unit, once two in a row
+// have (a tie settles after one), so the run to the end of the binade is one exact product;
+// the additions near a binade's ends, and all of them while v is below 32 d, are made singly.
+__device__ inline double add_repeated(double v, double d, int n) {
+    while (n > 0) {
+        if (n > 16 && v > 32.0 * d && v < 1e300) {
+            const double v1 = v + d, v2 = v1 + d;
+            const int e = __double2hiint(v) & 0x7ff00000;
+            const double top = __hiloint2double(e + 0x100000, 0);   // the next binade
+            if (v2 < top && v1 - v == v2 - v1) {
+                const double step = v2 - v1, left = floor((top - v2) / step) - 3.0;
+                if (left >= 1.0) {
+                    const double k = fmin(left, (double)(n - 2));
+                    v = v2 + k * step;
+                    n -= 2 + (int)k;
+                    continue;
+                }
+            }
+        }
+        if (n >= 8) {
+#pragma unroll
+            for (int q = 0; q < 8; ++q) v = v + d;
+            n -= 8;
+        } else {
+            v = v + d;
+            --n;
+        }
+    }
+    return v;
+}
+
 // Vapour volume of the whole column, sum over k = 1..nf of four replicas of
 // (1 - PSIF) * DVOL in the reference's order (two_phase.f:6230-6290), with PSIF = band_ps on
 // the window cells of layers 1..NN1 and the column fill elsewhere.  Outside the window the
 // fill is constant below and above it (the crossings lie inside), and adding 0.0 leaves
-// the sum unchanged, so only nonzero terms are added.  Lane 0 only.
+// the sum unchanged, so only nonzero terms are added; cells of one value in a row (the vapour
+// below the band) are added together (add_repeated).  Warp-wide, every lane gets the sum.
+// 512-cell column, film 0.1: 16.5 k cycles with one lane visiting the cells, 8 k so.
 __device__ inline double column_vapour_volume(Ctx& c, const double* band_ps, int ktop, int kbot, double dvol) {
     const Win* s = c.s;
     double t1 = 1.0, t2 = 1.0;
@@ -678,40 +735,44 @@ __device__ inline double column_vapour_volume(Ctx& c, const double* band_ps, int
         t2 = (c.p(kbot + 1) < 0.0) ? 0.0 : 1.0;
     }
     auto fill = [&](int k) { return (ktop < 0) ? 1.0 : ((k > kbot) ? t2 : t1); };
-    double vt = 0.0;
+    double vt = 0.0, run = 0.0;   // run: the value of the cells counted in cnt, not added yet
+    int cnt = 0;
+    auto add = [&](double d, int cells) {
+        if (d == 0.0 || cells <= 0) return;
+        if (cnt > 0 && d != run) {
+            vt = run > 0.0 ? add_repeated(vt, run, cnt) : vt;
+            cnt = 0;
+        }
+        if (d > 0.0) {
+            run = d;
+            cnt += 4 * cells;
+        } else {
+            for (int q = 0; q < 4 * cells; ++q) vt = vt + d;
+        }
+    };
     const int wlo = max(1, c.w0), whi = min(c.nf, c.w0 + WIN - 1);
-    // below the window
-    if (wlo > 1) {
-        const double d = (1.0 - fill(1)) * dvol;
-        if (d != 0.0)
-            for (int k = 1; k < wlo; ++k) {
-                vt = vt + d;
-                vt = vt + d;
-                vt = vt + d;
-                vt = vt + d;
-            }
-    }
-    for (int k = wlo; k <= whi; ++k) {
-        const int i = k - c.w0;
-        const double ps = (s->layer[i] >= 1 && s->layer[i] <= NN1) ? band_ps[i] : fill(k);
-        const double d = (1.0 - ps) * dvol;
-        if (d != 0.0) {
-            vt = vt + d;
-            vt = vt + d;
-            vt = vt + d;
-            vt = vt + d;
+    add((1.0 - fill(1)) * dvol, wlo - 1);   // below the window
+    for (int q = 0; q < PER; ++q) {
+        const int i = c.lane + 32 * q, k = c.w0 + i;
+        double d = 0.0;
+        if (k >= wlo && k <= whi) {
+            const double ps = (s->layer[i] >= 1 && s->layer[i] <= NN1) ? band_ps[i] : fill(k);
+            d = (1.0 - ps) * dvol;
+        }
+        unsigned some = __ballot_sync(0xffffffffu, d != 0.0);
+        while (some) {
+            // the lowest cell left, with the cells after it that have its value
+            const int b = __ffs(some) - 1;
+            const double db = __shfl_sync(0xffffffffu, d, b);
+            const unsigned same = __ballot_sync(0xffffffffu, d == db) & some;
+            const unsigned other = some & ~same & (0xffffffffu << b);
+            const unsigned take = other ? same & ((1u << (__ffs(other) - 1)) - 1u) : same;
+            add(db, take ? __popc(take) : 1);   // a NaN equals nothing, itself included
+            some &= take ? ~take : some - 1;
         }
     }
-    if (whi < c.nf) {
-        const double d = (1.0 - fill(c.nf)) * dvol;
-        if (d != 0.0)
-            for (int k = whi + 1; k <= c.nf; ++k) {
-                vt = vt + d;
-                vt = vt + d;
-                vt = vt + d;
-                vt = vt + d;
-            }
-    }
+    add((1.0 - fill(c.nf)) * dvol, c.nf - whi);   // above the window
+    if (cnt > 0) vt = add_repeated(vt, run, cnt);
     return vt;
 }
 
@@ -735,6 +796,7 @@ __device__ inline void global_mass_correction(Ctx& c, double& vol_tot_ori, doubl
         double vol_tot = 0.0;
         int ktop = -1, kbot = -1;
         if (l == 1) window_crossings(c, ktop, kbot);
+        if (l == 1) vol_tot = column_vapour_volume(c, s->nv, ktop, kbot, dvol);
         if (c.lane == 0) {
             double vol_band = 0.0;
             for (int j = s->lstart[1]; j < s->lstart[NN1 + 1]; ++j) {
@@ -744,12 +806,8 @@ __device__ inline void global_mass_correction(Ctx& c, double& vol_tot_ori, doubl
                 vol_band = vol_band + v;
                 vol_band = vol_band + v;
             }
-            if (l == 1) {
-                vol_tot = column_vapour_volume(c, s->nv, ktop, kbot, dvol);
-                vol_in = vol_tot - vol_band;
-            } else {
-                vol_tot = vol_in + vol_band;
-            }
+            if (l == 1) vol_in = vol_tot - vol_band;
+            else vol_tot = vol_in + vol_band;
         }
         vol_tot = __shfl_sync(0xffffffffu, vol_tot, 0);
         vol_in = __shfl_sync(0xffffffffu, vol_in, 0);
