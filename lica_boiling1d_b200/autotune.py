@@ -2,10 +2,9 @@
 
 The step kernel runs one CTA per column, persistent over all the steps of a launch.  The
 launch shape is the CTA width -- 32, 64, 128 or 256 threads -- which also fixes how many columns
-share an SM (the 32- and 64-thread forms are bounded for 8 and 5 CTAs per SM, the wider ones run one
-or two; a one-warp CTA runs TEMP_EXTP's two phases one after the other).  Results are identical;
-the speed is not: many short columns favour narrow CTAs and more columns per SM, a few long
-ones wide CTAs that finish each column sooner.
+share an SM (8, 4, 2 and 1; a one-warp CTA runs TEMP_EXTP's two phases one after the other).
+Results are identical; the speed is not: many short columns favour narrow CTAs and more columns
+per SM, a few long ones wide CTAs that finish each column sooner.
 
 ``tune(batch)`` times one warm-up step and ``trial_steps`` steps of each shape on a copy of
 the batch's device state (the batch itself does not advance), keeps the fastest, and

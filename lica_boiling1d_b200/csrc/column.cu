@@ -93,12 +93,13 @@ enum { PH_DT, PH_CONT, PH_ENERGY, PH_TEMPGRAD, PH_EXTP, PH_CONT2, PH_RHSZ, PH_LH
 struct Geo {
     int n, nf;
     double h, hf;
-    double ih, ihalf;   // 1/h (SSDZ, VVDZ inside) and 1/(h/2) (VVDZ at the walls), computed once
+    double ih, ihalf, ihf;   // 1/h (SSDZ, VVDZ inside), 1/(h/2) (VVDZ at the walls), 1/hf, computed once
     const col::ColGeoDev* cg;
     __device__ Geo(int n_, double L, const col::ColGeoDev* cg_ = nullptr)
         : n(n_), nf(2 * n_), h(L / n_), hf(L / (2 * n_)), cg(cg_) {
         ih = 1.0 / h;
         ihalf = 1.0 / (0.5 * h);
+        ihf = 1.0 / hf;
     }
     __device__ double sdz(int k) const { return cg ? cg->sdz[k] : ((k >= 1 && k <= n) ? h : 0.0); }
     __device__ double ssdz(int k) const { return cg ? cg->ssdz[k] : ih; }
@@ -608,7 +609,7 @@ __device__ void cal_continuity(const Geo& g, const Phys& ph, Col& c, double dtco
                         k1 = g.kcoump2(k);
                         k2 = g.kcoump1(k + 1);
                     }
-                    ps = col::box_mean(c.psif, nf, k1, k2, z1, z2, g.hf);
+                    ps = col::box_mean4(c.psif, nf, k1, k2, z1, z2, g.hf, g.ihf);
                 }
                 vzv[k] = ph.vism + (ph.visp - ph.vism) * ps;
                 vzd[k] = ph.denm + ph.den_diff * ps;
@@ -639,7 +640,7 @@ __device__ void cal_continuity(const Geo& g, const Phys& ph, Col& c, double dtco
                         k1 = g.kcou2(k + 1);
                         k2 = g.kcou1(k + 2);
                     }
-                    ps = col::box_mean(c.psif, nf, k1, k2, z1, z2, g.hf);
+                    ps = col::box_mean4(c.psif, nf, k1, k2, z1, z2, g.hf, g.ihf);
                 }
                 vcd[k] = ph.denm + ph.den_diff * ps;
             }
@@ -1307,21 +1308,15 @@ __device__ int temp_grad(const Geo& g, const Phys& ph, Col& c, Shared& sh, doubl
                 }
             }
             __syncwarp();
-            {
+            if (lane == 0) {
                 const int ktop = sh.ibuf[4], kbot = sh.ibuf[5];
-                double t1 = 1.0, t2 = 1.0;
+                sh.dbuf[2] = sh.dbuf[3] = 1.0;   // the fill below and above the crossing
                 if (ktop >= 0) {
-                    t1 = (cx.p(ktop) < 0.0) ? 0.0 : 1.0;
-                    t2 = (cx.p(kbot + 1) < 0.0) ? 0.0 : 1.0;
+                    sh.dbuf[2] = (cx.p(ktop) < 0.0) ? 0.0 : 1.0;
+                    sh.dbuf[3] = (cx.p(kbot + 1) < 0.0) ? 0.0 : 1.0;
                 }
-                for (int k = 1 + lane; k <= nf; k += 32) {
-                    const int i = k - cx.w0;
-                    double v;
-                    if (cx.in(k) && s->layer[i] >= 1 && s->layer[i] <= lvs::NN1) v = s->start[i];
-                    else if (ktop < 0) v = 1.0;
-                    else v = (k > kbot) ? t2 : t1;
-                    c.psif_mtp[k] = v;
-                }
+                sh.ibuf[6] = kbot;
+                sh.ibuf[7] = cx.w0;
             }
             __syncwarp();
             // VOL_TOT_MFDOT: trial advance of layers 1..NN1-2 by the mass flux, reinit,
@@ -1374,10 +1369,11 @@ __device__ int temp_grad(const Geo& g, const Phys& ph, Col& c, Shared& sh, doubl
             }
             for (int i = cx.blo + lane; i <= cx.bhi; i += 32) {
                 const int k = cx.w0 + i, m = s->layer[i];
-                if (m >= 1 && m <= lvs::NN1 - 2 && s->mf[i] != 0.0 && fabs(c.psif_mtp[k] - 0.5) != 0.5) {
-                    const double d = -(s->nv[i] - c.psif_mtp[k]);
+                const double mtp = s->start[i];   // PSIF_MTP of a cell of layers 1..NN1
+                if (m >= 1 && m <= lvs::NN1 - 2 && s->mf[i] != 0.0 && fabs(mtp - 0.5) != 0.5) {
+                    const double d = -(s->nv[i] - mtp);
                     if (s->wf[i] > 0.0) {
-                        c.sfgas[k] = -(s->nv[i] - c.psif_mtp[k]) * ph.denr;
+                        c.sfgas[k] = -(s->nv[i] - mtp) * ph.denr;
                         c.sfgas2[k] = d;
                     } else {
                         c.sfgas[k] = d;
@@ -1390,10 +1386,22 @@ __device__ int temp_grad(const Geo& g, const Phys& ph, Col& c, Shared& sh, doubl
     __syncthreads();
     const int iters = sh.ibuf[3];
     if (iters < 0) return iters == -1 ? -LICA_NOT_CONVERGED : iters;
+    // PSIF_MTP of the column: the band's values and the fill on either side of the crossing
+    {
+        const int kbot = sh.ibuf[6], w0 = sh.ibuf[7];
+        const double t1 = sh.dbuf[2], t2 = sh.dbuf[3];
+        FOR_K(1, nf) {
+            const int i = k - w0;
+            double v = k > kbot ? t2 : t1;
+            if (i >= 0 && i < lvs::WIN && s->layer[i] >= 1 && s->layer[i] <= lvs::NN1) v = s->start[i];
+            c.psif_mtp[k] = v;
+        }
+    }
+    __syncthreads();
     // (7) CAL_PSI_TMP(1) and IMASK_PH on the z faces (chphase.f:297-357)
     double* psi_tmp = c.a[S_PSITMP];
     FOR_K(1, n) {
-        const double v = col::box_mean(c.psif_mtp, nf, g.kcou2(k), g.kcou1(k + 1), g.z(k), g.z(k + 1), g.hf);
+        const double v = col::box_mean4(c.psif_mtp, nf, g.kcou2(k), g.kcou1(k + 1), g.z(k), g.z(k + 1), g.hf, g.ihf);
         psi_tmp[k] = (v <= 1e-3) ? 0.0 : (v >= 0.999 ? 1.0 : v);
     }
     __syncthreads();
@@ -1411,11 +1419,11 @@ __device__ void cal_continuity2(const Geo& g, const Phys& ph, Col& c) {
         if (k >= 2) {
             double v = psi_z[k];
             if (reg[k] == 2)
-                v = v - col::box_mean_sparse(c.sfgas2, nf, g.kcou2(k), g.kcou1(k + 1), g.zp(k - 1), g.zp(k), g.hf);
+                v = v - col::box_mean_sparse(c.sfgas2, nf, g.kcou2(k), g.kcou1(k + 1), g.zp(k - 1), g.zp(k), g.hf, g.ihf);
             psi_z[k] = (v > 1.0) ? 1.0 : (v < 0.0 ? 0.0 : v);
         }
         double v = psi_c[k];
-        if (reg[k] == 2) v = v - col::box_mean_sparse(c.sfgas2, nf, g.kcou2(k), g.kcou1(k + 1), g.z(k), g.z(k + 1), g.hf);
+        if (reg[k] == 2) v = v - col::box_mean_sparse(c.sfgas2, nf, g.kcou2(k), g.kcou1(k + 1), g.z(k), g.z(k + 1), g.hf, g.ihf);
         psi_c[k] = (v > 1.0) ? 1.0 : (v < 0.0 ? 0.0 : v);
     }
     __syncthreads();
@@ -1566,7 +1574,7 @@ __device__ void pressure_correction(const Geo& g, const Phys& ph, Col& c, Shared
         FOR_K(1, n) {
             double d = (k <= n - 1) ? (c.w[k + 1] - c.w[k]) * g.ssdz(k) : 0.0;
             if (ph.iphs == 1) {
-                const double ssum = col::box_mean_sparse(c.sfgas, g.nf, g.kcou2(k), g.kcou1(k + 1), g.z(k), g.z(k + 1), g.hf);
+                const double ssum = col::box_mean_sparse(c.sfgas, g.nf, g.kcou2(k), g.kcou1(k + 1), g.z(k), g.z(k + 1), g.hf, g.ihf);
                 d = d - ssum * (ph.den_diff / (ph.denp * ph.denm));
             }
             if (k >= 2) d = d * dtconsti;
@@ -1654,7 +1662,7 @@ __device__ int column_step(const Geo& g, const Phys& ph, Col& c, Shared& sh, dou
         FOR_K(1, n) {
             double d = (c.w[k + 1] - c.w[k]) * g.ssdz(k);
             if (ph.iphs == 1) {
-                const double ssum = col::box_mean_sparse(c.sfgas, g.nf, g.kcou2(k), g.kcou1(k + 1), g.z(k), g.z(k + 1), g.hf);
+                const double ssum = col::box_mean_sparse(c.sfgas, g.nf, g.kcou2(k), g.kcou1(k + 1), g.z(k), g.z(k + 1), g.hf, g.ihf);
                 d = d - ssum * (ph.den_diff / ph.denp);
             }
             dv = fmax(fabs(d), dv);
@@ -1685,14 +1693,22 @@ __device__ int column_step(const Geo& g, const Phys& ph, Col& c, Shared& sh, dou
         imass += sh.dbuf[2];
     }
     __syncthreads();
-    if (tid == 0) {
-        c.scal[1] = c.scal[1] + c.scal[0];
-        double zi = 0.0;
-        for (int k = 1; k < g.nf; ++k)
-            if (c.layer[k + 2] > 0 && c.layer[k + 3] > 0 && c.phi[k + 2] < 0.0 && c.phi[k + 3] >= 0.0) {
-                zi = g.zpf(k) - c.phi[k + 2] * (g.zpf(k + 1) - g.zpf(k)) / (c.phi[k + 3] - c.phi[k + 2]);
+    // the lowest crossing of the band, by warp 0: 32 refined cells at a time from the wall
+    double zi = 0.0;
+    if (warp == 0)
+        for (int k0 = 1; k0 < g.nf; k0 += 32) {
+            const int k = k0 + lane;
+            const bool here = k < g.nf && c.layer[k + 2] > 0 && c.layer[k + 3] > 0 && c.phi[k + 2] < 0.0 &&
+                              c.phi[k + 3] >= 0.0;
+            const unsigned b = __ballot_sync(0xffffffffu, here);
+            if (b) {
+                const int kc = k0 + __ffs(b) - 1;
+                zi = g.zpf(kc) - c.phi[kc + 2] * (g.zpf(kc + 1) - g.zpf(kc)) / (c.phi[kc + 3] - c.phi[kc + 2]);
                 break;
             }
+        }
+    if (tid == 0) {
+        c.scal[1] = c.scal[1] + c.scal[0];
         c.stats[1] = dvmax;
         c.stats[2] = iters;
         c.stats[3] = subcycles;
@@ -1708,9 +1724,10 @@ __device__ int column_step(const Geo& g, const Phys& ph, Col& c, Shared& sh, dou
 // NTH threads per column; one CTA per SM is enough for the register budget the sequential
 // parts want (no spills), more columns per SM come from smaller NTH.
 template <int NTH>
-// The 64-thread form is bounded for 5 CTAs per SM (about 200 registers): latency-bound
-// columns gain more from columns in flight than they lose to a few spilled registers.
-__global__ void __launch_bounds__(NTH, NTH == 32 ? 8 : (NTH == 64 ? 5 : 1)) k_column_steps(const __grid_constant__ Args A) {
+// The 64-thread form is bounded for 4 CTAs per SM, where it keeps its 252 registers: 4096 uneven
+// columns 9.5 ms a step, against 10.9 with 5 CTAs per SM (168 registers, some spilled) and 12.2
+// with 6.
+__global__ void __launch_bounds__(NTH, NTH == 32 ? 8 : (NTH == 64 ? 4 : 1)) k_column_steps(const __grid_constant__ Args A) {
     __shared__ Shared sh;
     if ((int)blockIdx.x >= A.ncol) return;
     const int col = A.order ? A.order[blockIdx.x] : (int)blockIdx.x;
@@ -2144,10 +2161,10 @@ bool state_ok(const lica_col_state* st) {
            st->mflvs && st->sfgas && st->sfgas2 && st->imask && st->scal && st->stats;
 }
 
-// The CTA width when the caller leaves it open: 256 threads while the batch has at most one
-// column per SM (each column is a latency chain, and a wider CTA finishes its phases sooner),
-// 64 beyond that (five columns per SM; on the 4096-column batch 64 threads take 25.6-25.8 ms
-// a step, 128 threads 38.7).
+// The CTA width when the caller leaves it open: as wide as lets every column run at once.  The
+// registers allow one 256-thread column per SM, two of 128 and four of 64.  512-cell columns, ms
+// a step with 256 / 128 / 64 threads: 148 columns 0.596 / 0.625 / 0.671, 149: 1.012 / 0.629 /
+// 0.669, 296: 1.176 / 0.671 / 0.715, 297: 1.488 / 1.123 / 0.740.
 int default_width(int ncol) {
     static int sms = 0;
     if (!sms) {
@@ -2156,7 +2173,7 @@ int default_width(int ncol) {
                                                       cudaSuccess || sms < 1)
             sms = 1;
     }
-    return ncol <= sms ? 256 : 64;
+    return ncol <= sms ? 256 : (ncol <= 2 * sms ? 128 : 64);
 }
 
 int launch_columns(const colk::Args& A, int threads, void* stream) {

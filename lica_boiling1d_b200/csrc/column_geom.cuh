@@ -76,14 +76,60 @@ static __device__ __noinline__ double box_mean(const double* f, int nf, int k1, 
     return sum / volf;
 }
 
+// The same where at most four refined cells meet the box, as a flow cell's or a swept face's do on
+// any grid here: each cell's term is formed once, in registers, and added once per replica (a
+// cell without a share adds 0).  ssdzf = 1 / hf.  About 900 cycles as the loop, 300 so.
+__device__ __forceinline__ double box_mean4(const double* f, int nf, int k1, int k2, double z1, double z2, double hf,
+                                            double ssdzf) {
+    if (k2 - k1 > 3) return box_mean(f, nf, k1, k2, z1, z2, hf);
+    double t[4], u[4];
+    bool open = true;
+#pragma unroll
+    for (int q = 0; q < 4; ++q) {
+        const int kk = min(k1 + q, k2);
+        const double v = f[kk < 1 ? 1 : (kk > nf ? nf : kk)];
+        const double za = grid_zf(hf, kk), zb = grid_zf(hf, kk + 1);
+        const bool here = open && k1 + q <= k2;
+        double share = 0.0;   // of the cell inside the box, in cells; whole cells keep v as it is
+        double term = 0.0;
+        if (za <= z1 && zb >= z2) {
+            share = 1.0;
+            term = v;
+            open = false;
+        } else if (za < z1 && zb > z1) {
+            share = (zb - z1) * ssdzf;
+            term = v * (zb - z1) * ssdzf;
+        } else if (za >= z1 && zb <= z2) {
+            share = 1.0;
+            term = v;
+        } else if (za < z2 && zb > z2) {
+            share = (z2 - za) * ssdzf;
+            term = v * (z2 - za) * ssdzf;
+        } else if (za >= z2) {
+            open = false;
+        }
+        t[q] = here ? term : 0.0;
+        u[q] = here ? share : 0.0;
+    }
+    double sum = 0.0, volf = 0.0;
+#pragma unroll
+    for (int rep = 0; rep < 4; ++rep)
+#pragma unroll
+        for (int q = 0; q < 4; ++q) {
+            sum = sum + t[q];
+            volf = volf + u[q];
+        }
+    return sum / volf;
+}
+
 // The same for fields that are zero away from the interface (SFGAS, SFGAS2): where every value
 // of the box is zero the mean is too, without the sums and divisions.  For boxes of some
 // extent inside the column, whose volume is not zero.
 __device__ __forceinline__ double box_mean_sparse(const double* f, int nf, int k1, int k2, double z1, double z2,
-                                                  double hf) {
+                                                  double hf, double ssdzf) {
     bool any = false;
     for (int kk = k1; kk <= k2; ++kk) any |= f[kk < 1 ? 1 : (kk > nf ? nf : kk)] != 0.0;
-    return any ? box_mean(f, nf, k1, k2, z1, z2, hf) : 0.0;
+    return any ? box_mean4(f, nf, k1, k2, z1, z2, hf, ssdzf) : 0.0;
 }
 
 }  // namespace col

@@ -138,13 +138,16 @@ __device__ inline void band_range(Ctx& c) {
 // column the same way)
 __device__ inline void build_lists(Ctx& c) {
     Win* s = c.s;
-    int pos = 0;
+    int pos = 0, lay[PER];
     const unsigned below = (1u << c.lane) - 1u;
+#pragma unroll
+    for (int q = 0; q < PER; ++q) lay[q] = s->layer[c.lane + 32 * q];
     for (int m = 1; m <= N_MAX; ++m) {
         if (c.lane == 0) s->lstart[m] = pos;
+#pragma unroll
         for (int q = 0; q < PER; ++q) {
             const int i = c.lane + 32 * q;
-            const bool pr = (s->layer[i] == m);
+            const bool pr = (lay[q] == m);
             const unsigned b = __ballot_sync(0xffffffffu, pr);
             if (pr) s->lst[pos + __popc(b & below)] = i;
             pos += __popc(b);
@@ -166,6 +169,31 @@ __device__ inline void lists_to_layer(Ctx& c) {
     band_range(c);
 }
 
+// First and last band cell of a column (k = -2..nf+4), eight loads of a lane in flight: one at a
+// time, the passes of one warp over a 512-cell column took 6 k cycles each.
+constexpr int AHEAD = 8;
+__device__ __forceinline__ void band_extent(const int* layer, int nf, int lane, int& kmin, int& kmax) {
+    kmin = 1 << 30;
+    kmax = -(1 << 30);
+    for (int kb = -2; kb <= nf + 4; kb += 32 * AHEAD) {
+        int m[AHEAD];
+#pragma unroll
+        for (int q = 0; q < AHEAD; ++q) {
+            const int k = kb + lane + 32 * q;
+            m[q] = (k <= nf + 4) ? layer[k + 2] : 0;
+        }
+#pragma unroll
+        for (int q = 0; q < AHEAD; ++q)
+            if (m[q] > 0) {
+                const int k = kb + lane + 32 * q;
+                kmin = min(kmin, k);
+                kmax = max(kmax, k);
+            }
+    }
+    kmin = __reduce_min_sync(0xffffffffu, kmin);
+    kmax = __reduce_max_sync(0xffffffffu, kmax);
+}
+
 // Window over the band of a column for work outside TRANSPORT (TEMP_GRAD): the same origin
 // rule as TRANSPORT, phi = band values and 0 elsewhere (ghosts included: TEMP_GRAD builds
 // ALPHI_EXT from the band alone, chphase.f:121-139), ascending band lists.  Returns
@@ -182,16 +210,8 @@ __device__ inline int load_band_window(Ctx& c, int lane, int n, double length, c
     c.ssdzf = 1.0 / c.hf;
     c.lane = lane;
     const int nf = c.nf;
-    int kmin = 1 << 30, kmax = -(1 << 30);
-    for (int k = -2 + lane; k <= nf + 4; k += 32)
-        if (layer[k + 2] > 0) {
-            kmin = min(kmin, k);
-            kmax = max(kmax, k);
-        }
-    for (int o = 16; o > 0; o >>= 1) {
-        kmin = min(kmin, __shfl_xor_sync(0xffffffffu, kmin, o));
-        kmax = max(kmax, __shfl_xor_sync(0xffffffffu, kmax, o));
-    }
+    int kmin, kmax;
+    band_extent(layer, nf, lane, kmin, kmax);
     if (kmax >= kmin && (kmin < 1 || kmax > nf)) return LICA_BAD_ARG;
     if (kmax >= kmin && kmax - kmin + 1 > WIN - 2 * HALO) return LICA_BAND_OVERFLOW;
     int w0 = (kmax >= kmin) ? (kmin + kmax + 1) / 2 - WIN / 2 : -2;
@@ -199,12 +219,20 @@ __device__ inline int load_band_window(Ctx& c, int lane, int n, double length, c
     w0 = min(w0, max(-2, nf + 4 - (WIN - 1)));
     c.w0 = w0;
     c.kw0 = flow_origin(c, w0);
+    int m[PER];
+    double p[PER];
+#pragma unroll
     for (int q = 0; q < PER; ++q) {
-        const int i = lane + 32 * q, k = w0 + i;
+        const int k = w0 + lane + 32 * q;
         const bool ok = (k >= -2 && k <= nf + 4);
-        const int m = ok ? layer[k + 2] : 0;
-        s->layer[i] = m;
-        s->phi[i] = (ok && (m > 0 || !band_only)) ? phi[k + 2] : 0.0;
+        m[q] = ok ? layer[k + 2] : 0;
+        p[q] = ok ? phi[k + 2] : 0.0;
+    }
+#pragma unroll
+    for (int q = 0; q < PER; ++q) {
+        const int i = lane + 32 * q;
+        s->layer[i] = m[q];
+        s->phi[i] = (m[q] > 0 || !band_only) ? p[q] : 0.0;
     }
     __syncwarp();
     build_lists(c);
@@ -632,10 +660,19 @@ __device__ inline int vel_intp(Ctx& c) {
             if (kk == n - 1) { z3 = z2 + vdz(kk + 1); z4 = z3 + 2.0 * vdz(n + 1); }
             else if (kk == n) { z3 = z2 + 2.0 * vdz(n + 1); z4 = z3 + vdz(n); }
             else { z3 = z2 + vdz(kk + 1); z4 = z3 + vdz(kk + 2); }
-            const double cz1 = ((zz - z2) * (zz - z3) * (zz - z4)) / ((z1 - z2) * (z1 - z3) * (z1 - z4));
-            const double cz2 = ((zz - z1) * (zz - z3) * (zz - z4)) / ((z2 - z1) * (z2 - z3) * (z2 - z4));
-            const double cz3 = ((zz - z1) * (zz - z2) * (zz - z4)) / ((z3 - z1) * (z3 - z2) * (z3 - z4));
-            const double cz4 = ((zz - z1) * (zz - z2) * (zz - z3)) / ((z4 - z1) * (z4 - z2) * (z4 - z3));
+            const double n1 = (zz - z2) * (zz - z3) * (zz - z4), d1 = (z1 - z2) * (z1 - z3) * (z1 - z4);
+            const double n2 = (zz - z1) * (zz - z3) * (zz - z4), d2 = (z2 - z1) * (z2 - z3) * (z2 - z4);
+            const double n3 = (zz - z1) * (zz - z2) * (zz - z4), d3 = (z3 - z1) * (z3 - z2) * (z3 - z4);
+            const double n4 = (zz - z1) * (zz - z2) * (zz - z3), d4 = (z4 - z1) * (z4 - z2) * (z4 - z3);
+            double cz1 = rn::quot(n1, d1, rn::recip(d1)), cz2 = rn::quot(n2, d2, rn::recip(d2)),
+                   cz3 = rn::quot(n3, d3, rn::recip(d3)), cz4 = rn::quot(n4, d4, rn::recip(d4));
+            auto fine = [](double a, double b) { return (a == 0.0 || rn::ordinary(a)) && rn::ordinary(b); };
+            if (!(fine(n1, d1) && fine(n2, d2) && fine(n3, d3) && fine(n4, d4))) {
+                cz1 = n1 / d1;
+                cz2 = n2 / d2;
+                cz3 = n3 / d3;
+                cz4 = n4 / d4;
+            }
             const double w = cz1 * wtv(kk - 1) + cz2 * wtv(kk) + cz3 * wtv(kk + 1) + cz4 * wtv(kk + 2);
             out = (m < NN2 - 1) ? w : w * 0.5;
         }
@@ -850,16 +887,8 @@ __device__ inline int transport_column(Win* s, int lane, int n, double length, d
     // band extent -> window origin (the band is centred; the window is clamped to the column).
     // Band cells live on k = 1..nf (BAND_GENERATION never goes past k = 1 or nf); a band
     // cell elsewhere is rejected, which keeps every stencil inside the window.
-    int kmin = 1 << 30, kmax = -(1 << 30);
-    for (int k = -2 + lane; k <= nf + 4; k += 32)
-        if (layer[k + 2] > 0) {
-            kmin = min(kmin, k);
-            kmax = max(kmax, k);
-        }
-    for (int o = 16; o > 0; o >>= 1) {
-        kmin = min(kmin, __shfl_xor_sync(0xffffffffu, kmin, o));
-        kmax = max(kmax, __shfl_xor_sync(0xffffffffu, kmax, o));
-    }
+    int kmin, kmax;
+    band_extent(layer, nf, lane, kmin, kmax);
     if (kmax >= kmin && (kmin < 1 || kmax > nf)) return LICA_BAD_ARG;
     if (kmax >= kmin && kmax - kmin + 1 > WIN - 2 * HALO) return LICA_BAND_OVERFLOW;
     int w0 = (kmax >= kmin) ? (kmin + kmax + 1) / 2 - WIN / 2 : -2;
@@ -870,15 +899,25 @@ __device__ inline int transport_column(Win* s, int lane, int n, double length, d
 
     // ALPHI_EXT = 0 outside the band, band phi inside (:750-767); ALPHI at entry for the
     // phase test of the source
-    for (int q = 0; q < PER; ++q) {
-        const int i = lane + 32 * q, k = w0 + i;
-        const bool ok = (k >= -2 && k <= nf + 4);
-        const int m = ok ? layer[k + 2] : 0;
-        s->layer[i] = m;
-        s->phi[i] = (ok && m > 0) ? phi[k + 2] : 0.0;
-        s->start[i] = s->phi[i];
-        s->mf[i] = ok ? mf[k + 2] : 0.0;
-        s->wf[i] = 0.0;
+    {
+        int m[PER];
+        double p[PER], f[PER];
+#pragma unroll
+        for (int q = 0; q < PER; ++q) {
+            const int k = w0 + lane + 32 * q;
+            const bool ok = (k >= -2 && k <= nf + 4);
+            m[q] = ok ? layer[k + 2] : 0;
+            p[q] = ok ? phi[k + 2] : 0.0;
+            f[q] = ok ? mf[k + 2] : 0.0;
+        }
+#pragma unroll
+        for (int q = 0; q < PER; ++q) {
+            const int i = lane + 32 * q;
+            s->layer[i] = m[q];
+            s->phi[i] = s->start[i] = m[q] > 0 ? p[q] : 0.0;
+            s->mf[i] = f[q];
+            s->wf[i] = 0.0;
+        }
     }
     if (lane < 7) s->ghost[lane] = 0.0;
     // VEL_INTP(2): UT = (U + UO)/2 with UO = U on the first call (:5567-5600); UO = U after
@@ -949,37 +988,64 @@ __device__ inline int transport_column(Win* s, int lane, int n, double length, d
 
     if (!skipped) {
         // CAL_PSIF(0): PSIF = CAL_PSIF_MTP on layers 1..NN1, then the snap of the whole
-        // array (:2600-2680)
-        for (int k = 1 + lane; k <= nf; k += 32) {
-            const int i = k - w0;
-            double v;
-            if (c.in(k) && s->layer[i] >= 1 && s->layer[i] <= NN1) {
-                v = psif_band(s, i);
-            } else {
-                v = psif[k];
-                if (v < 1e-5) v = 0.0;
-                else if (v > 0.99999) v = 1.0;
+        // array (:2600-2680), which away from the interface mostly changes nothing: only what it
+        // changes is written
+        for (int kb = 1; kb <= nf; kb += 32 * AHEAD) {
+            double v[AHEAD];
+#pragma unroll
+            for (int q = 0; q < AHEAD; ++q) {
+                const int k = kb + lane + 32 * q;
+                v[q] = (k <= nf) ? psif[k] : 0.0;
             }
-            psif[k] = v;
+#pragma unroll
+            for (int q = 0; q < AHEAD; ++q) {
+                const int k = kb + lane + 32 * q;
+                if (v[q] < 1e-5 && v[q] != 0.0 && k <= nf) psif[k] = 0.0;
+                else if (v[q] > 0.99999 && v[q] != 1.0 && k <= nf) psif[k] = 1.0;
+            }
+        }
+        __syncwarp();
+        for (int i = c.blo + lane; i <= c.bhi; i += 32) {
+            const int k = w0 + i, m = s->layer[i];
+            if (m >= 1 && m <= NN1 && k >= 1 && k <= nf) psif[k] = psif_band(s, i);
         }
         if (imass == 0 && P.iphs == 1) vo = vol_iphs;
     }
     // band phi and layers stored (ALPHI = ALPHI_EXT on the band); zero elsewhere except
     // the ghosts ALPHI_BC set
-    for (int k = -2 + lane; k <= nf + 4; k += 32) {
-        double v;
-        int m;
-        if (c.in(k)) {
-            v = s->phi[k - w0];
-            m = s->layer[k - w0];
-        } else {
-            m = 0;
-            v = (k <= 0) ? s->ghost[k + 2] : (k >= nf + 1 ? s->ghost[k - nf + 2] : 0.0);
+    for (int k = 1 + lane; k <= nf; k += 32)
+        if (!c.in(k)) {
+            phi[k + 2] = 0.0;
+            layer[k + 2] = 0;
         }
-        phi[k + 2] = v;
-        layer[k + 2] = m;
+    if (lane < 7) {
+        const int k = lane < 3 ? lane - 2 : nf + lane - 2;
+        if (!c.in(k)) {
+            phi[k + 2] = s->ghost[lane];
+            layer[k + 2] = 0;
+        }
     }
-    for (int k = lane; k <= n + 1; k += 32) wo[k] = w[k];
+#pragma unroll
+    for (int q = 0; q < PER; ++q) {
+        const int i = lane + 32 * q, k = w0 + i;
+        if (k >= -2 && k <= nf + 4) {
+            phi[k + 2] = s->phi[i];
+            layer[k + 2] = s->layer[i];
+        }
+    }
+    for (int kb = 0; kb <= n + 1; kb += 32 * AHEAD) {
+        double v[AHEAD];
+#pragma unroll
+        for (int q = 0; q < AHEAD; ++q) {
+            const int k = kb + lane + 32 * q;
+            v[q] = (k <= n + 1) ? w[k] : 0.0;
+        }
+#pragma unroll
+        for (int q = 0; q < AHEAD; ++q) {
+            const int k = kb + lane + 32 * q;
+            if (k <= n + 1) wo[k] = v[q];
+        }
+    }
     if (skipped) {
         if (lane == 0) {
             *vol_ori = vo;
@@ -1002,28 +1068,52 @@ __device__ inline int transport_column(Win* s, int lane, int n, double length, d
         }
     }
     __syncwarp();
-    for (int kk = 1 + lane; kk <= n; kk += 32) {
-        const int j = kk - c.kw0;
-        const bool mk = (j >= 0 && j < WTN) && s->fmask[j] != 0;
-        double zn = psi_zn[kk];
+    // the flow cells of the mask, in rising order, take a lane for each of their two means
+    int cells = 0;
+    for (int j0 = 0; j0 < WTN; j0 += 32) {
+        const int j = j0 + lane, kk = c.kw0 + j;
+        const bool mk = j < WTN && kk >= 1 && kk <= n && s->fmask[j] != 0;
+        const unsigned b = __ballot_sync(0xffffffffu, mk);
+        if (mk) s->lst2[cells + __popc(b & ((1u << lane) - 1u))] = kk;
+        cells += __popc(b);
+    }
+    __syncwarp();
+    auto snapped = [](double v) { return v < 1e-3 ? 0.0 : (v > 0.999 ? 1.0 : v); };
+    for (int it = lane; it < 2 * cells; it += 32) {
+        const int kk = s->lst2[it >> 1];
         const col::ColGeoDev* cg = c.cg;
-        // INTER_PSI over the face box [ZP(K-1), ZP(K)], refined cells KCOUMP2(K-1)..KCOUMP1(K)
-        if (kk >= 2 && mk)
-            zn = col::box_mean(psif, nf, cg ? cg->kcoump2[kk] : 2 * kk - 2, cg ? cg->kcoump1[kk + 1] : 2 * kk - 1,
-                               cg ? cg->zp[kk - 1] : col::grid_zp(c.h, n, kk - 1),
-                               cg ? cg->zp[kk] : col::grid_zp(c.h, n, kk), c.hf);
-        if (zn < 1e-3) zn = 0.0;
-        else if (zn > 0.999) zn = 1.0;
-        psi_zn[kk] = zn;
-        double cn = psi_cn[kk];
-        // over the cell box [Z(K), Z(K+1)], refined cells KCOU2(K)..KCOU1(K+1)
-        if (mk)
-            cn = col::box_mean(psif, nf, cg ? cg->kcou2[kk + 1] : 2 * kk - 1, cg ? cg->kcou1[kk + 2] : 2 * kk,
-                               cg ? cg->z[kk] : col::grid_z(c.h, kk), cg ? cg->z[kk + 1] : col::grid_z(c.h, kk + 1),
-                               c.hf);
-        if (cn < 1e-3) cn = 0.0;
-        else if (cn > 0.999) cn = 1.0;
-        psi_cn[kk] = cn;
+        if (it & 1) {
+            // INTER_PSI over the face box [ZP(K-1), ZP(K)], refined cells KCOUMP2(K-1)..KCOUMP1(K)
+            double zn = psi_zn[kk];
+            if (kk >= 2)
+                zn = col::box_mean4(psif, nf, cg ? cg->kcoump2[kk] : 2 * kk - 2, cg ? cg->kcoump1[kk + 1] : 2 * kk - 1,
+                                    cg ? cg->zp[kk - 1] : col::grid_zp(c.h, n, kk - 1),
+                                    cg ? cg->zp[kk] : col::grid_zp(c.h, n, kk), c.hf, c.ssdzf);
+            psi_zn[kk] = snapped(zn);
+        } else {
+            // over the cell box [Z(K), Z(K+1)], refined cells KCOU2(K)..KCOU1(K+1)
+            psi_cn[kk] = snapped(col::box_mean4(psif, nf, cg ? cg->kcou2[kk + 1] : 2 * kk - 1,
+                                                cg ? cg->kcou1[kk + 2] : 2 * kk, cg ? cg->z[kk] : col::grid_z(c.h, kk),
+                                                cg ? cg->z[kk + 1] : col::grid_z(c.h, kk + 1), c.hf, c.ssdzf));
+        }
+    }
+    __syncwarp();
+    // the snap of the others, written where it changes something (it leaves the means above)
+    for (int kb = 1; kb <= n; kb += 32 * AHEAD) {
+        double zn[AHEAD], cn[AHEAD];
+#pragma unroll
+        for (int q = 0; q < AHEAD; ++q) {
+            const int k = kb + lane + 32 * q;
+            zn[q] = (k <= n) ? psi_zn[k] : 0.0;
+            cn[q] = (k <= n) ? psi_cn[k] : 0.0;
+        }
+#pragma unroll
+        for (int q = 0; q < AHEAD; ++q) {
+            const int k = kb + lane + 32 * q;
+            const double z = snapped(zn[q]), v = snapped(cn[q]);
+            if (k <= n && z != zn[q]) psi_zn[k] = z;
+            if (k <= n && v != cn[q]) psi_cn[k] = v;
+        }
     }
     __syncwarp();
     if (lane == 0) {
