@@ -11,6 +11,7 @@
 
 #include "common.cuh"
 #include "unet_conv.cuh"
+#include "unet_wgrad.cuh"
 
 extern "C" void lica_count_launches(int64_t n);
 
@@ -356,24 +357,52 @@ __global__ void k_up(const bf16* __restrict__ in, bf16* __restrict__ out, int ni
     }
 }
 
-__global__ void k_head_bwd(const float* __restrict__ gout, const float* __restrict__ wh, bf16* __restrict__ g,
-                           size_t total) {
-    for (size_t p = blockIdx.x * (size_t)blockDim.x + threadIdx.x; p < total; p += (size_t)gridDim.x * blockDim.x)
-        for (int c = 0; c < kHead; ++c) g[p * kHead + c] = __float2bfloat16_rn(gout[p] * wh[c]);
+__device__ __forceinline__ float bf_lo(uint32_t u) { return __uint_as_float(u << 16); }
+__device__ __forceinline__ float bf_hi(uint32_t u) { return __uint_as_float(u & 0xffff0000u); }
+__device__ __forceinline__ uint32_t bf_pack(float lo, float hi) {
+    const __nv_bfloat162 b = __floats2bfloat162_rn(lo, hi);
+    return *reinterpret_cast<const uint32_t*>(&b);
+}
+// the gradients v of eight channels where the layer's output y is positive, in BF16
+__device__ __forceinline__ uint4 relu_mask8(const float* v, const uint4 y) {
+    const uint32_t u[4] = {y.x, y.y, y.z, y.w};
+    uint32_t r[4];
+#pragma unroll
+    for (int q = 0; q < 4; ++q)
+        r[q] = bf_pack(bf_lo(u[q]) > 0.f ? v[2 * q] : 0.f, bf_hi(u[q]) > 0.f ? v[2 * q + 1] : 0.f);
+    return make_uint4(r[0], r[1], r[2], r[3]);
 }
 
-// Per-block partial sums of the head's gradients: part[b][c] = sum gout*d1b[:, c] (c < 32),
-// part[b][32] = sum gout, over the pixels of block b (fixed order).
-__global__ void k_head_grad_part(const float* __restrict__ gout, const bf16* __restrict__ d, float* __restrict__ part,
-                                 size_t total) {
+// The head's backward pass, one sweep over d1b (d) and gout: per-block partial sums of its
+// gradients, part[b][c] = sum gout * d1b[:, c] (c < 32), part[b][32] = sum gout, over the pixels of
+// block b (fixed order), and dz = gout * wh through the last layer's ReLU.
+__global__ void k_head_bwd(const float* __restrict__ gout, const float* __restrict__ wh, const bf16* __restrict__ d,
+                           bf16* __restrict__ dz, float* __restrict__ part, size_t total) {
     __shared__ float red[kNT / 32][kHead + 1];
+    __shared__ float w[kHead];
+    if (threadIdx.x < kHead) w[threadIdx.x] = wh[threadIdx.x];
+    __syncthreads();
     float acc[kHead + 1];
 #pragma unroll
     for (int c = 0; c <= kHead; ++c) acc[c] = 0.f;
     for (size_t p = blockIdx.x * (size_t)blockDim.x + threadIdx.x; p < total; p += (size_t)gridDim.x * blockDim.x) {
         const float g = gout[p];
+        const uint4* src = reinterpret_cast<const uint4*>(d + p * kHead);
+        uint4* dst = reinterpret_cast<uint4*>(dz + p * kHead);
 #pragma unroll
-        for (int c = 0; c < kHead; ++c) acc[c] += g * __bfloat162float(d[p * kHead + c]);
+        for (int q = 0; q < 4; ++q) {
+            const uint4 y = src[q];
+            const uint32_t u[4] = {y.x, y.y, y.z, y.w};
+            float v[8];
+#pragma unroll
+            for (int i = 0; i < 4; ++i) {
+                acc[8 * q + 2 * i] += g * bf_lo(u[i]);
+                acc[8 * q + 2 * i + 1] += g * bf_hi(u[i]);
+            }
+#pragma unroll
+            for (int i = 0; i < 8; ++i) v[i] = g * w[8 * q + i];
+            dst[q] = relu_mask8(v, y);
+        }
         acc[kHead] += g;
     }
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
@@ -386,116 +415,109 @@ __global__ void k_head_grad_part(const float* __restrict__ gout, const bf16* __r
     __syncthreads();
     if (threadIdx.x <= kHead) {
         float v = 0.f;
-        for (int w = 0; w < kNT / 32; ++w) v += red[w][threadIdx.x];
+        for (int w_ = 0; w_ < kNT / 32; ++w_) v += red[w_][threadIdx.x];
         part[(size_t)blockIdx.x * (kHead + 1) + threadIdx.x] = v;
     }
 }
 
-// dz = g * (y > 0), g read as a channel slice [g_c0, g_c0 + c) of a tensor with g_cs channels,
-// plus (optionally) 0.25 * gp at the parent cell of a half-size tensor (pool backward).
+// dz = g through the layer's ReLU (y > 0), eight channels a thread; g = the channel slice
+// [g_c0, g_c0 + c) of a tensor with g_cs channels, plus (optionally) 0.25 * gp at the parent cell
+// of a half-size tensor (pool backward).  H and W are the image's, c a multiple of 8.
 __global__ void k_relu_bwd(const bf16* __restrict__ g, int g_cs, int g_c0, const bf16* __restrict__ gp,
                            const bf16* __restrict__ y, bf16* __restrict__ dz, int nimg, int H, int W, int c) {
-    const size_t total = (size_t)nimg * H * W * c;
+    const int c8 = c / 8;
+    const size_t total = (size_t)nimg * H * W * c8;
     for (size_t q = blockIdx.x * (size_t)blockDim.x + threadIdx.x; q < total; q += (size_t)gridDim.x * blockDim.x) {
-        const int ch = (int)(q % c);
-        const size_t pix = q / c;
-        float v = g ? __bfloat162float(g[pix * g_cs + g_c0 + ch]) : 0.f;
+        const int ch = (int)(q % c8) * 8;
+        const size_t pix = q / c8;
+        const uint4 gv = *reinterpret_cast<const uint4*>(g + pix * g_cs + g_c0 + ch);
+        const uint32_t u[4] = {gv.x, gv.y, gv.z, gv.w};
+        float v[8];
+#pragma unroll
+        for (int i = 0; i < 4; ++i) {
+            v[2 * i] = bf_lo(u[i]);
+            v[2 * i + 1] = bf_hi(u[i]);
+        }
         if (gp) {
             const int x = (int)(pix % W);
             const size_t r = pix / W;
             const int yy = (int)(r % H);
             const int img = (int)(r / H);
-            v += 0.25f * __bfloat162float(gp[(((size_t)img * (H / 2) + yy / 2) * (W / 2) + x / 2) * c + ch]);
+            const uint4 pv = *reinterpret_cast<const uint4*>(
+                gp + (((size_t)img * (H / 2) + yy / 2) * (W / 2) + x / 2) * c + ch);
+            const uint32_t w[4] = {pv.x, pv.y, pv.z, pv.w};
+#pragma unroll
+            for (int i = 0; i < 4; ++i) {
+                v[2 * i] += 0.25f * bf_lo(w[i]);
+                v[2 * i + 1] += 0.25f * bf_hi(w[i]);
+            }
         }
-        dz[q] = __bfloat162float(y[q]) > 0.f ? __float2bfloat16_rn(v) : __float2bfloat16_rn(0.f);
+        *reinterpret_cast<uint4*>(dz + pix * c + ch) =
+            relu_mask8(v, *reinterpret_cast<const uint4*>(y + pix * c + ch));
     }
 }
 
-// upsampling backward: out[n, Y, X, c] = sum of the 4 children of g (channel slice [g_c0, g_c0 + c)).
-__global__ void k_up_bwd(const bf16* __restrict__ g, int g_cs, int g_c0, bf16* __restrict__ out, int nimg, int Ho,
-                         int Wo, int c) {
-    const size_t total = (size_t)nimg * Ho * Wo * c;
-    const int W = 2 * Wo;
+// Upsampling backward and the layer's ReLU: dz[n, Y, X, c] = the sum of the 4 children of g
+// (channel slice [g_c0, g_c0 + c) of a tensor with g_cs channels), rounded to BF16, where y > 0.
+__global__ void k_up_relu_bwd(const bf16* __restrict__ g, int g_cs, int g_c0, const bf16* __restrict__ y,
+                              bf16* __restrict__ dz, int nimg, int Ho, int Wo, int c) {
+    const int c8 = c / 8, W = 2 * Wo;
+    const size_t total = (size_t)nimg * Ho * Wo * c8;
     for (size_t q = blockIdx.x * (size_t)blockDim.x + threadIdx.x; q < total; q += (size_t)gridDim.x * blockDim.x) {
-        const int ch = (int)(q % c);
-        size_t r = q / c;
-        const int X = (int)(r % Wo);
-        r /= Wo;
+        const int ch = (int)(q % c8) * 8;
+        const size_t pix = q / c8;
+        const int X = (int)(pix % Wo);
+        const size_t r = pix / Wo;
         const int Y = (int)(r % Ho);
         const int img = (int)(r / Ho);
-        const size_t b = (((size_t)img * 2 * Ho + 2 * Y) * W + 2 * X) * g_cs + g_c0 + ch;
-        const float s = (__bfloat162float(g[b]) + __bfloat162float(g[b + g_cs])) +
-                        (__bfloat162float(g[b + (size_t)W * g_cs]) + __bfloat162float(g[b + (size_t)W * g_cs + g_cs]));
-        out[q] = __float2bfloat16_rn(s);
-    }
-}
-
-// Weight gradient of a 3x3 convolution, per pixel chunk:
-//   part[chunk][co][tap][ci] = sum_{p in chunk} dz[p, co] * x[p + off(tap), ci]
-// (x = [x0, x1] along channels, zero outside the image), and bpart[chunk][co] = sum dz.
-// Block: one tap, a 32 x 32 (co, ci) block; 256 threads, 4 outputs each, 32-pixel stages.
-constexpr int kDwChunk = 2048;
-__global__ void __launch_bounds__(kNT) k_dw_part(const bf16* __restrict__ dz, int cout, const bf16* __restrict__ x0,
-                                                 int c0, const bf16* __restrict__ x1, int c1, int nimg, int H, int W,
-                                                 float* __restrict__ part, float* __restrict__ bpart) {
-    __shared__ float sd[32][33];
-    __shared__ float sx[32][33];
-    const int ctot = c0 + c1;
-    const int tap = blockIdx.y, dy = tap / 3 - 1, dx = tap % 3 - 1;
-    const int cob = blockIdx.z % (cout / 32), cib = blockIdx.z / (cout / 32);  // ci blocks of 32 (last one partial)
-    const int chunk = blockIdx.x;
-    const size_t npix = (size_t)nimg * H * W;
-    const size_t p0 = (size_t)chunk * kDwChunk, p1 = min(npix, p0 + kDwChunk);
-    const int t = threadIdx.x, co = t >> 3, ci4 = (t & 7) * 4;
-    float acc[4] = {0.f, 0.f, 0.f, 0.f};
-    float bacc = 0.f;
-    for (size_t pb = p0; pb < p1; pb += 32) {
-        // stage dz[32 px][32 co] and x[32 px][32 ci] (4 values per thread each)
-        for (int e = t; e < 32 * 32; e += kNT) {
-            const int pi = e >> 5, cc = e & 31;
-            const size_t p = pb + pi;
-            float vd = 0.f, vx = 0.f;
-            if (p < p1) {
-                vd = __bfloat162float(dz[p * cout + cob * 32 + cc]);
-                const int xx = (int)(p % W);
-                const size_t r = p / W;
-                const int yy = (int)(r % H);
-                const int sx_ = xx + dx, sy_ = yy + dy;
-                const int ci = cib * 32 + cc;
-                if (ci < ctot && sx_ >= 0 && sx_ < W && sy_ >= 0 && sy_ < H) {
-                    const size_t q = p + (ptrdiff_t)dy * W + dx;
-                    vx = ci < c0 ? __bfloat162float(x0[q * c0 + ci]) : __bfloat162float(x1[q * c1 + (ci - c0)]);
-                }
-            }
-            sd[pi][cc] = vd;
-            sx[pi][cc] = vx;
-        }
-        __syncthreads();
-#pragma unroll 8
-        for (int pi = 0; pi < 32; ++pi) {
-            const float a = sd[pi][co];
-            acc[0] += a * sx[pi][ci4];
-            acc[1] += a * sx[pi][ci4 + 1];
-            acc[2] += a * sx[pi][ci4 + 2];
-            acc[3] += a * sx[pi][ci4 + 3];
-            if (tap == 0 && cib == 0 && (t & 7) == 0) bacc += a;
-        }
-        __syncthreads();
-    }
-    float* dst = part + (size_t)chunk * cout * 9 * ctot;
+        const bf16* b = g + (((size_t)img * 2 * Ho + 2 * Y) * W + 2 * X) * g_cs + g_c0 + ch;
+        const uint4 c00 = *reinterpret_cast<const uint4*>(b), c01 = *reinterpret_cast<const uint4*>(b + g_cs),
+                    c10 = *reinterpret_cast<const uint4*>(b + (size_t)W * g_cs),
+                    c11 = *reinterpret_cast<const uint4*>(b + (size_t)W * g_cs + g_cs);
+        const uint32_t p[4] = {c00.x, c00.y, c00.z, c00.w}, s[4] = {c01.x, c01.y, c01.z, c01.w},
+                       t[4] = {c10.x, c10.y, c10.z, c10.w}, u[4] = {c11.x, c11.y, c11.z, c11.w};
+        float v[8];
 #pragma unroll
-    for (int j = 0; j < 4; ++j)
-        if (cib * 32 + ci4 + j < ctot) dst[((size_t)(cob * 32 + co) * 9 + tap) * ctot + cib * 32 + ci4 + j] = acc[j];
-    if (tap == 0 && cib == 0 && (t & 7) == 0) bpart[(size_t)chunk * cout + cob * 32 + co] = bacc;
+        for (int i = 0; i < 4; ++i) {
+            v[2 * i] = (bf_lo(p[i]) + bf_lo(s[i])) + (bf_lo(t[i]) + bf_lo(u[i]));
+            v[2 * i + 1] = (bf_hi(p[i]) + bf_hi(s[i])) + (bf_hi(t[i]) + bf_hi(u[i]));
+        }
+        *reinterpret_cast<uint4*>(dz + pix * c + ch) =
+            relu_mask8(v, *reinterpret_cast<const uint4*>(y + pix * c + ch));
+    }
 }
 
-// grad[k] = sum over chunks of part[chunk][k] (chunk order), for k < n.
-__global__ void k_sum_parts(const float* __restrict__ part, int nchunk, size_t n, float* __restrict__ grad) {
-    for (size_t k = blockIdx.x * (size_t)blockDim.x + threadIdx.x; k < n; k += (size_t)gridDim.x * blockDim.x) {
-        float s = 0.f;
-        for (int c = 0; c < nchunk; ++c) s += part[(size_t)c * n + k];
-        grad[k] = s;
+// grad[k] = sum over chunks of part[chunk][k], for k < n, and the same of a second set (bpart, nb
+// values to bgrad, may be empty): 8 threads per value take every 8th chunk, then add up in a
+// fixed order.  Block: 32 values x 8 threads.
+__global__ void __launch_bounds__(256) k_sum_parts(const float* __restrict__ part, int nchunk, size_t n,
+                                                   float* __restrict__ grad, const float* __restrict__ bpart, size_t nb,
+                                                   float* __restrict__ bgrad) {
+    __shared__ float red[8][33];
+    const int x = threadIdx.x & 31, y = threadIdx.x >> 5;
+    const size_t blocks = (n + 31) / 32;
+    const bool second = blockIdx.x >= blocks;
+    const float* src = second ? bpart : part;
+    const size_t len = second ? nb : n, k = (blockIdx.x - (second ? blocks : 0)) * 32 + x;
+    float s = 0.f;
+    if (k < len) {
+#pragma unroll 4
+        for (int c = y; c < nchunk; c += 8) s += src[(size_t)c * len + k];
     }
+    red[y][x] = s;
+    __syncthreads();
+    if (y == 0 && k < len) {
+        const float v = ((red[0][x] + red[1][x]) + (red[2][x] + red[3][x])) +
+                        ((red[4][x] + red[5][x]) + (red[6][x] + red[7][x]));
+        (second ? bgrad : grad)[k] = v;
+    }
+}
+int sum_parts(const float* part, int nchunk, size_t n, float* grad, const float* bpart, size_t nb, float* bgrad,
+              cudaStream_t s) {
+    k_sum_parts<<<(unsigned)((n + 31) / 32 + (nb + 31) / 32), 256, 0, s>>>(part, nchunk, n, grad, bpart, nb, bgrad);
+    LICA_CUDA_TRY(cudaGetLastError());
+    lica_count_launches(1);
+    return LICA_OK;
 }
 
 // Adam (FP32 master weights).
@@ -685,11 +707,10 @@ struct lica_unet {
     // training buffers
     bool train_ready = false;
     float* gout = nullptr;
-    bf16* gy = nullptr;      // gradient w.r.t. a layer output / input (largest level-0 tensor)
-    bf16* gcat = nullptr;    // input gradient of a layer (up to 192 channels at its level)
-    bf16* dz = nullptr;
-    bf16* gsave[3] = {};     // skip gradients kept across the backward pass (e1b, e2b) and pool grads
-    bf16* gpool = nullptr;
+    bf16* gin = nullptr;     // input gradient of a layer with one input
+    bf16* gcat0 = nullptr;   // input gradients of the decoder layers, [upsampled | skip]: L8's (96 channels,
+    bf16* gcat1 = nullptr;   // level 0) and L6's (192, level 1), kept for the encoder's layers
+    bf16* dz = nullptr;      // a layer's output gradient through its ReLU
     float* part = nullptr;
     float* bpart = nullptr;
     size_t part_elems = 0;
@@ -773,6 +794,15 @@ int forward(lica_unet* u, const double* rho, const double* f, double hsq, double
     return conv_layer(u, 9, u->y[8], nullptr, keep_last ? u->y[9] : nullptr, s, &head);
 }
 
+// CTAs along the pixels for a layer's weight gradient: one per SM over the blocks of input
+// channels, at most one per pixel tile.
+int wgrad_chunks(const lica_unet* u, int l) {
+    const LayerDef& L = kNet[l];
+    const int blocks = (L.cin0 + L.cin1) / (L.cin0 % 32 ? 16 : 32);
+    const int tiles = (int)(level_pixels(u, L.level) / kTileM);
+    return std::max(1, std::min(tiles, 148 / blocks));
+}
+
 int alloc_training(lica_unet* u) {
     if (u->train_ready) return LICA_OK;
     const size_t p0 = level_pixels(u, 0), p1 = level_pixels(u, 1), p2 = level_pixels(u, 2);
@@ -782,19 +812,17 @@ int alloc_training(lica_unet* u) {
     if ((st = dev_alloc(&u->adam_v, u->nparams))) return st;
     LICA_CUDA_TRY(cudaMemset(u->adam_m, 0, sizeof(float) * u->nparams));
     LICA_CUDA_TRY(cudaMemset(u->adam_v, 0, sizeof(float) * u->nparams));
-    const size_t big = std::max({p0 * 96, p1 * 192, p2 * 128});
+    const size_t one = std::max({p0 * 32, p1 * 64, p2 * 128});   // a layer's own channels at its level
     if ((st = dev_alloc(&u->gout, p0))) return st;
-    if ((st = dev_alloc(&u->gy, big))) return st;
-    if ((st = dev_alloc(&u->gcat, big))) return st;
-    if ((st = dev_alloc(&u->dz, big))) return st;
-    if ((st = dev_alloc(&u->gsave[0], p0 * 32))) return st;   // d(e1b) from the decoder
-    if ((st = dev_alloc(&u->gsave[1], p1 * 64))) return st;   // d(e2b) from the decoder
-    if ((st = dev_alloc(&u->gpool, big))) return st;
+    if ((st = dev_alloc(&u->gin, one))) return st;
+    if ((st = dev_alloc(&u->dz, one))) return st;
+    if ((st = dev_alloc(&u->gcat0, p0 * 96))) return st;
+    if ((st = dev_alloc(&u->gcat1, p1 * 192))) return st;
     // weight-gradient partials: the largest layer's chunks x weights
     size_t pe = 0, be = 0;
     for (int l = 0; l < kLayers; ++l) {
         const LayerDef& L = kNet[l];
-        const size_t chunks = (level_pixels(u, L.level) + kDwChunk - 1) / kDwChunk;
+        const size_t chunks = (size_t)wgrad_chunks(u, l);
         pe = std::max(pe, chunks * L.cout * 9 * (L.cin0 + L.cin1));
         be = std::max(be, chunks * L.cout);
     }
@@ -810,98 +838,115 @@ int alloc_training(lica_unet* u) {
 int layer_wgrad(lica_unet* u, int l, const bf16* x0, const bf16* x1, cudaStream_t s) {
     const LayerDef& L = kNet[l];
     const int H = u->h >> L.level, W = u->w >> L.level, ctot = L.cin0 + L.cin1;
-    const size_t npix = (size_t)u->n * H * W;
-    const int chunks = (int)((npix + kDwChunk - 1) / kDwChunk);
-    dim3 grid(chunks, 9, (L.cout / 32) * ((ctot + 31) / 32));
-    k_dw_part<<<grid, kNT, 0, s>>>(u->dz, L.cout, x0, L.cin0, x1, L.cin1, u->n, H, W, u->part, u->bpart);
+    static std::once_flag attr_once;
+    static cudaError_t attr_err = cudaSuccess;
+    constexpr int kSmem = 220 * 1024;
+    std::call_once(attr_once, [] {
+        attr_err = cudaFuncSetAttribute(k_wgrad3x3, cudaFuncAttributeMaxDynamicSharedMemorySize, kSmem);
+    });
+    LICA_CUDA_TRY(attr_err);
+    WgradParams P{};
+    P.h = H;
+    P.w = W;
+    P.tiles = (int)(level_pixels(u, L.level) / kTileM);
+    P.cout = L.cout;
+    P.ctot = ctot;
+    P.cblk = L.cin0 % 32 ? 16 : 32;
+    P.c0 = L.cin0;
+    P.stage = (L.cout / 32) * kWgDzBox + (3 * kHaloRows * 2 * P.cblk + 1023) / 1024 * 1024;
+    P.nstages = std::min(kWgMaxStages, (kSmem - 1024 - kWgBehind) / P.stage);
+    P.part = u->part;
+    P.bpart = u->bpart;
+    P.err = u->err;
+    CUtensorMap mdz, m0, m1;
+    int st;
+    if ((st = act_map(&mdz, u->dz, L.cout, W, H, u->n, 32, kTileW, kTileH))) return st;
+    if ((st = act_map(&m0, x0, L.cin0, W, H, u->n, P.cblk, kTileW, kTileH + 2))) return st;
+    m1 = m0;
+    if (L.cin1 && (st = act_map(&m1, x1, L.cin1, W, H, u->n, P.cblk, kTileW, kTileH + 2))) return st;
+    const int chunks = wgrad_chunks(u, l);
+    k_wgrad3x3<<<dim3(chunks, ctot / P.cblk), kWgThreads, 1024 + P.nstages * P.stage + kWgBehind, s>>>(mdz, m0, m1, P);
     LICA_CUDA_TRY(cudaGetLastError());
-    const size_t nw = (size_t)L.cout * 9 * ctot;
-    k_sum_parts<<<grid_for(nw), kNT, 0, s>>>(u->part, chunks, nw, u->grad + u->woff[l]);
-    k_sum_parts<<<grid_for(L.cout), kNT, 0, s>>>(u->bpart, chunks, (size_t)L.cout, u->grad + u->boff[l]);
-    LICA_CUDA_TRY(cudaGetLastError());
-    lica_count_launches(3);
-    return LICA_OK;
+    lica_count_launches(1);
+    return sum_parts(u->part, chunks, (size_t)L.cout * 9 * ctot, u->grad + u->woff[l], u->bpart, (size_t)L.cout,
+                     u->grad + u->boff[l], s);
 }
 
-// Input gradient of layer l: gcat = conv3x3(dz, wf) (channels [x0 | x1]).
-int layer_igrad(lica_unet* u, int l, cudaStream_t s) {
+// Input gradient of layer l: out = conv3x3(dz, wf) (channels [x0 | x1]).
+int layer_igrad(lica_unet* u, int l, bf16* out, cudaStream_t s) {
     const LayerDef& L = kNet[l];
     const int ctot = L.cin0 + L.cin1;
     return conv3x3(u->dz, L.cout, nullptr, 0, u->wf[l], nullptr, u->n, u->h >> L.level, u->w >> L.level, ctot, 0,
-                   u->gcat, nullptr, ctot, 0, u->err, s);
+                   out, nullptr, ctot, 0, u->err, s);
 }
 
 // dz = g (channel slice of a tensor) [+ pool backward of gp] masked by the layer's ReLU.
 int relu_bwd(lica_unet* u, int l, const bf16* g, int g_cs, int g_c0, const bf16* gp, cudaStream_t s) {
     const LayerDef& L = kNet[l];
     const int H = u->h >> L.level, W = u->w >> L.level;
-    return launch(level_pixels(u, L.level) * L.cout, s, k_relu_bwd, g, g_cs, g_c0, gp, (const bf16*)u->y[l], u->dz,
+    return launch(level_pixels(u, L.level) * (L.cout / 8), s, k_relu_bwd, g, g_cs, g_c0, gp, (const bf16*)u->y[l], u->dz,
                   u->n, H, W, L.cout);
 }
 
-// Backward pass from gout (dL/d out32): every parameter gradient into u->grad.
+// dz = the upsampling's backward of a slice of g masked by the ReLU of layer l (before it).
+int up_relu_bwd(lica_unet* u, int l, const bf16* g, int g_cs, cudaStream_t s) {
+    const LayerDef& L = kNet[l];
+    const int H = u->h >> L.level, W = u->w >> L.level;
+    return launch(level_pixels(u, L.level) * (L.cout / 8), s, k_up_relu_bwd, g, g_cs, 0, (const bf16*)u->y[l], u->dz,
+                  u->n, H, W, L.cout);
+}
+
+// Backward pass from gout (dL/d out32): every parameter gradient into u->grad.  Every pass over
+// the activations between the convolutions reads and writes 16 bytes a thread, applies the next
+// ReLU on the way, and takes the decoder's two input gradients where their convolutions left them
+// (gcat1, gcat0): as separate passes of one value a thread with copies of the skip slices, they
+// took 0.37 ms of four 256 x 256 images' 1.19, 0.08 so.
 int backward(lica_unet* u, cudaStream_t s) {
-    const int h = u->h, w = u->w, n = u->n;
     const size_t p0 = level_pixels(u, 0);
     int st;
-    // head
+    // head and the ReLU of L9
     const int hb = grid_for(p0);
-    k_head_grad_part<<<hb, kNT, 0, s>>>(u->gout, u->y[9], u->hpart, p0);
-    k_sum_parts<<<1, kNT, 0, s>>>(u->hpart, hb, (size_t)(kHead + 1), u->grad + u->hoff);
-    k_head_bwd<<<grid_for(p0), kNT, 0, s>>>(u->gout, u->param + u->hoff, u->gy, p0);
+    k_head_bwd<<<hb, kNT, 0, s>>>(u->gout, u->param + u->hoff, u->y[9], u->dz, u->hpart, p0);
     LICA_CUDA_TRY(cudaGetLastError());
-    lica_count_launches(3);
+    lica_count_launches(1);
+    if ((st = sum_parts(u->hpart, hb, (size_t)(kHead + 1), u->grad + u->hoff, nullptr, 0, nullptr, s))) return st;
     // L9 (input d1a)
-    if ((st = relu_bwd(u, 9, u->gy, 32, 0, nullptr, s))) return st;
     if ((st = layer_wgrad(u, 9, u->y[8], nullptr, s))) return st;
-    if ((st = layer_igrad(u, 9, s))) return st;  // gcat = d(d1a), 32 ch
+    if ((st = layer_igrad(u, 9, u->gin, s))) return st;  // d(d1a), 32 ch
     // L8 (inputs [u1 (64), e1b (32)])
-    if ((st = relu_bwd(u, 8, u->gcat, 32, 0, nullptr, s))) return st;
+    if ((st = relu_bwd(u, 8, u->gin, 32, 0, nullptr, s))) return st;
     if ((st = layer_wgrad(u, 8, u->u1, u->y[1], s))) return st;
-    if ((st = layer_igrad(u, 8, s))) return st;  // gcat = [d(u1) 64 | d(e1b) 32]
-    LICA_CUDA_TRY(cudaMemcpy2DAsync(u->gsave[0], 32 * sizeof(bf16), u->gcat + 64, 96 * sizeof(bf16),
-                                    32 * sizeof(bf16), p0, cudaMemcpyDeviceToDevice, s));
-    if ((st = launch(level_pixels(u, 1) * 64, s, k_up_bwd, (const bf16*)u->gcat, 96, 0, u->gy, n, h / 2, w / 2, 64)))
-        return st;  // gy = d(d2b)
+    if ((st = layer_igrad(u, 8, u->gcat0, s))) return st;  // [d(u1) 64 | d(e1b) 32]
     // L7 (input d2a)
-    if ((st = relu_bwd(u, 7, u->gy, 64, 0, nullptr, s))) return st;
+    if ((st = up_relu_bwd(u, 7, u->gcat0, 96, s))) return st;
     if ((st = layer_wgrad(u, 7, u->y[6], nullptr, s))) return st;
-    if ((st = layer_igrad(u, 7, s))) return st;  // gcat = d(d2a)
+    if ((st = layer_igrad(u, 7, u->gin, s))) return st;  // d(d2a)
     // L6 (inputs [u2 (128), e2b (64)])
-    if ((st = relu_bwd(u, 6, u->gcat, 64, 0, nullptr, s))) return st;
+    if ((st = relu_bwd(u, 6, u->gin, 64, 0, nullptr, s))) return st;
     if ((st = layer_wgrad(u, 6, u->u2, u->y[3], s))) return st;
-    if ((st = layer_igrad(u, 6, s))) return st;  // gcat = [d(u2) 128 | d(e2b) 64]
-    LICA_CUDA_TRY(cudaMemcpy2DAsync(u->gsave[1], 64 * sizeof(bf16), u->gcat + 128, 192 * sizeof(bf16),
-                                    64 * sizeof(bf16), level_pixels(u, 1), cudaMemcpyDeviceToDevice, s));
-    if ((st = launch(level_pixels(u, 2) * 128, s, k_up_bwd, (const bf16*)u->gcat, 192, 0, u->gy, n, h / 4, w / 4,
-                     128)))
-        return st;  // gy = d(e3b)
+    if ((st = layer_igrad(u, 6, u->gcat1, s))) return st;  // [d(u2) 128 | d(e2b) 64]
     // L5 (input e3a)
-    if ((st = relu_bwd(u, 5, u->gy, 128, 0, nullptr, s))) return st;
+    if ((st = up_relu_bwd(u, 5, u->gcat1, 192, s))) return st;
     if ((st = layer_wgrad(u, 5, u->y[4], nullptr, s))) return st;
-    if ((st = layer_igrad(u, 5, s))) return st;  // gcat = d(e3a)
+    if ((st = layer_igrad(u, 5, u->gin, s))) return st;  // d(e3a)
     // L4 (input p2)
-    if ((st = relu_bwd(u, 4, u->gcat, 128, 0, nullptr, s))) return st;
+    if ((st = relu_bwd(u, 4, u->gin, 128, 0, nullptr, s))) return st;
     if ((st = layer_wgrad(u, 4, u->p2, nullptr, s))) return st;
-    if ((st = layer_igrad(u, 4, s))) return st;  // gcat = d(p2), 64 ch at level 2
-    LICA_CUDA_TRY(cudaMemcpyAsync(u->gpool, u->gcat, sizeof(bf16) * level_pixels(u, 2) * 64,
-                                  cudaMemcpyDeviceToDevice, s));
+    if ((st = layer_igrad(u, 4, u->gin, s))) return st;  // d(p2), 64 ch at level 2
     // L3 (input e2a): d(e2b) = decoder part + pool backward of d(p2)
-    if ((st = relu_bwd(u, 3, u->gsave[1], 64, 0, u->gpool, s))) return st;
+    if ((st = relu_bwd(u, 3, u->gcat1, 192, 128, u->gin, s))) return st;
     if ((st = layer_wgrad(u, 3, u->y[2], nullptr, s))) return st;
-    if ((st = layer_igrad(u, 3, s))) return st;  // gcat = d(e2a)
+    if ((st = layer_igrad(u, 3, u->gin, s))) return st;  // d(e2a)
     // L2 (input p1)
-    if ((st = relu_bwd(u, 2, u->gcat, 64, 0, nullptr, s))) return st;
+    if ((st = relu_bwd(u, 2, u->gin, 64, 0, nullptr, s))) return st;
     if ((st = layer_wgrad(u, 2, u->p1, nullptr, s))) return st;
-    if ((st = layer_igrad(u, 2, s))) return st;  // gcat = d(p1), 32 ch at level 1
-    LICA_CUDA_TRY(cudaMemcpyAsync(u->gpool, u->gcat, sizeof(bf16) * level_pixels(u, 1) * 32,
-                                  cudaMemcpyDeviceToDevice, s));
+    if ((st = layer_igrad(u, 2, u->gin, s))) return st;  // d(p1), 32 ch at level 1
     // L1 (input e1a): d(e1b) = decoder part + pool backward of d(p1)
-    if ((st = relu_bwd(u, 1, u->gsave[0], 32, 0, u->gpool, s))) return st;
+    if ((st = relu_bwd(u, 1, u->gcat0, 96, 64, u->gin, s))) return st;
     if ((st = layer_wgrad(u, 1, u->y[0], nullptr, s))) return st;
-    if ((st = layer_igrad(u, 1, s))) return st;  // gcat = d(e1a)
+    if ((st = layer_igrad(u, 1, u->gin, s))) return st;  // d(e1a)
     // L0 (input x16): weights only
-    if ((st = relu_bwd(u, 0, u->gcat, 32, 0, nullptr, s))) return st;
+    if ((st = relu_bwd(u, 0, u->gin, 32, 0, nullptr, s))) return st;
     return layer_wgrad(u, 0, u->x16, nullptr, s);
 }
 
@@ -984,8 +1029,8 @@ int lica_unet_create(lica_unet** out, int32_t n, int32_t h, int32_t w, uint64_t 
 int lica_unet_destroy(lica_unet* u) {
     if (!u) return LICA_OK;
     void* ptrs[] = {u->param, u->grad, u->adam_m, u->adam_v, u->x16, u->p1, u->p2, u->u2, u->u1, u->out32,
-                    u->sigma, u->rms_part, u->x0, u->ax, u->rr, u->den, u->part2, u->gout, u->gy, u->gcat, u->dz,
-                    u->gsave[0], u->gsave[1], u->gsave[2], u->gpool, u->part, u->bpart, u->hpart, u->err};
+                    u->sigma, u->rms_part, u->x0, u->ax, u->rr, u->den, u->part2, u->gout, u->gin, u->gcat0,
+                    u->gcat1, u->dz, u->part, u->bpart, u->hpart, u->err};
     for (void* p : ptrs) cudaFree(p);
     for (int l = 0; l < kLayers; ++l) {
         cudaFree(u->wb[l]);
