@@ -55,7 +55,6 @@ constexpr int TY = 32;
 constexpr int NT = 256;          // threads of a CG / set-up grid-kernel CTA
 constexpr int NT_CTA = 512;      // threads of the single-CTA coarse kernel (fewer idle warps per barrier than 1024)
 constexpr int kMaxLevels = 16;
-constexpr int kSmallCells = 64;  // levels with <= this many cells run in warp 0 alone
 constexpr int kMaxDense = 64;    // bottom-level unknowns solved by dense elimination
 constexpr double kStallFactor = 1e3;  // a rise of the residual below this x tol ends the PCG (LICA_STALLED)
 
@@ -781,18 +780,18 @@ struct CtaLevel {
     int nx, ny, half;
     unsigned mag_h, mag_nx;  // division multipliers for half and nx (t / c = umulhi(t, mag), c > 1)
     unsigned off_u[2], off_f[2], off_ax[2], off_ay[2], off_di[2];  // byte offsets into dynamic smem
-    const void* gax;                                                // AX, AY, DINV of this level (T or double)
-    const void* gay;
-    const void* gdi;
+    int warps;                                                      // warps that work on this level
 };
 
 struct CtaParams {
     int lcta, lc, bottom;
     int nu1, nu2, ncoarse;
     unsigned off_dense, off_rhs;
-    const double* glu; // bottom-level elimination (multipliers below, U on and above the diagonal)
+    const void* image; // the weights of every level and the bottom elimination as they lie in shared memory,
+    unsigned image_bytes;  // from its start (k_cta_image)
     const void* f_in;  // f of level lcta (T)
     void* u_out;       // u of level lcta (T)
+    State* st;
     CtaLevel lv[kMaxLevels];
 };
 
@@ -808,8 +807,8 @@ struct SL {
 };
 
 template <typename E>
-__device__ __forceinline__ SL<E> make_sl(const CtaParams& P, unsigned char* sm, int l) {
-    const CtaLevel& L = P.lv[l];
+__device__ __forceinline__ SL<E> make_sl(const CtaLevel* lv, unsigned char* sm, int l) {
+    const CtaLevel& L = lv[l];
     SL<E> s;
 #pragma unroll
     for (int c = 0; c < 2; ++c) {
@@ -825,15 +824,6 @@ __device__ __forceinline__ SL<E> make_sl(const CtaParams& P, unsigned char* sm, 
     s.mag_h = L.mag_h;
     s.mag_nx = L.mag_nx;
     return s;
-}
-
-template <bool W>
-__device__ __forceinline__ int g_tid() { return W ? (int)(threadIdx.x & 31) : (int)threadIdx.x; }
-template <bool W>
-__device__ __forceinline__ constexpr int g_nthr() { return W ? 32 : NT_CTA; }
-template <bool W>
-__device__ __forceinline__ void g_sync() {
-    if (W) __syncwarp(); else __syncthreads();
 }
 
 // Items it = t, t + G, ... of a (rows x cols) range as an incremental (row, col) pair.
@@ -901,21 +891,83 @@ __device__ __forceinline__ void split_sums(const Colour<E>& V, int j, int m, int
     d = dd;
 }
 
-template <typename E, bool W>
-__device__ void s_sweeps(const SL<E>& L, int nsw, bool reverse) {
+// The warps of a level: the first `warps` of the CTA, one item a lane on the small levels, so that
+// a half-sweep's barrier counts no warp without a cell.  The levels' groups are nested (warps does
+// not rise with the level); barrier 1 + l is level l's.
+struct Group {
+    int n, t, id;   // threads, this thread, barrier
+    __device__ __forceinline__ Group(const CtaLevel& L, int l) : n(32 * L.warps), t(threadIdx.x), id(1 + l) {}
+    __device__ __forceinline__ void sync() const {
+        if (n == 32) __syncwarp();
+        else asm volatile("bar.sync %0, %1;" ::"r"(id), "r"(n) : "memory");
+    }
+};
+
+// Red-black sweeps of level l.  The weights of a thread's two cells stay in registers over the
+// half-sweeps where a thread has one cell of each colour (a half-sweep is then four shared loads,
+// nine operations, a store and the group's barrier); larger levels walk their cells.  Out of line,
+// one copy for all levels: the kernel runs each path a few times, and its code is read as often.
+// The kernels' dynamic shared memory, as such (a pointer handed to a function that is not inlined
+// would be a generic one).
+extern __shared__ __align__(16) unsigned char cta_dynamic_smem[];
+__device__ __forceinline__ unsigned char* cta_smem_base() { return cta_dynamic_smem; }
+
+template <typename E>
+__device__ __noinline__ void s_sweeps(const CtaLevel* lv, int l, int nsw, bool reverse) {
+    const SL<E> L = make_sl<E>(lv, cta_smem_base(), l);
+    const Group G(lv[l], l);
     const int items = L.ny * L.h;
+    if (items <= G.n) {
+        const bool own = G.t < items;
+        const int it = own ? G.t : 0, h = L.h, j = div_mag(it, h, L.mag_h), m = it - j * h;
+        const E* up[2];   // the other colour's u at the cell; its west and east entries
+        int w[2], e[2];
+        E aw[2], ae[2], as[2], an[2], fc[2], dc[2];
+#pragma unroll
+        for (int c = 0; c < 2; ++c) {
+            const int o = (j + c) & 1;
+            int wi = m - 1 + o, ei = m + o;
+            if (wi < 0) wi += h;
+            if (ei >= h) ei -= h;
+            w[c] = wi - m;
+            e[c] = ei - m;
+            up[c] = L.u[1 - c] + it;
+            aw[c] = L.ax[c][it];
+            ae[c] = L.ax[1 - c][it + e[c]];
+            as[c] = L.ay[c][it];
+            an[c] = L.ay[1 - c][it + h];
+            fc[c] = L.f[c][it];
+            dc[c] = L.di[c][it];
+        }
+        auto half = [&](int c, E* uc) {
+            E s = aw[c] * up[c][w[c]];
+            s += ae[c] * up[c][e[c]];
+            s += as[c] * up[c][-h];
+            s += an[c] * up[c][h];
+            if (own) uc[it] = (s - fc[c]) * dc[c];
+            G.sync();
+        };
+#pragma unroll 1
+        for (int q = 0; q < nsw; ++q) {
+            if (reverse) half(1, L.u[1]);
+            half(0, L.u[0]);
+            if (!reverse) half(1, L.u[1]);
+        }
+        return;
+    }
+#pragma unroll 1
     for (int q = 0; q < 2 * nsw; ++q) {
         const Colour<E> V(L, reverse ? 1 - (q & 1) : (q & 1));
-        ItemWalk wk(g_tid<W>(), g_nthr<W>(), L.h, L.mag_h);
+        ItemWalk wk(G.t, G.n, L.h, L.mag_h);
 #pragma unroll 2
-        for (int it = g_tid<W>(); it < items; it += g_nthr<W>()) {
+        for (int it = G.t; it < items; it += G.n) {
             const int k = wk.r * L.h + wk.q;
             E s, d;
             split_sums(V, wk.r, wk.q, k, s, d);
             V.uc[k] = (s - V.fc[k]) * V.dc[k];
             wk.next();
         }
-        g_sync<W>();
+        G.sync();
     }
 }
 
@@ -928,14 +980,17 @@ __device__ __forceinline__ E split_res(const Colour<E>& V, int j, int m) {
     return V.fc[k] - (s - d * V.uc[k]);
 }
 
-// fc(I, J) = 0.25*((r00 + r10) + (r01 + r11)) of the residual, and uc = 0.
-template <typename E, typename EC, bool W>
-__device__ void s_restrict(const SL<E>& F, const SL<EC>& C) {
+// Level l + 1: fc(I, J) = 0.25*((r00 + r10) + (r01 + r11)) of the residual of level l, and uc = 0.
+template <typename E, typename EC>
+__device__ __noinline__ void s_restrict(const CtaLevel* lv, int l) {
+    const SL<E> F = make_sl<E>(lv, cta_smem_base(), l);
+    const SL<EC> C = make_sl<EC>(lv, cta_smem_base(), l + 1);
+    const Group G(lv[l], l);
     const int items = C.nx * C.ny;
     const Colour<E> R(F, 0), B(F, 1);
-    ItemWalk wk(g_tid<W>(), g_nthr<W>(), C.nx, C.mag_nx);
-#pragma unroll 2
-    for (int it = g_tid<W>(); it < items; it += g_nthr<W>()) {
+    ItemWalk wk(G.t, G.n, C.nx, C.mag_nx);
+#pragma unroll 1
+    for (int it = G.t; it < items; it += G.n) {
         const int J = wk.r, I = wk.q;
         const E r00 = split_res(R, 2 * J, I);
         const E r10 = split_res(B, 2 * J, I);
@@ -947,16 +1002,21 @@ __device__ void s_restrict(const SL<E>& F, const SL<EC>& C) {
         pick(C.u, cc)[kc] = EC(0);
         wk.next();
     }
-    g_sync<W>();
+    G.sync();
 }
 
-// u += P uc (piecewise constant): the four children of coarse cell (I, J).
-template <typename E, typename EC, bool W>
-__device__ void s_prolong(const SL<EC>& C, const SL<E>& F) {
+// Level l: u += P uc (piecewise constant), the four children of coarse cell (I, J).  Starts with
+// the barrier that waits for the warps of level l + 1.
+template <typename E, typename EC>
+__device__ __noinline__ void s_prolong(const CtaLevel* lv, int l) {
+    const SL<E> F = make_sl<E>(lv, cta_smem_base(), l);
+    const SL<EC> C = make_sl<EC>(lv, cta_smem_base(), l + 1);
+    const Group G(lv[l], l);
+    G.sync();
     const int items = C.nx * C.ny;
-    ItemWalk wk(g_tid<W>(), g_nthr<W>(), C.nx, C.mag_nx);
-#pragma unroll 2
-    for (int it = g_tid<W>(); it < items; it += g_nthr<W>()) {
+    ItemWalk wk(G.t, G.n, C.nx, C.mag_nx);
+#pragma unroll 1
+    for (int it = G.t; it < items; it += G.n) {
         const int J = wk.r, I = wk.q;
         const E e = E(pick(C.u, (I + J) & 1)[J * C.h + (I >> 1)]);
         const int k0 = 2 * J * F.h + I, k1 = k0 + F.h;
@@ -966,117 +1026,118 @@ __device__ void s_prolong(const SL<EC>& C, const SL<E>& F) {
         F.u[1][k1] += e;
         wk.next();
     }
-    g_sync<W>();
+    G.sync();
 }
 
 // Plain-index accessors of a colour-split level (the dense solve's assembly).
 template <typename E>
 __device__ __forceinline__ int split_index(const SL<E>& L, int i, int j) { return j * L.h + (i >> 1); }
 
-// Dense solve of the bottom level, unknown row = j*nx + i, with the elimination of the
-// matrix done once per solve (k_dense_factor): the oracle's b[i] -= m*b[k] in its order,
-// then its back substitution s = b[i] - sum_j U[i][j] u[j] (j ascending), u[i] = s / U[i][i].
-template <bool W>
-__device__ void s_dense(const SL<double>& L, const double* A, double* b) {
-    const int nx = L.nx, n = nx * L.ny;
-    for (int k = g_tid<W>(); k < n; k += g_nthr<W>()) {
+// Dense solve of the bottom level by warp 0, unknown row = j*nx + i, with the elimination of the
+// matrix done once per solve (k_dense_factor): the oracle's b[i] -= m*b[k] in its order, then
+// its back substitution s = b[i] - sum_j U[i][j] u[j] (j ascending), u[i] = s / U[i][i].  Up to 32
+// unknowns lie one a lane: a step of the elimination is one broadcast, and a row's products are
+// formed side by side before their sum in order.
+__device__ __noinline__ void s_dense(const CtaLevel* lv, int l, unsigned off_dense, unsigned off_rhs) {
+    const double* A = reinterpret_cast<const double*>(cta_smem_base() + off_dense);
+    double* b = reinterpret_cast<double*>(cta_smem_base() + off_rhs);
+    const SL<double> L = make_sl<double>(lv, cta_smem_base(), l);
+    const int nx = L.nx, n = nx * L.ny, lane = threadIdx.x;
+    if (n <= 32) {
+        const int i = min(lane, n - 1), jr = i / nx, ir = i - jr * nx, c = (ir + jr) & 1, at = split_index(L, ir, jr);
+        const double diag = A[i * n + i], y = rn::recip(diag);
+        double v = pick(L.f, c)[at];
+#pragma unroll 4
+        for (int k = 0; k + 1 < n; ++k) {
+            const double bk = __shfl_sync(0xffffffffu, v, k);
+            const double t = v - A[i * n + k] * bk;
+            if (i > k) v = t;
+        }
+        double u = 0.0;   // the solution of this lane's row, once it is known
+        for (int r = n - 1; r >= 0; --r) {
+            const double pr = A[r * n + i] * u;
+            double s = __shfl_sync(0xffffffffu, v, r);
+#pragma unroll 4
+            for (int j = r + 1; j < n; ++j) s -= __shfl_sync(0xffffffffu, pr, j);
+            if (lane == r)
+                u = (rn::ordinary(diag) && rn::ordinary(s)) ? rn::quot(s, diag, y) : s / diag;
+        }
+        if (lane < n) pick(L.u, c)[at] = u;
+        __syncwarp();
+        return;
+    }
+    for (int k = lane; k < n; k += 32) {
         const int j = k / nx, i = k - j * nx;
         b[k] = pick(L.f, (i + j) & 1)[split_index(L, i, j)];
     }
-    g_sync<W>();
+    __syncwarp();
     for (int k = 0; k + 1 < n; ++k) {
         const double bk = b[k];
-        for (int i = k + 1 + g_tid<W>(); i < n; i += g_nthr<W>()) b[i] -= A[i * n + k] * bk;
-        g_sync<W>();
+        for (int i = k + 1 + lane; i < n; i += 32) b[i] -= A[i * n + k] * bk;
+        __syncwarp();
     }
-    if (g_tid<W>() == 0) {
+    if (lane == 0) {
         for (int i = n - 1; i >= 0; --i) {
             double s = b[i];
             for (int j = i + 1; j < n; ++j) s -= A[i * n + j] * b[j];
             b[i] = s / A[i * n + i];
         }
     }
-    g_sync<W>();
-    for (int k = g_tid<W>(); k < n; k += g_nthr<W>()) {
+    __syncwarp();
+    for (int k = lane; k < n; k += 32) {
         const int j = k / nx, i = k - j * nx;
         pick(L.u, (i + j) & 1)[split_index(L, i, j)] = b[k];
     }
-    g_sync<W>();
+    __syncwarp();
 }
 
-// First level in [l0, bottom] small enough for warp 0 alone.
-__device__ __forceinline__ int first_small(const CtaParams& P, int l0) {
+// One inner V-cycle on the FP64 levels [l0, bottom] starting from the iterate in u(l0), by the
+// warps of l0; a warp goes down as far as it has cells and waits there for the others.
+__device__ __forceinline__ void s_vcycle_inner(const CtaParams& P, const CtaLevel* lv, int l0) {
+    const int warp = threadIdx.x >> 5;
     int l = l0;
-    while (l < P.bottom && P.lv[l].nx * P.lv[l].ny > kSmallCells) ++l;
-    return l;
-}
-
-// Down-and-up over FP64 levels [la, lb] by group W: sweeps + restriction going down to
-// lb (dense solve there when lb is the bottom) and prolongation + sweeps coming back.
-template <bool W>
-__device__ void s_inner_range_down(const CtaParams& P, unsigned char* sm, int la, int lb) {
-    for (int l = la; l < lb; ++l) {
-        const SL<double> L = make_sl<double>(P, sm, l);
-        const SL<double> C = make_sl<double>(P, sm, l + 1);
-        s_sweeps<double, W>(L, P.nu1, false);
-        s_restrict<double, double, W>(L, C);
+    for (; l < P.bottom && warp < lv[l].warps; ++l) {
+        s_sweeps<double>(lv, l, P.nu1, false);
+        s_restrict<double, double>(lv, l);
     }
-}
-template <bool W>
-__device__ void s_inner_range_up(const CtaParams& P, unsigned char* sm, int la, int lb) {
-    for (int l = lb - 1; l >= la; --l) {
-        const SL<double> L = make_sl<double>(P, sm, l);
-        const SL<double> C = make_sl<double>(P, sm, l + 1);
-        s_prolong<double, double, W>(C, L);
-        s_sweeps<double, W>(L, P.nu2, true);
+    if (l == P.bottom && warp == 0)
+        s_dense(lv, P.bottom, P.off_dense, P.off_rhs);
+    for (--l; l >= l0; --l) {
+        s_prolong<double, double>(lv, l);
+        s_sweeps<double>(lv, l, P.nu2, true);
     }
-}
-
-// One inner V-cycle on the FP64 levels [l0, bottom] starting from the iterate in u(l0).
-// Levels above the first small level run block-wide, the rest in warp 0.
-__device__ void s_vcycle_inner(const CtaParams& P, unsigned char* sm, int l0) {
-    double* A = reinterpret_cast<double*>(sm + P.off_dense);
-    double* b = reinterpret_cast<double*>(sm + P.off_rhs);
-    const int ls = first_small(P, l0);
-    s_inner_range_down<false>(P, sm, l0, ls);
-    if (threadIdx.x < 32) {
-        s_inner_range_down<true>(P, sm, ls, P.bottom);
-        s_dense<true>(make_sl<double>(P, sm, P.bottom), A, b);
-        s_inner_range_up<true>(P, sm, ls, P.bottom);
-    }
-    __syncthreads();
-    s_inner_range_up<false>(P, sm, l0, ls);
 }
 
 // Levels [lcta, lc) in T, then the coarsest outer level lc (FP64): ncoarse inner
-// V-cycles from a zero iterate, or the dense solve when lc is the bottom level.
+// V-cycles from a zero iterate, or the dense solve when lc is the bottom level.  Ends without a
+// barrier over the CTA.
 template <typename T>
-__device__ void s_outer(const CtaParams& P, unsigned char* sm) {
-    for (int l = P.lcta; l < P.lc; ++l) {
-        const SL<T> L = make_sl<T>(P, sm, l);
-        s_sweeps<T, false>(L, P.nu1, false);
-        if (l + 1 == P.lc) s_restrict<T, double, false>(L, make_sl<double>(P, sm, l + 1));
-        else s_restrict<T, T, false>(L, make_sl<T>(P, sm, l + 1));
+__device__ __forceinline__ void s_outer(const CtaParams& P, const CtaLevel* lv) {
+    const int warp = threadIdx.x >> 5;
+    int l = P.lcta;
+    for (; l < P.lc && warp < lv[l].warps; ++l) {
+        s_sweeps<T>(lv, l, P.nu1, false);
+        if (l + 1 == P.lc) s_restrict<T, double>(lv, l);
+        else s_restrict<T, T>(lv, l);
     }
-    {
-        const SL<double> L = make_sl<double>(P, sm, P.lc);
+    if (l == P.lc && warp < lv[P.lc].warps) {
         if (P.lcta == P.lc) {  // no restriction wrote u(lc)
-            for (int k = threadIdx.x; k < L.ny * L.h; k += NT_CTA) { L.u[0][k] = 0.0; L.u[1][k] = 0.0; }
-            __syncthreads();
+            const SL<double> L = make_sl<double>(lv, cta_smem_base(), P.lc);
+            const Group G(lv[P.lc], P.lc);
+            for (int k = G.t; k < L.ny * L.h; k += G.n) { L.u[0][k] = 0.0; L.u[1][k] = 0.0; }
+            G.sync();
         }
         if (P.lc == P.bottom) {
-            if (threadIdx.x < 32)
-                s_dense<true>(L, reinterpret_cast<double*>(sm + P.off_dense), reinterpret_cast<double*>(sm + P.off_rhs));
-            __syncthreads();
+            if (warp == 0)
+                s_dense(lv, P.lc, P.off_dense, P.off_rhs);
         } else {
-            for (int c = 0; c < P.ncoarse; ++c) s_vcycle_inner(P, sm, P.lc);
+            for (int c = 0; c < P.ncoarse; ++c) s_vcycle_inner(P, lv, P.lc);
         }
     }
-    for (int l = P.lc - 1; l >= P.lcta; --l) {
-        const SL<T> L = make_sl<T>(P, sm, l);
-        if (l + 1 == P.lc) s_prolong<T, double, false>(make_sl<double>(P, sm, l + 1), L);
-        else s_prolong<T, T, false>(make_sl<T>(P, sm, l + 1), L);
-        s_sweeps<T, false>(L, P.nu2, true);
+    for (--l; l >= P.lcta; --l) {
+        if (l + 1 == P.lc) s_prolong<T, double>(lv, l);
+        else s_prolong<T, T>(lv, l);
+        s_sweeps<T>(lv, l, P.nu2, true);
     }
 }
 
@@ -1107,47 +1168,54 @@ __device__ __forceinline__ void stage_split(E* X0, E* X1, const E* __restrict__ 
     }
 }
 
+// The zero ghost rows of u of the CTA's levels (T below the coarsest outer level, then FP64).
 template <typename T>
-__global__ void __launch_bounds__(NT_CTA, 1) k_cta(const __grid_constant__ CtaParams P) {
-    extern __shared__ __align__(16) unsigned char sm[];
-    // stage beta of every level handled here and the bottom elimination, zero the ghost
-    // rows of u, stage f(lcta)
+__device__ __forceinline__ void zero_ghosts(const CtaParams& P, unsigned char* sm) {
     for (int l = P.lcta; l <= P.bottom; ++l) {
         const CtaLevel& L = P.lv[l];
-        if (l < P.lc) {
-            const SL<T> S = make_sl<T>(P, sm, l);
-            stage_split(S.ax[0], S.ax[1], reinterpret_cast<const T*>(L.gax), L.nx, L.ny, L.mag_h);
-            stage_split(S.ay[0], S.ay[1], reinterpret_cast<const T*>(L.gay), L.nx, L.ny + 1, L.mag_h);
-            stage_split(S.di[0], S.di[1], reinterpret_cast<const T*>(L.gdi), L.nx, L.ny, L.mag_h);
+        auto rows = [&](auto zero) {
+            const SL<decltype(zero)> S = make_sl<decltype(zero)>(P.lv, sm, l);
             for (int k = threadIdx.x; k < L.half; k += NT_CTA) {
-                S.u[0][k - L.half] = T(0); S.u[1][k - L.half] = T(0);
-                S.u[0][L.ny * L.half + k] = T(0); S.u[1][L.ny * L.half + k] = T(0);
+                S.u[0][k - L.half] = zero; S.u[1][k - L.half] = zero;
+                S.u[0][L.ny * L.half + k] = zero; S.u[1][L.ny * L.half + k] = zero;
             }
-        } else {
-            const SL<double> S = make_sl<double>(P, sm, l);
-            stage_split(S.ax[0], S.ax[1], reinterpret_cast<const double*>(L.gax), L.nx, L.ny, L.mag_h);
-            stage_split(S.ay[0], S.ay[1], reinterpret_cast<const double*>(L.gay), L.nx, L.ny + 1, L.mag_h);
-            stage_split(S.di[0], S.di[1], reinterpret_cast<const double*>(L.gdi), L.nx, L.ny, L.mag_h);
-            for (int k = threadIdx.x; k < L.half; k += NT_CTA) {
-                S.u[0][k - L.half] = 0.0; S.u[1][k - L.half] = 0.0;
-                S.u[0][L.ny * L.half + k] = 0.0; S.u[1][L.ny * L.half + k] = 0.0;
-            }
-        }
+        };
+        if (l < P.lc) rows(T(0));
+        else rows(0.0);
     }
-    {
-        const int nb = P.lv[P.bottom].nx * P.lv[P.bottom].ny;
-        double* A = reinterpret_cast<double*>(sm + P.off_dense);
-        for (int k = threadIdx.x; k < nb * nb; k += NT_CTA) cp_async_elem(A + k, P.glu + k);
+}
+
+// The weights of every level lie in global memory as they do in shared memory (k_cta_image, once
+// per solve), so staging them is one bulk copy under an mbarrier while the threads stage f: as
+// element copies of each level's arrays it took 7.2 k of a V-cycle's 43 k cycles on one SM.
+// With the sweeps' weights in registers, groups of warps as wide as their level, one copy of the
+// code for all levels and the bottom solve on lanes, the rest went from 36 k to 24 k (1024 x 1024
+// cells: a launch 20.6 -> 14.2 us).
+template <typename T>
+__global__ void __launch_bounds__(NT_CTA, 1) k_cta(const __grid_constant__ CtaParams P) {
+    unsigned char* sm = cta_smem_base();
+    const CtaLevel* lv = P.lv;
+    // in the bottom solve's scratch until the copy is in
+    const unsigned barrier = (unsigned)__cvta_generic_to_shared(sm + P.off_rhs);
+    if (threadIdx.x == 0) {
+        asm volatile("mbarrier.init.shared::cta.b64 [%0], 1;" ::"r"(barrier) : "memory");
+        asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
+        asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;" ::"r"(barrier), "r"(P.image_bytes) : "memory");
+        asm volatile("cp.async.bulk.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1], %2, [%3];" ::"r"(
+                         (unsigned)__cvta_generic_to_shared(sm)),
+                     "l"(P.image), "r"(P.image_bytes), "r"(barrier)
+                     : "memory");
     }
+    zero_ghosts<T>(P, sm);
     {
         const CtaLevel& L = P.lv[P.lcta];
         const T* fin = reinterpret_cast<const T*>(P.f_in);
         if (P.lcta < P.lc) {
-            const SL<T> S = make_sl<T>(P, sm, P.lcta);
+            const SL<T> S = make_sl<T>(P.lv, sm, P.lcta);
             stage_split(S.f[0], S.f[1], fin, L.nx, L.ny, L.mag_h);
             for (int k = threadIdx.x; k < L.ny * L.half; k += NT_CTA) { S.u[0][k] = T(0); S.u[1][k] = T(0); }
         } else {
-            const SL<double> S = make_sl<double>(P, sm, P.lcta);
+            const SL<double> S = make_sl<double>(P.lv, sm, P.lcta);
             if (std::is_same<T, double>::value) {
                 stage_split(S.f[0], S.f[1], reinterpret_cast<const double*>(fin), L.nx, L.ny, L.mag_h);
             } else {
@@ -1164,8 +1232,23 @@ __global__ void __launch_bounds__(NT_CTA, 1) k_cta(const __grid_constant__ CtaPa
         }
     }
     async_wait_all();
+    __syncthreads();   // also the barrier's initialisation
+    {
+        // the copy of at most 227 KB from this GPU's memory; bounded all the same
+        unsigned ok = 0;
+        for (int tries = 0; tries < 1000000 && !ok; ++tries)
+            asm volatile(
+                "{\n\t.reg .pred p;\n\t"
+                "mbarrier.try_wait.parity.shared::cta.b64 p, [%1], 0;\n\t"
+                "selp.u32 %0, 1, 0, p;\n\t}"
+                : "=r"(ok)
+                : "r"(barrier)
+                : "memory");
+        if (!ok) P.st->kerr = 1;
+    }
     __syncthreads();
-    s_outer<T>(P, sm);
+    if (threadIdx.x == 0) asm volatile("mbarrier.inval.shared::cta.b64 [%0];" ::"r"(barrier) : "memory");
+    s_outer<T>(P, lv);
     __syncthreads();
     {
         const CtaLevel& L = P.lv[P.lcta];
@@ -1176,11 +1259,11 @@ __global__ void __launch_bounds__(NT_CTA, 1) k_cta(const __grid_constant__ CtaPa
             const int j = wk.r, m = wk.q, k = j * h + m;
             T a, b;
             if (P.lcta < P.lc) {
-                const SL<T> S = make_sl<T>(P, sm, P.lcta);
+                const SL<T> S = make_sl<T>(P.lv, sm, P.lcta);
                 a = (j & 1) ? S.u[1][k] : S.u[0][k];
                 b = (j & 1) ? S.u[0][k] : S.u[1][k];
             } else {
-                const SL<double> S = make_sl<double>(P, sm, P.lcta);
+                const SL<double> S = make_sl<double>(P.lv, sm, P.lcta);
                 a = T((j & 1) ? S.u[1][k] : S.u[0][k]);
                 b = T((j & 1) ? S.u[0][k] : S.u[1][k]);
             }
@@ -1188,6 +1271,316 @@ __global__ void __launch_bounds__(NT_CTA, 1) k_cta(const __grid_constant__ CtaPa
             uo[j * L.nx + 2 * m + 1] = b;
             wk.next();
         }
+    }
+}
+
+// The weights of level l (row-major AX, AY, DINV) into the image at the level's offsets.
+template <typename E>
+__global__ void k_cta_image(const E* __restrict__ ax, const E* __restrict__ ay, const E* __restrict__ di,
+                            unsigned char* __restrict__ image, const CtaLevel L) {
+    const int nx = L.nx, n = nx * L.ny;
+    for (int k = blockIdx.x * blockDim.x + threadIdx.x; k < n + nx; k += gridDim.x * blockDim.x) {
+        const int j = k / nx, i = k - j * nx, c = (i + j) & 1, at = j * L.half + (i >> 1);
+        reinterpret_cast<E*>(image + L.off_ay[c])[at] = ay[k];
+        if (k < n) {
+            reinterpret_cast<E*>(image + L.off_ax[c])[at] = ax[k];
+            reinterpret_cast<E*>(image + L.off_di[c])[at] = di[k];
+        }
+    }
+}
+
+// ------------------------------------------------------------------------------------
+// Whole solves of small systems (FP64, red-black smoothing): level 0 and its hierarchy in one
+// CTA's shared memory, the CG vectors in registers, set-up, V-cycles and CG in one launch.  Such
+// a solve is launches and gaps otherwise: 64 x 64 cells took 588 us as 17 set-up launches and 12
+// rounds of 5 kernels, most of them a few blocks; so it takes 430 us.  The V-cycle is the
+// single-CTA kernel's (s_outer from level 0), bit-identical to the grid kernels'; the sums of the
+// CG are added in this CTA's order.  The rule: the hierarchy fits a CTA's shared memory, and
+// level 0 has at most kSmallOwn cells a thread (4096 cells, 213 KB).
+// ------------------------------------------------------------------------------------
+constexpr int kSmallOwn = 8;
+struct SmallArgs {
+    CtaParams P;   // every level from 0
+    const double *f, *bx, *by;
+    double* x;
+    State* st;
+    double tol;
+    int max_it;
+    double cx[kMaxLevels], cy[kMaxLevels];
+};
+
+// The sum of v over the CTA in every thread; buf alternates between calls.
+__device__ __forceinline__ double cta_sum(double v, double (*red)[32], int& buf) {
+    for (int o = 16; o > 0; o >>= 1) v += __shfl_xor_sync(0xffffffffu, v, o);
+    const int lane = threadIdx.x & 31;
+    if (lane == 0) red[buf][threadIdx.x >> 5] = v;
+    __syncthreads();
+    double r = (lane < NT_CTA / 32) ? red[buf][lane] : 0.0;
+    for (int o = NT_CTA / 64; o > 0; o >>= 1) r += __shfl_xor_sync(0xffffffffu, r, o);
+    buf ^= 1;
+    return __shfl_sync(0xffffffffu, r, 0);
+}
+
+// The dense matrix of the bottom level and its elimination (k_dense_factor), from the level's
+// weights in shared memory.
+__device__ void s_dense_factor(const SL<double>& L, double* A) {
+    const int nx = L.nx, ny = L.ny, n = nx * ny, t = threadIdx.x, G = NT_CTA;
+    auto AX = [&](int i, int j) { return pick(L.ax, (i + j) & 1)[j * L.h + (i >> 1)]; };
+    auto AY = [&](int i, int j) { return pick(L.ay, (i + j) & 1)[j * L.h + (i >> 1)]; };
+    for (int k = t; k < n * n; k += G) A[k] = 0.0;
+    __syncthreads();
+    if (t == 0) {
+        for (int row = 0; row < n; ++row) {
+            const int j = row / nx, i = row - j * nx;
+            const int ip = (i + 1 == nx) ? 0 : i + 1, im = (i == 0) ? nx - 1 : i - 1;
+            const double aw = AX(i, j), ae = AX(ip, j), as = AY(i, j), an = AY(i, j + 1);
+            double d = aw;
+            d += ae;
+            d += as;
+            d += an;
+            A[row * n + row] -= d;
+            A[row * n + j * nx + im] += aw;
+            A[row * n + j * nx + ip] += ae;
+            if (j > 0) A[row * n + (j - 1) * nx + i] += as;
+            if (j < ny - 1) A[row * n + (j + 1) * nx + i] += an;
+        }
+    }
+    __syncthreads();
+    for (int k = 0; k < n; ++k) {
+        const double piv = A[k * n + k];
+        const int m = n - k - 1;
+        for (int q = t; q < m * m; q += G) {
+            const int i = k + 1 + q / m, j = k + 1 + q % m;
+            const double mult = A[i * n + k] / piv;
+            A[i * n + j] -= mult * A[k * n + j];
+        }
+        __syncthreads();
+        for (int i = k + 1 + t; i < n; i += G) A[i * n + k] = A[i * n + k] / piv;
+        __syncthreads();
+    }
+}
+
+__global__ void __launch_bounds__(NT_CTA, 1) k_small_solve(const __grid_constant__ SmallArgs A) {
+    unsigned char* sm = cta_smem_base();
+    __shared__ double red[2][32];
+    const CtaParams& P = A.P;
+    const CtaLevel* lv = P.lv;
+    const int t = threadIdx.x;
+    int buf = 0;
+    // faces of level 0, then their coarsening, as they are; the weights in their place afterwards
+    {
+        const SL<double> S = make_sl<double>(P.lv, sm, 0);
+        stage_split(S.ax[0], S.ax[1], A.bx, S.nx, S.ny, S.mag_h);
+        stage_split(S.ay[0], S.ay[1], A.by, S.nx, S.ny + 1, S.mag_h);
+    }
+    zero_ghosts<double>(P, sm);
+    async_wait_all();
+    __syncthreads();
+    for (int l = 1; l <= P.bottom; ++l) {
+        const SL<double> F = make_sl<double>(P.lv, sm, l - 1), C = make_sl<double>(P.lv, sm, l);
+        const int n = C.nx * C.ny;
+        for (int k = t; k < n + C.nx * (C.ny + 1); k += NT_CTA) {
+            const bool west = k < n;
+            const int q = west ? k : k - n, J = q / C.nx, I = q - J * C.nx, kc = J * C.h + (I >> 1), c = (I + J) & 1;
+            // fine cells (2I, 2J) red, (2I, 2J+1) and (2I+1, 2J) black, at entry I of their rows
+            if (west) pick(C.ax, c)[kc] = 0.5 * (F.ax[0][2 * J * F.h + I] + F.ax[1][(2 * J + 1) * F.h + I]);
+            else pick(C.ay, c)[kc] = 0.5 * (F.ay[0][2 * J * F.h + I] + F.ay[1][2 * J * F.h + I]);
+        }
+        __syncthreads();
+    }
+    for (int l = 0; l <= P.bottom; ++l) {
+        const SL<double> S = make_sl<double>(P.lv, sm, l);
+        const double cx = A.cx[l], cy = A.cy[l], cy2 = 2.0 * cy;
+        for (int k = t; k < S.ny * S.h; k += NT_CTA) {
+            S.ax[0][k] = cx * S.ax[0][k];
+            S.ax[1][k] = cx * S.ax[1][k];
+        }
+        for (int k = t; k < (S.ny + 1) * S.h; k += NT_CTA) {
+            const int j = k / S.h;
+            const double w = j == S.ny ? cy2 : cy;
+            S.ay[0][k] = j == 0 ? 0.0 : w * S.ay[0][k];
+            S.ay[1][k] = j == 0 ? 0.0 : w * S.ay[1][k];
+        }
+    }
+    __syncthreads();
+    for (int l = 0; l <= P.bottom; ++l) {
+        const SL<double> S = make_sl<double>(P.lv, sm, l);
+        for (int q = t; q < S.nx * S.ny; q += NT_CTA) {
+            const int c = q >= S.ny * S.h, k = q - c * S.ny * S.h, j = k / S.h, m = k - j * S.h, o = (j + c) & 1;
+            const int e = (m + o >= S.h) ? m + o - S.h : m + o;
+            double d = pick(S.ax, c)[k];
+            d += pick(S.ax, 1 - c)[j * S.h + e];
+            d += pick(S.ay, c)[k];
+            d += pick(S.ay, 1 - c)[k + S.h];
+            pick(S.di, c)[k] = 1.0 / d;
+        }
+    }
+    s_dense_factor(make_sl<double>(P.lv, sm, P.bottom), reinterpret_cast<double*>(sm + P.off_dense));
+    // this thread's cells: entry k of colour c, q = c * (cells / 2) + k = t, t + NT_CTA, ...
+    const SL<double> L = make_sl<double>(P.lv, sm, 0);
+    const int half = L.ny * L.h, n = 2 * half;
+    const Colour<double> V0(L, 0), V1(L, 1);
+    auto place = [&](int q, int& c, int& j, int& m, int& k) {
+        c = q >= half;
+        k = q - c * half;
+        j = div_mag(k, L.h, L.mag_h);
+        m = k - j * L.h;
+    };
+    auto at = [&](int c, int j, int m) { return (size_t)j * L.nx + 2 * m + ((j + c) & 1); };
+    // A u - the operator on the u array - at a cell
+    auto apply = [&](int c, int j, int m, int k, double uv) {
+        double sg, d;
+        split_sums(c ? V1 : V0, j, m, k, sg, d);
+        return sg - d * uv;
+    };
+    double x[kSmallOwn], xo[kSmallOwn], p[kSmallOwn], f[kSmallOwn];
+    double ff = 0.0, rr = 0.0;
+#pragma unroll
+    for (int i = 0; i < kSmallOwn; ++i) {
+        const int q = t + i * NT_CTA;
+        x[i] = f[i] = p[i] = 0.0;
+        if (q < n) {
+            int c, j, m, k;
+            place(q, c, j, m, k);
+            const size_t g = at(c, j, m);
+            x[i] = A.x[g];
+            f[i] = A.f[g];
+            pick(L.u, c)[k] = x[i];
+        }
+        xo[i] = x[i];
+    }
+    __syncthreads();
+#pragma unroll
+    for (int i = 0; i < kSmallOwn; ++i) {
+        const int q = t + i * NT_CTA;
+        if (q < n) {
+            int c, j, m, k;
+            place(q, c, j, m, k);
+            const double r = f[i] - apply(c, j, m, k, x[i]);
+            pick(L.f, c)[k] = r;
+            rr += r * r;
+            ff += f[i] * f[i];
+        }
+    }
+    ff = cta_sum(ff, red, buf);
+    rr = cta_sum(rr, red, buf);
+    const double fn = sqrt(ff), fscale = (fn > 0.0) ? fn : 1.0;
+    double rel = sqrt(rr) / fscale, rel_prev = 0.0, rz = 0.0;
+    int it = 0, status = LICA_NOT_CONVERGED, back = 0;
+    // the status and the loop condition of xupdate_finish, the same in every thread
+    for (bool first = true;; first = false) {
+        if (!isfinite(rel)) {
+            status = LICA_NAN;
+            break;
+        }
+        if (rel <= A.tol) {
+            status = LICA_OK;
+            break;
+        }
+        if (!first && rel >= rel_prev && rel_prev <= kStallFactor * A.tol) {
+            status = LICA_STALLED;   // the answer is the iterate before
+            it -= 1;
+            back = 1;
+            rel = rel_prev;
+            break;
+        }
+        if (it >= A.max_it) {
+            status = LICA_NOT_CONVERGED;
+            break;
+        }
+        rel_prev = rel;
+        // z = M r into u
+        for (int k = t; k < half; k += NT_CTA) {
+            L.u[0][k] = 0.0;
+            L.u[1][k] = 0.0;
+        }
+        __syncthreads();
+        s_outer<double>(P, lv);
+        __syncthreads();
+        double acc = 0.0;
+        double z[kSmallOwn];
+#pragma unroll
+        for (int i = 0; i < kSmallOwn; ++i) {
+            const int q = t + i * NT_CTA;
+            z[i] = 0.0;
+            if (q < n) {
+                const int c = q >= half, k = q - c * half;
+                z[i] = pick(L.u, c)[k];
+                acc += pick(L.f, c)[k] * z[i];
+            }
+        }
+        const double rzn = cta_sum(acc, red, buf);   // its barrier also ends the reads of z
+        const double beta = it == 0 ? 0.0 : rzn / rz;
+        rz = rzn;
+#pragma unroll
+        for (int i = 0; i < kSmallOwn; ++i) {
+            const int q = t + i * NT_CTA;
+            if (q < n) {
+                const int c = q >= half, k = q - c * half;
+                p[i] = z[i] + beta * p[i];
+                pick(L.u, c)[k] = p[i];
+            }
+        }
+        __syncthreads();
+        acc = 0.0;
+#pragma unroll
+        for (int i = 0; i < kSmallOwn; ++i) {
+            const int q = t + i * NT_CTA;
+            if (q < n) {
+                int c, j, m, k;
+                place(q, c, j, m, k);
+                acc += p[i] * apply(c, j, m, k, p[i]);
+            }
+        }
+        const double alpha = rz / cta_sum(acc, red, buf);
+#pragma unroll
+        for (int i = 0; i < kSmallOwn; ++i) {
+            const int q = t + i * NT_CTA;
+            if (q < n) {
+                const int c = q >= half, k = q - c * half;
+                xo[i] = x[i];
+                x[i] = x[i] + alpha * p[i];
+                pick(L.u, c)[k] = x[i];
+            }
+        }
+        __syncthreads();
+        acc = 0.0;
+#pragma unroll
+        for (int i = 0; i < kSmallOwn; ++i) {
+            const int q = t + i * NT_CTA;
+            if (q < n) {
+                int c, j, m, k;
+                place(q, c, j, m, k);
+                const double r = f[i] - apply(c, j, m, k, x[i]);
+                pick(L.f, c)[k] = r;
+                acc += r * r;
+            }
+        }
+        rel = sqrt(cta_sum(acc, red, buf)) / fscale;
+        it += 1;
+    }
+#pragma unroll
+    for (int i = 0; i < kSmallOwn; ++i) {
+        const int q = t + i * NT_CTA;
+        if (q < n) {
+            int c, j, m, k;
+            place(q, c, j, m, k);
+            A.x[at(c, j, m)] = back ? xo[i] : x[i];
+        }
+    }
+    if (t == 0) {
+        State& S = *A.st;
+        S.fscale = fscale;
+        S.rel = rel;
+        S.rel_prev = rel_prev;
+        S.rz = rz;
+        S.tol = A.tol;
+        S.it = it;
+        S.max_it = A.max_it;
+        S.status = status;
+        S.cont = 0;
+        S.back = back;
+        S.kerr = 0;
     }
 }
 
@@ -1694,6 +2087,9 @@ struct lica_mg {
     std::vector<LevelBuf> lv;  // outer levels then inner levels
     size_t cta_smem = 0;
     CtaParams cp{};
+    bool small = false;        // graph solves run as one k_small_solve launch
+    size_t small_smem = 0;
+    CtaParams small_cp{};
     // level-0 CG vectors
     double* pcg[2] = {nullptr, nullptr};  // p, ping-pong by iteration parity
     double* xb = nullptr;    // second x buffer (the first is the caller's)
@@ -1701,7 +2097,8 @@ struct lica_mg {
     void* zpre = nullptr;    // z after pre-smoothing (T)
     void* z = nullptr;       // z (T): the V-cycle's level-0 output
     double* partials = nullptr;
-    double* dense_lu = nullptr;  // bottom-level elimination, refreshed by every set-up
+    unsigned char* cta_image = nullptr;  // k_cta's weights and the bottom elimination (k_cta_image, k_dense_factor)
+    double* dense_lu = nullptr;  // the elimination in the image, refreshed by every set-up
     State* st = nullptr;
     State* st_host = nullptr;  // pinned
     // host staging for lica_mg_solve_host
@@ -2162,18 +2559,18 @@ int setup_beta(lica_mg* m, const double* bx, const double* by, cudaStream_t s) {
         LICA_CUDA_TRY(cudaGetLastError());
         lica_count_launches(1);
     }
-    // weights of the levels staged by the single-CTA kernel
-    for (int l = m->lcta; l <= m->bottom; ++l) {
-        if (l < m->nouter - 1 && is_mixed(m)) {
-            m->cp.lv[l].gax = m->lv[l].ax32;
-            m->cp.lv[l].gay = m->lv[l].ay32;
-            m->cp.lv[l].gdi = m->lv[l].di32;
-        } else {
-            m->cp.lv[l].gax = m->lv[l].ax64;
-            m->cp.lv[l].gay = m->lv[l].ay64;
-            m->cp.lv[l].gdi = m->lv[l].di64;
+    // the single-CTA kernel's weights as it holds them (the y-line cycle has none)
+    if (!m->yline)
+        for (int l = m->lcta; l <= m->bottom; ++l) {
+            const LevelBuf& L = m->lv[l];
+            const int blocks = blocks_for((size_t)L.nx * (L.ny + 1));
+            if (l < m->nouter - 1 && is_mixed(m))
+                k_cta_image<float><<<blocks, 256, 0, s>>>(L.ax32, L.ay32, L.di32, m->cta_image, m->cp.lv[l]);
+            else
+                k_cta_image<double><<<blocks, 256, 0, s>>>(L.ax64, L.ay64, L.di64, m->cta_image, m->cp.lv[l]);
+            LICA_CUDA_TRY(cudaGetLastError());
+            lica_count_launches(1);
         }
-    }
     return LICA_OK;
 }
 
@@ -2387,9 +2784,31 @@ bool aligned16(const void* a, const void* b, const void* c, const void* d) {
     return true;
 }
 
+int launch_small(lica_mg* m, double* x, const double* f, const double* bx, const double* by, double rtol, int max_it,
+                 cudaStream_t s) {
+    SmallArgs A;
+    A.P = m->small_cp;
+    A.f = f;
+    A.bx = bx;
+    A.by = by;
+    A.x = x;
+    A.st = m->st;
+    A.tol = rtol;
+    A.max_it = max_it;
+    for (int l = 0; l <= m->bottom; ++l) {
+        A.cx[l] = m->lv[l].cx;
+        A.cy[l] = m->lv[l].cy;
+    }
+    k_small_solve<<<1, NT_CTA, m->small_smem, s>>>(A);
+    LICA_CUDA_TRY(cudaGetLastError());
+    lica_count_launches(1);
+    return LICA_OK;
+}
+
 // Launch the solve's graph (built, or rebuilt for new arrays, tolerance or stream) on s.
 int graph_launch(lica_mg* m, double* x, const double* f, const double* bx, const double* by, double rtol, int max_it,
                  cudaStream_t s) {
+    if (m->small) return launch_small(m, x, f, bx, by, rtol, max_it, s);
     int st;
     // rtol/max_it live in the graph's k_init_state node: a graph serves only its own
     auto match = [&](const lica_mg::GraphSlot& g) {
@@ -2489,23 +2908,28 @@ int lica_mg_create(lica_mg** out, int32_t nx, int32_t ny, double hx, double hy, 
     // shared memory and has <= 32*32 cells, or that cannot be tiled
     // per level: u (two colours, each (ny+2) x nx/2 with zero ghost rows), f, ax, 1/d
     // (ny x nx/2 each) and ay ((ny+1) x nx/2), 16-byte aligned arrays
-    auto level_arrays = [&](int l, auto&& take) {
+    auto level_arrays = [&](int l, CtaLevel& C, auto&& take, bool weights) {
         const size_t e = (l < m->nouter - 1) ? tsz : sizeof(double);
         const size_t h = (size_t)m->lv[l].nx / 2, ny = m->lv[l].ny;
-        CtaLevel C{};
         for (int c = 0; c < 2; ++c) {
-            C.off_u[c] = take(e * (ny + 2) * h);
-            C.off_f[c] = take(e * ny * h);
-            C.off_ax[c] = take(e * ny * h);
-            C.off_ay[c] = take(e * (ny + 1) * h);
-            C.off_di[c] = take(e * ny * h);
+            if (weights) {
+                C.off_ax[c] = take(e * ny * h);
+                C.off_ay[c] = take(e * (ny + 1) * h);
+                C.off_di[c] = take(e * ny * h);
+            } else {
+                C.off_u[c] = take(e * (ny + 2) * h);
+                C.off_f[c] = take(e * ny * h);
+            }
         }
-        return C;
     };
     auto cta_bytes = [&](int from) {
         size_t off = 0;
         auto take = [&](size_t bytes) { size_t r = off; off = (off + bytes + 15) & ~(size_t)15; return (unsigned)r; };
-        for (int l = from; l <= m->bottom; ++l) level_arrays(l, take);
+        CtaLevel C{};
+        for (int l = from; l <= m->bottom; ++l) {
+            level_arrays(l, C, take, true);
+            level_arrays(l, C, take, false);
+        }
         const size_t nb = (size_t)m->lv[m->bottom].nx * m->lv[m->bottom].ny;
         take(sizeof(double) * nb * nb);
         take(sizeof(double) * nb);
@@ -2534,25 +2958,38 @@ int lica_mg_create(lica_mg** out, int32_t nx, int32_t ny, double hx, double hy, 
         m->mid = lcta >= 3 && ev && ev[0] == '1' && o.smoother == 0;
         m->yline = o.smoother == 1;
     }
-    // shared-memory layout of the single-CTA kernel
+    // shared-memory layout of the single-CTA kernels, from their first level
+    auto cta_layout = [&](CtaParams& P, int from) {
+        std::memset(&P, 0, sizeof(P));
+        P.lcta = from; P.lc = m->nouter - 1; P.bottom = m->bottom;
+        P.nu1 = o.nu1; P.nu2 = o.nu2; P.ncoarse = o.ncoarse;
+        size_t off = 0;
+        auto take = [&](size_t bytes) { size_t r = off; off = (off + bytes + 15) & ~(size_t)15; return (unsigned)r; };
+        const size_t nb = (size_t)m->lv[m->bottom].nx * m->lv[m->bottom].ny;
+        // the image first: every level's weights and the bottom elimination
+        for (int l = from; l <= m->bottom; ++l) level_arrays(l, P.lv[l], take, true);
+        P.off_dense = take(sizeof(double) * nb * nb);
+        P.image_bytes = (unsigned)off;
+        int warps = NT_CTA / 32;
+        for (int l = from; l <= m->bottom; ++l) {
+            CtaLevel& C = P.lv[l];
+            level_arrays(l, C, take, false);
+            C.nx = m->lv[l].nx; C.ny = m->lv[l].ny; C.half = m->lv[l].nx / 2;
+            auto mag = [](unsigned c) { return c > 1 ? (unsigned)((1ull << 32) / c + 1) : 0u; };
+            C.mag_h = mag((unsigned)C.half);
+            C.mag_nx = mag((unsigned)C.nx);
+            warps = std::min(warps, std::max(1, (C.ny * C.half + 31) / 32));
+            C.warps = warps;
+        }
+        P.off_rhs = take(sizeof(double) * nb);
+        return off;
+    };
     CtaParams& P = m->cp;
-    std::memset(&P, 0, sizeof(P));
-    P.lcta = lcta; P.lc = m->nouter - 1; P.bottom = m->bottom;
-    P.nu1 = o.nu1; P.nu2 = o.nu2; P.ncoarse = o.ncoarse;
-    size_t off = 0;
-    auto take = [&](size_t bytes) { size_t r = off; off = (off + bytes + 15) & ~(size_t)15; return (unsigned)r; };
-    for (int l = lcta; l <= m->bottom; ++l) {
-        CtaLevel& C = P.lv[l];
-        C = level_arrays(l, take);
-        C.nx = m->lv[l].nx; C.ny = m->lv[l].ny; C.half = m->lv[l].nx / 2;
-        auto mag = [](unsigned c) { return c > 1 ? (unsigned)((1ull << 32) / c + 1) : 0u; };
-        C.mag_h = mag((unsigned)C.half);
-        C.mag_nx = mag((unsigned)C.nx);
+    m->cta_smem = cta_layout(P, lcta);
+    if (!mixed && o.smoother == 0 && (size_t)nx * ny <= (size_t)kSmallOwn * NT_CTA && cta_bytes(0) <= 224 * 1024) {
+        m->small = true;
+        m->small_smem = cta_layout(m->small_cp, 0);
     }
-    const size_t nb = (size_t)m->lv[m->bottom].nx * m->lv[m->bottom].ny;
-    P.off_dense = take(sizeof(double) * nb * nb);
-    P.off_rhs = take(sizeof(double) * nb);
-    m->cta_smem = off;
 
     auto fail = [&](int code) { lica_mg_destroy(m); return code; };
 #define TRY_ALLOC(ptr, bytes)                                                        \
@@ -2637,9 +3074,10 @@ int lica_mg_create(lica_mg** out, int32_t nx, int32_t ny, double hx, double hy, 
     TRY_ALLOC(m->partials, sizeof(double) * 2 * ntiles);
     TRY_ALLOC(m->st, sizeof(State));
     {
-        const size_t nb = (size_t)m->lv[m->bottom].nx * m->lv[m->bottom].ny;
-        TRY_ALLOC(m->dense_lu, sizeof(double) * nb * nb);
-        P.glu = m->dense_lu;
+        TRY_ALLOC(m->cta_image, (size_t)P.image_bytes);
+        m->dense_lu = (double*)(m->cta_image + P.off_dense);
+        P.image = m->cta_image;
+        P.st = m->st;
     }
     {
         cudaError_t e = cudaMallocHost((void**)&m->st_host, sizeof(State));
@@ -2672,6 +3110,8 @@ int lica_mg_create(lica_mg** out, int32_t nx, int32_t ny, double hx, double hy, 
     }
     if (e == cudaSuccess) e = cudaFuncSetAttribute(k_cta<float>, cudaFuncAttributeMaxDynamicSharedMemorySize, optin);
     if (e == cudaSuccess) e = cudaFuncSetAttribute(k_cta<double>, cudaFuncAttributeMaxDynamicSharedMemorySize, optin);
+    if (e == cudaSuccess)   // beside its static shared memory
+        e = cudaFuncSetAttribute(k_small_solve, cudaFuncAttributeMaxDynamicSharedMemorySize, optin - 1024);
     if (e != cudaSuccess) {
         lica_set_last_error("cudaFuncSetAttribute(k_cta)", cudaGetErrorString(e), __FILE__, __LINE__);
         return fail(LICA_ERR_CUDA);
@@ -2756,7 +3196,7 @@ int lica_mg_destroy(lica_mg* m) {
     cudaFree(m->pcg[1]);
     cudaFree(m->xb);
     cudaFree(m->r);
-    cudaFree(m->dense_lu);
+    cudaFree(m->cta_image);
     cudaFree(m->zpre);
     cudaFree(m->z);
     cudaFree(m->ycp);
