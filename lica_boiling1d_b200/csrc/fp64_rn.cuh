@@ -21,12 +21,17 @@
 namespace lica {
 namespace rn {
 
-// exponent of b within 2^-400 .. 2^400, and not a mantissa of all ones
-__device__ __forceinline__ bool ordinary(double b) {
-    const int hi = __double2hiint(b), lo = __double2loint(b);
-    const unsigned e = ((unsigned)hi >> 20) & 0x7ffu;
-    return (e - 623u) <= 800u && !((hi & 0xfffff) == 0xfffff && lo == -1);
+// |b| within 2^-400 .. 2^400
+__device__ __forceinline__ bool in_range(double b) {
+    return ((unsigned)__double2hiint(b) & 0x7fffffffu) - 0x26f00000u < 0x32000000u;
 }
+// and its mantissa not all ones
+__device__ __forceinline__ bool ordinary(double b) {
+    return in_range(b) && !(__double2loint(b) == -1 && (__double2hiint(b) & 0xfffff) == 0xfffff);
+}
+
+// ordinary, and a little less: without a branch, for the inside of a chain
+__device__ __forceinline__ bool plain(double b) { return in_range(b) & (__double2loint(b) != -1); }
 
 __device__ __forceinline__ double recip(double b) {
     double y;

@@ -321,7 +321,12 @@ __device__ __forceinline__ double hjweno(double a, double b, double cc, double d
     const double a1 = rn::recip(e1), a2 = rn::quot(6.0, e2, rn::recip(e2)), a3 = rn::quot(3.0, e3, rn::recip(e3));
     const double sum = a1 + a2 + a3, rs = rn::recip(sum);
     const double w1 = rn::quot(a1, sum, rs), w3 = rn::quot(a3, sum, rs);
-    ok = ok && rn::ordinary(e1) && rn::ordinary(e2) && rn::ordinary(e3) && rn::ordinary(sum);
+    // every e is at least eps^2 and the sum, of quotients by them, in between: what is left of
+    // rn::ordinary is the terms' upper end (a NaN is above it) and the mantissas of all ones
+    const unsigned top = max(max((unsigned)__double2hiint(e1), (unsigned)__double2hiint(e2)), (unsigned)__double2hiint(e3));
+    const unsigned low = max(max((unsigned)__double2loint(e1), (unsigned)__double2loint(e2)),
+                             max((unsigned)__double2loint(e3), (unsigned)__double2loint(sum)));
+    ok = ok && top < 0x58f00000u && low != 0xffffffffu;   // below 2^400
     return 1.0 / 3.0 * w1 * (a - 2.0 * b + cc) + 1.0 / 6.0 * (w3 - 0.5) * (b - 2.0 * cc + dd);
 }
 
@@ -472,7 +477,7 @@ __device__ __forceinline__ double godunov(double sg, double ap, double am) {
 
 // REINITIALIZATION_RK3, two_phase.f:2174-2445 (1-D), of one cell: dz its central difference,
 // a0 its phi at entry; Peng's smoothed sign with eps = min(h)^2.  The x and y parts of GODUNOV
-// are 0, and the root of a square is the value itself where the square neither over- nor
+// are 0 (PLAIN: with the plain operators; else a0 is ordinary and the others are tested), and the root of a square is the value itself where the square neither over- nor
 // underflows (a square and its root each rounded to nearest); below that 1 less it is 1 both ways.
 template <bool PLAIN>
 __device__ __forceinline__ double reinit_cell(double phi, double a0, double dz, double dm, double dpl, double eps,
@@ -485,7 +490,7 @@ __device__ __forceinline__ double reinit_cell(double phi, double a0, double dz, 
     } else {
         const double den = rn::root(sq, ok);
         sg = rn::quot(a0, den, rn::recip(den));
-        ok = ok && rn::ordinary(sq) && rn::ordinary(a0) && rn::ordinary(den);
+        ok = ok && rn::in_range(sq) && __double2loint(den) != -1;   // a0: the caller's
     }
     const double az = godunov(sg, dpl, dm);
     double mod = fabs(az);
@@ -572,6 +577,7 @@ __device__ inline void reinitialization(Ctx& c, int ilimit) {
         const bool mine = c.lane < b.c10;
         const bool first_order = c.lane >= b.c8;
         const double a0 = s->phi[b.i];
+        const bool ok0 = rn::ordinary(a0);
         double p = a0;
         for (int it = 0; it < ilimit; ++it) {
             const double rk = p;
@@ -580,7 +586,7 @@ __device__ inline void reinitialization(Ctx& c, int ilimit) {
                 const double dz = 0.5 * (pp - pm) * c.ssdzf;
                 const double fm = (p - pm) * c.ssdzf, fp = (pp - p) * c.ssdzf;
                 double dm, dpl;
-                bool ok = true;
+                bool ok = ok0;
                 compact_weno<false>(c, b, dm, dpl, ok);
                 double q = reinit_cell<false>(p, a0, dz, first_order ? fm : dm, first_order ? fp : dpl, eps, redtl, ok);
                 if (!__all_sync(0xffffffffu, ok)) q = reinit_stage_plain(c.s, b.wi, first_order, c.ssdzf, p, a0, eps, redtl, b.i);
