@@ -50,6 +50,43 @@ extern "C" void lica_count_launches(int64_t n);
 namespace lica {
 namespace mg {
 
+// Chained launches.  The kernels of a solve are a chain of short launches, each of which needs all
+// of the one before it, and between two of them the chip stood idle for the launch, the CTAs' start
+// and their first loads.  A kernel launched by launch_next may start early, set itself up and read
+// what no kernel since the set-up writes (the weights); it waits in after_previous() until the one
+// before has ended, which itself waited for the one before it, and its stores can be seen.  What the
+// kernels before wrote is read through pointers that are not both const and __restrict__, so that no
+// read of it can be moved above the wait.
+//
+// EARLY: the next kernel may start once all CTAs of this one have, otherwise once they have all
+// passed the wait.  A kernel starts only after every CTA of the one before it has, so those that
+// wait take no room from one that must still start.  Early is better where the CTAs are large and
+// their weights many (red-black, 1024 x 1024 cells: a solve 1.57 -> 1.49 ms chained, 1.45 early;
+// two 512 x 1536 film steps 9.9 -> 9.66, 9.50), late where a launch is a few small CTAs (y-lines,
+// 256 x 256: 12.1 -> 11.0 ms, 11.6 early).
+template <bool EARLY = true>
+__device__ __forceinline__ void after_previous() {
+    if (EARLY) asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
+    asm volatile("griddepcontrol.wait;" ::: "memory");
+    if (!EARLY) asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
+}
+
+template <typename... P, typename... A>
+cudaError_t launch_next(void (*kernel)(P...), dim3 grid, dim3 block, size_t smem, cudaStream_t s, A... args) {
+    cudaLaunchConfig_t cfg = {};
+    cfg.gridDim = grid;
+    cfg.blockDim = block;
+    cfg.dynamicSmemBytes = smem;
+    cfg.stream = s;
+    cudaLaunchAttribute at[1];
+    at[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    at[0].val.programmaticStreamSerializationAllowed = 1;
+    cfg.attrs = at;
+    cfg.numAttrs = 1;
+    return cudaLaunchKernelEx(&cfg, kernel, static_cast<P>(args)...);
+}
+
+
 constexpr int TX = 32;
 constexpr int TY = 32;
 constexpr int NT = 256;          // threads of a CG / set-up grid-kernel CTA
@@ -172,8 +209,9 @@ struct RBGeom {
 // Loads f, 1/d and the four weights of the thread's cells (zero outside the domain rows).
 // COH: f was written earlier in the same launch (the cross-level kernels), so it is read
 // through L2 (ld.global.cg), never through the non-coherent read-only path.
-template <typename T, class C, bool COH = false>
-__device__ __forceinline__ void rb_load(RBCells<T, C::K>& cl, const RBGeom<C>& g, const T* __restrict__ f,
+// NEXT: a chained launch, f is read after the kernel before has ended.
+template <typename T, class C, bool COH = false, bool NEXT = false>
+__device__ __forceinline__ void rb_load(RBCells<T, C::K>& cl, const RBGeom<C>& g, const T* f,
                                         const T* __restrict__ ax, const T* __restrict__ ay,
                                         const T* __restrict__ dinv, int nx, int ny, int gi0, int gj0) {
     int i = gi0 + g.x;
@@ -189,7 +227,7 @@ __device__ __forceinline__ void rb_load(RBCells<T, C::K>& cl, const RBGeom<C>& g
             T vf = T(0), vd = T(0), vw = T(0), ve = T(0), vs = T(0), vn = T(0);
             if (ok) {
                 const int o = j * nx;
-                vf = COH ? __ldcg(f + o + i) : f[o + i];
+                if (!NEXT) vf = COH ? __ldcg(f + o + i) : f[o + i];
                 vd = dinv[o + i];
                 vw = ax[o + i];
                 ve = ax[o + ip];
@@ -204,6 +242,14 @@ __device__ __forceinline__ void rb_load(RBCells<T, C::K>& cl, const RBGeom<C>& g
             cl.an[c][k] = vn;
             cl.valid |= (ok ? 1u : 0u) << (c * C::K + k);
         }
+    }
+    if (NEXT) {
+        after_previous();
+#pragma unroll
+        for (int c = 0; c < 2; ++c)
+#pragma unroll
+            for (int k = 0; k < C::K; ++k)
+                if (cl.valid & (1u << (c * C::K + k))) cl.f[c][k] = f[(gj0 + g.row(c, k)) * nx + i];
     }
     // The west read of column 0 (east read of column RX-1) lands on the previous (next)
     // row's far column, a cell of the same colour: the edge columns, outside the valid
@@ -319,7 +365,7 @@ __device__ __forceinline__ void down_body(const RBCells<T, RBCfg<NSW, TXX, TYY, 
 
 template <typename T, int NSW, int TXX, int TYY, int R>
 __global__ void __launch_bounds__(RBCfg<NSW, TXX, TYY, R>::NTH, 2)
-    k_down(const T* __restrict__ f, const T* __restrict__ ax, const T* __restrict__ ay, const T* __restrict__ dinv,
+    k_down(const T* f, const T* __restrict__ ax, const T* __restrict__ ay, const T* __restrict__ dinv,
            T* __restrict__ u_out, T* __restrict__ fc_out, int nx, int ny) {
     using C = RBCfg<NSW, TXX, TYY, R>;
     __shared__ __align__(16) T su[C::WORDS];
@@ -327,7 +373,7 @@ __global__ void __launch_bounds__(RBCfg<NSW, TXX, TYY, R>::NTH, 2)
     const RBGeom<C> g;
     RBCells<T, C::K> cl;
     rb_zero<T, C>(su);
-    rb_load<T, C>(cl, g, f, ax, ay, dinv, nx, ny, gi0, gj0);
+    rb_load<T, C, false, true>(cl, g, f, ax, ay, dinv, nx, ny, gi0, gj0);
     __syncthreads();  // zero fill done
     down_body<T, NSW, TXX, TYY, R>(cl, g, su, u_out, fc_out, nx, blockIdx.x * TXX, blockIdx.y * TYY);
 }
@@ -383,9 +429,9 @@ __device__ __forceinline__ double up_body(const RBCells<T, RBCfg<NSW, TXX, TYY, 
 
 template <typename T, int NSW, int TXX, int TYY, int R, bool LEVEL0>
 __global__ void __launch_bounds__(RBCfg<NSW, TXX, TYY, R>::NTH, std::is_same<T, float>::value ? 3 : 2)
-    k_up(const T* __restrict__ u_pre, T* __restrict__ u_post, const T* __restrict__ uc, const T* __restrict__ f,
+    k_up(const T* u_pre, T* __restrict__ u_post, const T* uc, const T* f,
          const T* __restrict__ ax, const T* __restrict__ ay, const T* __restrict__ dinv, int nx, int ny,
-         State* __restrict__ st, double* __restrict__ partials) {
+         State* st, double* partials) {
     using C = RBCfg<NSW, TXX, TYY, R>;
     __shared__ __align__(16) T su[C::WORDS];
     __shared__ double red[32];
@@ -394,7 +440,7 @@ __global__ void __launch_bounds__(RBCfg<NSW, TXX, TYY, R>::NTH, std::is_same<T, 
     const RBGeom<C> g;
     RBCells<T, C::K> cl;
     rb_zero<T, C>(su);
-    rb_load<T, C>(cl, g, f, ax, ay, dinv, nx, ny, gi0, gj0);
+    rb_load<T, C, false, true>(cl, g, f, ax, ay, dinv, nx, ny, gi0, gj0);
     T uv[2][C::K];
     {
         int i = gi0 + g.x;
@@ -604,10 +650,10 @@ constexpr int PAREA = PRX * PRY;
 // device by the iteration parity (p_old = pp[it&1], p_new = pp[(it+1)&1]), so the halo is
 // always read from a buffer no block of this launch writes.
 template <typename TZ>
-__global__ void __launch_bounds__(NT) k_pupdate(double* __restrict__ p0, double* __restrict__ p1,
-                                                const TZ* __restrict__ z, const double* __restrict__ ax,
+__global__ void __launch_bounds__(NT) k_pupdate(double* p0, double* p1,
+                                                const TZ* z, const double* __restrict__ ax,
                                                 const double* __restrict__ ay, int nx, int ny,
-                                                State* __restrict__ st, double* __restrict__ partials) {
+                                                State* st, double* partials) {
     extern __shared__ __align__(16) unsigned char smem_raw[];
     double* sp = reinterpret_cast<double*>(smem_raw);
     double* sax = sp + PAREA;
@@ -615,13 +661,14 @@ __global__ void __launch_bounds__(NT) k_pupdate(double* __restrict__ p0, double*
     TZ* sz = reinterpret_cast<TZ*>(say + PAREA);
     __shared__ double red[32];
     const int gi0 = blockIdx.x * TX - PH, gj0 = blockIdx.y * TY - PH;
+    load_plain(sax, ax, nx, ny, gi0, gj0);
+    load_plain(say, ay, nx, ny + 1, gi0, gj0);
+    after_previous();
     const int par = st->it & 1;
-    const double* __restrict__ p = par ? p1 : p0;
+    const double* p = par ? p1 : p0;
     double* __restrict__ pn = par ? p0 : p1;
     load_plain(sp, p, nx, ny, gi0, gj0);
     load_plain(sz, z, nx, ny, gi0, gj0);
-    load_plain(sax, ax, nx, ny, gi0, gj0);
-    load_plain(say, ay, nx, ny + 1, gi0, gj0);
     const double beta = st->beta;
     async_wait_all();
     __syncthreads();
@@ -652,11 +699,10 @@ __device__ __noinline__ void xupdate_finish(State* __restrict__ st, double tot, 
                                             cudaGraphConditionalHandle cond, int use_cond);
 
 template <typename TR>
-__global__ void __launch_bounds__(NT) k_xupdate(double* __restrict__ x0, double* __restrict__ x1,
-                                                const double* __restrict__ p0, const double* __restrict__ p1,
+__global__ void __launch_bounds__(NT) k_xupdate(double* x0, double* x1, const double* p0, const double* p1,
                                                 const double* __restrict__ f, const double* __restrict__ ax,
                                                 const double* __restrict__ ay, TR* __restrict__ r_out, int nx, int ny,
-                                                State* __restrict__ st, double* __restrict__ partials, int first,
+                                                State* st, double* partials, int first,
                                                 cudaGraphConditionalHandle cond, int use_cond) {
     extern __shared__ __align__(16) unsigned char smem_raw[];
     double* sxv = reinterpret_cast<double*>(smem_raw);
@@ -666,15 +712,16 @@ __global__ void __launch_bounds__(NT) k_xupdate(double* __restrict__ x0, double*
     double* sf = say + PAREA;
     __shared__ double red[32];
     const int gi0 = blockIdx.x * TX - PH, gj0 = blockIdx.y * TY - PH;
-    const int par = first ? 0 : (st->it & 1);
-    const double* __restrict__ x = par ? x1 : x0;
-    double* __restrict__ xn = par ? x0 : x1;
-    const double* __restrict__ p = par ? p0 : p1;
-    load_plain(sxv, x, nx, ny, gi0, gj0);
-    if (!first) load_plain(spv, p, nx, ny, gi0, gj0);
     load_plain(sax, ax, nx, ny, gi0, gj0);
     load_plain(say, ay, nx, ny + 1, gi0, gj0);
     load_plain(sf, f, nx, ny, gi0, gj0);
+    after_previous();
+    const int par = first ? 0 : (st->it & 1);
+    const double* x = par ? x1 : x0;
+    double* __restrict__ xn = par ? x0 : x1;
+    const double* p = par ? p0 : p1;
+    load_plain(sxv, x, nx, ny, gi0, gj0);
+    if (!first) load_plain(spv, p, nx, ny, gi0, gj0);
     const double alpha = first ? 0.0 : st->alpha;
     async_wait_all();
     __syncthreads();
@@ -1207,6 +1254,7 @@ __global__ void __launch_bounds__(NT_CTA, 1) k_cta(const __grid_constant__ CtaPa
                      : "memory");
     }
     zero_ghosts<T>(P, sm);
+    after_previous();
     {
         const CtaLevel& L = P.lv[P.lcta];
         const T* fin = reinterpret_cast<const T*>(P.f_in);
@@ -1276,8 +1324,9 @@ __global__ void __launch_bounds__(NT_CTA, 1) k_cta(const __grid_constant__ CtaPa
 
 // The weights of level l (row-major AX, AY, DINV) into the image at the level's offsets.
 template <typename E>
-__global__ void k_cta_image(const E* __restrict__ ax, const E* __restrict__ ay, const E* __restrict__ di,
-                            unsigned char* __restrict__ image, const CtaLevel L) {
+__global__ void k_cta_image(const E* ax, const E* ay, const E* di, unsigned char* __restrict__ image,
+                            const CtaLevel L) {
+    after_previous();
     const int nx = L.nx, n = nx * L.ny;
     for (int k = blockIdx.x * blockDim.x + threadIdx.x; k < n + nx; k += gridDim.x * blockDim.x) {
         const int j = k / nx, i = k - j * nx, c = (i + j) & 1, at = j * L.half + (i >> 1);
@@ -1588,8 +1637,9 @@ __global__ void __launch_bounds__(NT_CTA, 1) k_small_solve(const __grid_constant
 // set-up kernels
 // ------------------------------------------------------------------------------------
 template <typename T>
-__global__ void k_coarsen_beta(const T* __restrict__ bxf, const T* __restrict__ byf, T* __restrict__ bxc,
+__global__ void k_coarsen_beta(const T* bxf, const T* byf, T* __restrict__ bxc,
                                T* __restrict__ byc, int nxc, int nyc) {
+    after_previous();
     const int nxf = 2 * nxc;
     const int n = nxc * nyc, nb = nxc * (nyc + 1);
     for (int k = blockIdx.x * blockDim.x + threadIdx.x; k < n + nb; k += gridDim.x * blockDim.x) {
@@ -1607,10 +1657,11 @@ __global__ void k_coarsen_beta(const T* __restrict__ bxf, const T* __restrict__ 
 // AX = cx*bx; AY = cy*by inside, 0 on the bottom wall row, (2*cy)*by on the top wall row;
 // DINV = 1/d with d = ((aw + ae) + as) + an, the diagonal the oracle forms per update.
 template <typename T>
-__global__ void k_scale_beta(const T* __restrict__ bx, const T* __restrict__ by, T* __restrict__ ax,
+__global__ void k_scale_beta(const T* bx, const T* by, T* __restrict__ ax,
                              T* __restrict__ ay, T* __restrict__ dinv, int nx, int ny, T cx, T cy) {
     const size_t n = (size_t)nx * ny, nb = n + nx;
     const T cy2 = T(2) * cy;
+    after_previous();
     for (size_t k = blockIdx.x * (size_t)blockDim.x + threadIdx.x; k < n + nb; k += (size_t)gridDim.x * blockDim.x) {
         if (k < n) {
             const size_t j = k / nx, i = k - j * nx;
@@ -1636,11 +1687,12 @@ __global__ void k_scale_beta(const T* __restrict__ bx, const T* __restrict__ by,
 // Elimination of the bottom level's dense matrix, done once per solve in shared memory:
 // the oracle's dense_solve without its right-hand side (same assembly, pivots and
 // products).  Output: U on and above the diagonal, the multipliers A[i][k] / piv below.
-__global__ void k_dense_factor(const double* __restrict__ ax, const double* __restrict__ ay,
+__global__ void k_dense_factor(const double* ax, const double* ay,
                                double* __restrict__ out, int nx, int ny) {
     extern __shared__ __align__(16) double A[];
     const int n = nx * ny, t = threadIdx.x, G = blockDim.x;
     for (int k = t; k < n * n; k += G) A[k] = 0.0;
+    after_previous();
     __syncthreads();
     if (t == 0) {
         for (int row = 0; row < n; ++row) {
@@ -1674,7 +1726,8 @@ __global__ void k_dense_factor(const double* __restrict__ ax, const double* __re
     for (int k = t; k < n * n; k += G) out[k] = A[k];
 }
 
-__global__ void k_to_float(const double* __restrict__ a, float* __restrict__ b, size_t n) {
+__global__ void k_to_float(const double* a, float* __restrict__ b, size_t n) {
+    after_previous();
     for (size_t k = blockIdx.x * (size_t)blockDim.x + threadIdx.x; k < n; k += (size_t)gridDim.x * blockDim.x)
         b[k] = float(a[k]);
 }
@@ -1798,7 +1851,7 @@ constexpr int kYlThreads = 128;
 constexpr int kYlArrays = 7;
 __host__ __device__ inline int yl_pitch(int ny) { return (ny + 7) & ~7; }
 __global__ void __launch_bounds__(kYlThreads)
-    k_yline_column(double* __restrict__ u, const double* __restrict__ f, const double* __restrict__ ax,
+    k_yline_column(double* u, const double* f, const double* __restrict__ ax,
                    const double* __restrict__ ay, const double* __restrict__ yc, const double* __restrict__ yd,
                    const double* __restrict__ yi, int nx, int ny, int parity) {
     extern __shared__ double ysm[];
@@ -1810,18 +1863,24 @@ __global__ void __launch_bounds__(kYlThreads)
     for (int j = tid; j < np; j += kYlThreads) {
         if (j < ny) {
             const size_t k = (size_t)j * nx;
-            double r = f[k + i];
-            r -= ax[k + i] * u[k + im];
-            r -= ax[k + ip] * u[k + ip];
-            rhs[j] = r;
             as[j] = ay[k + i];
             den[j] = yd[k + i];
             inv[j] = yi[k + i];
             c[j] = yc[k + i];
+            e[j] = ax[k + i];
+            x[j] = ax[k + ip];
         } else {
             rhs[j] = as[j] = c[j] = 0.0;
             den[j] = inv[j] = 1.0;
         }
+    }
+    after_previous<false>();
+    for (int j = tid; j < ny; j += kYlThreads) {  // the thread's own rows of e and x
+        const size_t k = (size_t)j * nx;
+        double r = f[k + i];
+        r -= e[j] * u[k + im];
+        r -= x[j] * u[k + ip];
+        rhs[j] = r;
     }
     __syncthreads();
     const bool first = tid == 0;
@@ -1898,9 +1957,10 @@ __global__ void __launch_bounds__(kYlThreads)
 
 // The elimination of every column of a level: yc = c'_j, yd = the pivots, yi = their reciprocals.
 __global__ void __launch_bounds__(kYlThreads)
-    k_yline_factor(const double* __restrict__ ax, const double* __restrict__ ay, double* __restrict__ yc,
-                   double* __restrict__ yd, double* __restrict__ yi, int nx, int ny) {
+    k_yline_factor(const double* ax, const double* ay, double* __restrict__ yc, double* __restrict__ yd,
+                   double* __restrict__ yi, int nx, int ny) {
     extern __shared__ double ysm[];
+    after_previous();
     const int np = yl_pitch(ny), tid = threadIdx.x;
     double *as = ysm, *sup = ysm + np, *diag = ysm + 2 * np, *c = ysm + 3 * np, *den = ysm + 4 * np,
            *inv = ysm + 5 * np;
@@ -1958,10 +2018,12 @@ __global__ void __launch_bounds__(kYlThreads)
 }
 
 // Residual r = f - (s - d u) of the four children of coarse cell (I, J) and their 2x2
-// average, fc = (r00 + r01) + (r10 + r11) times 1/4 in the oracle's order.
-__global__ void k_resid_restrict(const double* __restrict__ u, const double* __restrict__ f,
-                                 const double* __restrict__ ax, const double* __restrict__ ay, double* __restrict__ fc,
-                                 int nx, int ny) {
+// average, fc = (r00 + r01) + (r10 + r11) times 1/4 in the oracle's order; the coarse iterate
+// starts from zero.
+__global__ void k_resid_restrict(const double* u, const double* f, const double* __restrict__ ax,
+                                 const double* __restrict__ ay, double* __restrict__ fc, double* __restrict__ uc, int nx,
+                                 int ny) {
+    after_previous<false>();
     const int ncx = nx >> 1, ncy = ny >> 1;
     const int I = blockIdx.x * blockDim.x + threadIdx.x, J = blockIdx.y * blockDim.y + threadIdx.y;
     if (I >= ncx || J >= ncy) return;
@@ -1989,10 +2051,12 @@ __global__ void k_resid_restrict(const double* __restrict__ u, const double* __r
         }
     }
     fc[(size_t)J * ncx + I] = 0.25 * ((r[0][0] + r[0][1]) + (r[1][0] + r[1][1]));
+    uc[(size_t)J * ncx + I] = 0.0;
 }
 
 // u += P uc, piecewise constant.
-__global__ void k_prolong_add(double* __restrict__ u, const double* __restrict__ uc, int nx, int ny) {
+__global__ void k_prolong_add(double* u, const double* uc, int nx, int ny) {
+    after_previous<false>();
     const int i = blockIdx.x * blockDim.x + threadIdx.x, j = blockIdx.y * blockDim.y + threadIdx.y;
     if (i >= nx || j >= ny) return;
     u[(size_t)j * nx + i] += uc[(size_t)(j >> 1) * (nx >> 1) + (i >> 1)];
@@ -2001,9 +2065,10 @@ __global__ void k_prolong_add(double* __restrict__ u, const double* __restrict__
 // The bottom level's dense solve on row-major arrays (unknown row = j*nx + i): the
 // elimination factors of k_dense_factor applied to f in the oracle's order, then its back
 // substitution by thread 0 (the same arithmetic as s_dense).
-__global__ void __launch_bounds__(64) k_dense_solve(const double* __restrict__ lu, const double* __restrict__ f,
+__global__ void __launch_bounds__(64) k_dense_solve(const double* __restrict__ lu, const double* f,
                                                     double* __restrict__ u, int n) {
     __shared__ double b[kMaxDense];
+    after_previous<false>();
     for (int k = threadIdx.x; k < n; k += blockDim.x) b[k] = f[k];
     __syncthreads();
     for (int k = 0; k + 1 < n; ++k) {
@@ -2024,9 +2089,10 @@ __global__ void __launch_bounds__(64) k_dense_solve(const double* __restrict__ l
 
 // r.z of the level-0 preconditioner application and the CG beta (the part of k_up's
 // level-0 epilogue the y-line cycle needs).
-__global__ void __launch_bounds__(256) k_rz(const double* __restrict__ r, const double* __restrict__ z, size_t n,
-                                            State* __restrict__ st, double* __restrict__ partials) {
+__global__ void __launch_bounds__(256) k_rz(const double* r, const double* z, size_t n, State* st,
+                                            double* partials) {
     __shared__ double red[32];
+    after_previous<false>();
     double acc = 0.0;
     for (size_t k = blockIdx.x * (size_t)blockDim.x + threadIdx.x; k < n; k += (size_t)gridDim.x * blockDim.x)
         acc += r[k] * z[k];
@@ -2241,8 +2307,8 @@ template <typename T, int NS, int TS>
 void down_tile(const LevelBuf& L, const LevelBuf& C, cudaStream_t s) {
     using Cfg = RBCfg<NS, TS, TS, RB_R>;
     dim3 grid(L.nx / TS, L.ny / TS);
-    k_down<T, NS, TS, TS, RB_R><<<grid, Cfg::NTH, 0, s>>>((const T*)L.f, lvl_ax<T>(L), lvl_ay<T>(L), lvl_di<T>(L),
-                                                          (T*)L.u, (T*)C.f, L.nx, L.ny);
+    (void)launch_next(k_down<T, NS, TS, TS, RB_R>, grid, Cfg::NTH, 0, s, (const T*)L.f, lvl_ax<T>(L), lvl_ay<T>(L),
+                      lvl_di<T>(L), (T*)L.u, (T*)C.f, L.nx, L.ny);
 }
 
 template <typename T, int NS>
@@ -2271,13 +2337,11 @@ void up_tile(lica_mg* m, const LevelBuf& L, const T* uc, bool level0, cudaStream
     using Cfg = RBCfg<NS, TS, TS, RB_R>;
     dim3 grid(L.nx / TS, L.ny / TS);
     if (level0)
-        k_up<T, NS, TS, TS, RB_R, true><<<grid, Cfg::NTH, 0, s>>>((const T*)L.u, (T*)L.up, uc, (const T*)L.f,
-                                                                  lvl_ax<T>(L), lvl_ay<T>(L), lvl_di<T>(L), L.nx,
-                                                                  L.ny, m->st, m->partials);
+        (void)launch_next(k_up<T, NS, TS, TS, RB_R, true>, grid, Cfg::NTH, 0, s, (const T*)L.u, (T*)L.up, uc,
+                          (const T*)L.f, lvl_ax<T>(L), lvl_ay<T>(L), lvl_di<T>(L), L.nx, L.ny, m->st, m->partials);
     else
-        k_up<T, NS, TS, TS, RB_R, false><<<grid, Cfg::NTH, 0, s>>>((const T*)L.u, (T*)L.up, uc, (const T*)L.f,
-                                                                   lvl_ax<T>(L), lvl_ay<T>(L), lvl_di<T>(L), L.nx,
-                                                                   L.ny, m->st, m->partials);
+        (void)launch_next(k_up<T, NS, TS, TS, RB_R, false>, grid, Cfg::NTH, 0, s, (const T*)L.u, (T*)L.up, uc,
+                          (const T*)L.f, lvl_ax<T>(L), lvl_ay<T>(L), lvl_di<T>(L), L.nx, L.ny, m->st, m->partials);
 }
 
 template <typename T, int NS>
@@ -2376,7 +2440,7 @@ int launch_cta(lica_mg* m, cudaStream_t s) {
     P.f_in = m->lv[m->lcta].f;
     P.u_out = m->lv[m->lcta].u;
     ProfScope ps(m, LICA_MG_CTA, s);
-    k_cta<T><<<1, NT_CTA, m->cta_smem, s>>>(P);
+    LICA_CUDA_TRY(launch_next(k_cta<T>, 1, NT_CTA, m->cta_smem, s, P));
     LICA_CUDA_TRY(cudaGetLastError());
     lica_count_launches(1);
     return LICA_OK;
@@ -2410,8 +2474,8 @@ int yl_smooth(lica_mg* m, int l, double* u, const double* f, int nsw, bool rever
         for (int c = 0; c < 2; ++c) {
             const int parity = reverse ? 1 - c : c;
             if (L.yc)
-                k_yline_column<<<cols, kYlThreads, yl_smem(L.ny), s>>>(u, f, L.ax64, L.ay64, L.yc, L.yd, L.yi, L.nx,
-                                                                      L.ny, parity);
+                LICA_CUDA_TRY(launch_next(k_yline_column, cols, kYlThreads, yl_smem(L.ny), s, u, f, L.ax64, L.ay64, L.yc,
+                                          L.yd, L.yi, L.nx, L.ny, parity));
             else
                 k_yline_half<<<(cols + 127) / 128, 128, 0, s>>>(u, f, L.ax64, L.ay64, m->ycp, m->ydp, L.nx, L.ny,
                                                                parity);
@@ -2424,9 +2488,8 @@ int yl_smooth(lica_mg* m, int l, double* u, const double* f, int nsw, bool rever
 int yl_restrict(lica_mg* m, int l, const double* u, const double* f, cudaStream_t s) {
     const LevelBuf& L = m->lv[l];
     const dim3 blk(32, 8), grid((L.nx / 2 + 31) / 32, (L.ny / 2 + 7) / 8);
-    k_resid_restrict<<<grid, blk, 0, s>>>(u, f, L.ax64, L.ay64, (double*)m->lv[l + 1].f, L.nx, L.ny);
-    LICA_CUDA_TRY(cudaGetLastError());
-    LICA_CUDA_TRY(cudaMemsetAsync(m->lv[l + 1].u, 0, sizeof(double) * (size_t)m->lv[l + 1].nx * m->lv[l + 1].ny, s));
+    LICA_CUDA_TRY(launch_next(k_resid_restrict, grid, blk, 0, s, u, f, L.ax64, L.ay64, (double*)m->lv[l + 1].f,
+                              (double*)m->lv[l + 1].u, L.nx, L.ny));
     lica_count_launches(1);
     return LICA_OK;
 }
@@ -2434,16 +2497,14 @@ int yl_restrict(lica_mg* m, int l, const double* u, const double* f, cudaStream_
 int yl_prolong(lica_mg* m, int l, double* u, cudaStream_t s) {
     const LevelBuf& L = m->lv[l];
     const dim3 blk(32, 8), grid((L.nx + 31) / 32, (L.ny + 7) / 8);
-    k_prolong_add<<<grid, blk, 0, s>>>(u, (const double*)m->lv[l + 1].u, L.nx, L.ny);
-    LICA_CUDA_TRY(cudaGetLastError());
+    LICA_CUDA_TRY(launch_next(k_prolong_add, grid, blk, 0, s, u, (const double*)m->lv[l + 1].u, L.nx, L.ny));
     lica_count_launches(1);
     return LICA_OK;
 }
 
 int yl_dense(lica_mg* m, cudaStream_t s) {
     const LevelBuf& B = m->lv[m->bottom];
-    k_dense_solve<<<1, 64, 0, s>>>(m->dense_lu, (const double*)B.f, (double*)B.u, B.nx * B.ny);
-    LICA_CUDA_TRY(cudaGetLastError());
+    LICA_CUDA_TRY(launch_next(k_dense_solve, 1, 64, 0, s, m->dense_lu, (const double*)B.f, (double*)B.u, B.nx * B.ny));
     lica_count_launches(1);
     return LICA_OK;
 }
@@ -2491,8 +2552,7 @@ int vcycle_yline(lica_mg* m, cudaStream_t s) {
     }
     const size_t n0 = (size_t)m->nx * m->ny;
     const int nb = (int)std::min<size_t>(148, (n0 + 255) / 256);
-    k_rz<<<nb, 256, 0, s>>>((const double*)m->r, (const double*)m->z, n0, m->st, m->partials);
-    LICA_CUDA_TRY(cudaGetLastError());
+    LICA_CUDA_TRY(launch_next(k_rz, nb, 256, 0, s, (const double*)m->r, (const double*)m->z, n0, m->st, m->partials));
     lica_count_launches(1);
     return LICA_OK;
 }
@@ -2516,47 +2576,44 @@ int setup_beta(lica_mg* m, const double* bx, const double* by, cudaStream_t s) {
         const size_t work = (size_t)C.nx * C.ny * 2 + C.nx;
         if (l > 0) {
             LevelBuf& F = m->lv[l - 1];
-            k_coarsen_beta<double><<<blocks_for(work), 256, 0, s>>>(F.bx64, F.by64, C.bx64, C.by64, C.nx, C.ny);
-            LICA_CUDA_TRY(cudaGetLastError());
+            LICA_CUDA_TRY(launch_next(k_coarsen_beta<double>, blocks_for(work), 256, 0, s, F.bx64, F.by64, C.bx64,
+                                      C.by64, C.nx, C.ny));
             lica_count_launches(1);
         }
-        k_scale_beta<double><<<blocks_for(work), 256, 0, s>>>(C.bx64, C.by64, C.ax64, C.ay64, C.di64, C.nx, C.ny,
-                                                               C.cx, C.cy);
-        LICA_CUDA_TRY(cudaGetLastError());
+        LICA_CUDA_TRY(launch_next(k_scale_beta<double>, blocks_for(work), 256, 0, s, C.bx64, C.by64, C.ax64, C.ay64,
+                                  C.di64, C.nx, C.ny, C.cx, C.cy));
         lica_count_launches(1);
         if (C.yc) {
-            k_yline_factor<<<C.nx, kYlThreads, yl_smem(C.ny), s>>>(C.ax64, C.ay64, C.yc, C.yd, C.yi, C.nx, C.ny);
-            LICA_CUDA_TRY(cudaGetLastError());
+            LICA_CUDA_TRY(launch_next(k_yline_factor, C.nx, kYlThreads, yl_smem(C.ny), s, C.ax64, C.ay64, C.yc, C.yd,
+                                      C.yi, C.nx, C.ny));
             lica_count_launches(1);
         }
     }
     if (is_mixed(m)) {
         LevelBuf& L0 = m->lv[0];
         const size_t n = (size_t)L0.nx * L0.ny;
-        k_to_float<<<1184, 256, 0, s>>>(bx, L0.bx32, n);
-        k_to_float<<<1184, 256, 0, s>>>(by, L0.by32, n + L0.nx);
-        LICA_CUDA_TRY(cudaGetLastError());
+        LICA_CUDA_TRY(launch_next(k_to_float, 1184, 256, 0, s, bx, L0.bx32, n));
+        LICA_CUDA_TRY(launch_next(k_to_float, 1184, 256, 0, s, by, L0.by32, n + L0.nx));
         lica_count_launches(2);
         for (int l = 0; l < m->nouter - 1; ++l) {
             LevelBuf& C = m->lv[l];
             const size_t work = (size_t)C.nx * C.ny * 2 + C.nx;
             if (l > 0) {
                 LevelBuf& F = m->lv[l - 1];
-                k_coarsen_beta<float><<<blocks_for(work), 256, 0, s>>>(F.bx32, F.by32, C.bx32, C.by32, C.nx, C.ny);
-                LICA_CUDA_TRY(cudaGetLastError());
+                LICA_CUDA_TRY(launch_next(k_coarsen_beta<float>, blocks_for(work), 256, 0, s, F.bx32, F.by32, C.bx32,
+                                          C.by32, C.nx, C.ny));
                 lica_count_launches(1);
             }
-            k_scale_beta<float><<<blocks_for(work), 256, 0, s>>>(C.bx32, C.by32, C.ax32, C.ay32, C.di32, C.nx, C.ny,
-                                                                  float(C.cx), float(C.cy));
-            LICA_CUDA_TRY(cudaGetLastError());
+            LICA_CUDA_TRY(launch_next(k_scale_beta<float>, blocks_for(work), 256, 0, s, C.bx32, C.by32, C.ax32, C.ay32,
+                                      C.di32, C.nx, C.ny, float(C.cx), float(C.cy)));
             lica_count_launches(1);
         }
     }
     {
         const LevelBuf& B = m->lv[m->bottom];
         const int nb = B.nx * B.ny;
-        k_dense_factor<<<1, 256, sizeof(double) * nb * nb, s>>>(B.ax64, B.ay64, m->dense_lu, B.nx, B.ny);
-        LICA_CUDA_TRY(cudaGetLastError());
+        LICA_CUDA_TRY(launch_next(k_dense_factor, 1, 256, sizeof(double) * nb * nb, s, B.ax64, B.ay64, m->dense_lu, B.nx,
+                                  B.ny));
         lica_count_launches(1);
     }
     // the single-CTA kernel's weights as it holds them (the y-line cycle has none)
@@ -2565,10 +2622,11 @@ int setup_beta(lica_mg* m, const double* bx, const double* by, cudaStream_t s) {
             const LevelBuf& L = m->lv[l];
             const int blocks = blocks_for((size_t)L.nx * (L.ny + 1));
             if (l < m->nouter - 1 && is_mixed(m))
-                k_cta_image<float><<<blocks, 256, 0, s>>>(L.ax32, L.ay32, L.di32, m->cta_image, m->cp.lv[l]);
+                LICA_CUDA_TRY(launch_next(k_cta_image<float>, blocks, 256, 0, s, L.ax32, L.ay32, L.di32, m->cta_image,
+                                          m->cp.lv[l]));
             else
-                k_cta_image<double><<<blocks, 256, 0, s>>>(L.ax64, L.ay64, L.di64, m->cta_image, m->cp.lv[l]);
-            LICA_CUDA_TRY(cudaGetLastError());
+                LICA_CUDA_TRY(launch_next(k_cta_image<double>, blocks, 256, 0, s, L.ax64, L.ay64, L.di64, m->cta_image,
+                                          m->cp.lv[l]));
             lica_count_launches(1);
         }
     return LICA_OK;
@@ -2608,8 +2666,7 @@ int launch_cg_tma(lica_mg* m, double* x, cudaGraphConditionalHandle h, int use_c
     A.cond = h;
     A.use_cond = use_cond;
     const int grid = std::min(A.ntx * A.nty, m->nsm);
-    k_cg_tma<TZ, XUP><<<grid, CG_NT, CgLayout<TZ, XUP>::BYTES, s>>>(A);
-    LICA_CUDA_TRY(cudaGetLastError());
+    LICA_CUDA_TRY(launch_next(k_cg_tma<TZ, XUP>, grid, CG_NT, CgLayout<TZ, XUP>::BYTES, s, A));
     lica_count_launches(1);
     return LICA_OK;
 }
@@ -2626,9 +2683,14 @@ int launch_xupdate(lica_mg* m, double* x, const double* f, int first, cudaGraphC
     }
     dim3 grid(L.nx / TX, L.ny / TY);
     ProfScope ps(m, LICA_MG_XUPDATE, s);
-    k_xupdate<TR><<<grid, NT, xupdate_smem(), s>>>(x, m->xb, m->pcg[0], m->pcg[1], f, L.ax64, L.ay64, (TR*)m->r, L.nx, L.ny,
-                                      m->st, m->partials, first, h, use_cond);
-    LICA_CUDA_TRY(cudaGetLastError());
+    if (first) {  // after the set-up kernels, whose weights it reads before it would wait
+        k_xupdate<TR><<<grid, NT, xupdate_smem(), s>>>(x, m->xb, m->pcg[0], m->pcg[1], f, L.ax64, L.ay64, (TR*)m->r, L.nx,
+                                                       L.ny, m->st, m->partials, first, h, use_cond);
+        LICA_CUDA_TRY(cudaGetLastError());
+    } else {
+        LICA_CUDA_TRY(launch_next(k_xupdate<TR>, grid, NT, xupdate_smem(), s, x, m->xb, m->pcg[0], m->pcg[1], f, L.ax64,
+                                  L.ay64, (TR*)m->r, L.nx, L.ny, m->st, m->partials, first, h, use_cond));
+    }
     lica_count_launches(1);
     return LICA_OK;
 }
@@ -2642,9 +2704,8 @@ int launch_pupdate(lica_mg* m, cudaStream_t s) {
     }
     dim3 grid(L.nx / TX, L.ny / TY);
     ProfScope ps(m, LICA_MG_PUPDATE, s);
-    k_pupdate<TZ><<<grid, NT, pupdate_smem<TZ>(), s>>>(m->pcg[0], m->pcg[1], (const TZ*)m->z, L.ax64, L.ay64, L.nx, L.ny, m->st,
-                                      m->partials);
-    LICA_CUDA_TRY(cudaGetLastError());
+    LICA_CUDA_TRY(launch_next(k_pupdate<TZ>, grid, NT, pupdate_smem<TZ>(), s, m->pcg[0], m->pcg[1], (const TZ*)m->z, L.ax64,
+                              L.ay64, L.nx, L.ny, m->st, m->partials));
     lica_count_launches(1);
     return LICA_OK;
 }

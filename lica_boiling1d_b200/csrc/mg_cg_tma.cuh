@@ -127,12 +127,13 @@ __global__ void __launch_bounds__(CG_NT, 1) k_cg_tma(const __grid_constant__ CgA
     __shared__ __align__(8) uint64_t bar[CG_STAGES];
     __shared__ double red[32];
     const int ntiles = A.ntx * A.nty;
-    const int par = A.st->it & 1;
-    const double coef = XUP ? A.st->alpha : A.st->beta;
     if (threadIdx.x == 0) {
         for (int q = 0; q < CG_STAGES; ++q) tc::mbar_init(&bar[q], 1);
         tc::fence_barrier_init();
     }
+    after_previous();
+    const int par = A.st->it & 1;
+    const double coef = XUP ? A.st->alpha : A.st->beta;
     __syncthreads();
     // the first CG_STAGES - 1 tiles in flight
     if (threadIdx.x == 0)
