@@ -244,8 +244,7 @@ int conv3x3(const __nv_bfloat16* x0, int c0, const __nv_bfloat16* x1, int c1, co
     LICA_CUDA_TRY(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, k_conv3x3_tcp, kConvThreads, smem));
     per_sm = std::max(1, std::min(per_sm, 512 / (2 * P.tmem_cols)));
     const int grid = std::min(tiles, per_sm * num_sms);
-    k_conv3x3_tcp<<<grid, kConvThreads, smem, s>>>(mx0, mx1, mw0, mw1, P);
-    LICA_CUDA_TRY(cudaGetLastError());
+    LICA_CUDA_TRY(launch_next(k_conv3x3_tcp, grid, kConvThreads, smem, s, mx0, mx1, mw0, mw1, P));
     lica_count_launches(1);
     return LICA_OK;
 }
@@ -309,7 +308,8 @@ __global__ void k_rms_part(const double* __restrict__ f, double* __restrict__ pa
     s = block_sum(s, red);
     if (threadIdx.x == 0) part[blockIdx.y * kRmsParts + blockIdx.x] = s;
 }
-__global__ void k_rms_final(const double* __restrict__ part, double* __restrict__ sigma, int npix) {
+__global__ void k_rms_final(const double* part, double* __restrict__ sigma, int npix) {
+    after_previous();
     __shared__ double red[32];
     double s = 0.0;
     for (int k = threadIdx.x; k < kRmsParts; k += blockDim.x) s += part[blockIdx.x * kRmsParts + k];
@@ -320,8 +320,9 @@ __global__ void k_rms_final(const double* __restrict__ part, double* __restrict_
     }
 }
 
-__global__ void k_input(const double* __restrict__ rho, const double* __restrict__ f, const double* __restrict__ sigma,
+__global__ void k_input(const double* rho, const double* f, const double* sigma,
                         bf16* __restrict__ x, int npix, int nimg) {
+    after_previous();
     const size_t total = (size_t)npix * nimg;
     for (size_t p = blockIdx.x * (size_t)blockDim.x + threadIdx.x; p < total; p += (size_t)gridDim.x * blockDim.x) {
         const int img = (int)(p / npix);
@@ -338,7 +339,8 @@ __global__ void k_input(const double* __restrict__ rho, const double* __restrict
 
 // nearest upsampling x2 (H x W the output size): each thread copies one 8-channel group
 // of an input pixel to its 2 x 2 output pixels.
-__global__ void k_up(const bf16* __restrict__ in, bf16* __restrict__ out, int nimg, int H, int W, int c) {
+__global__ void k_up(const bf16* in, bf16* __restrict__ out, int nimg, int H, int W, int c) {
+    after_previous();
     const int c8 = c / 8, Hi = H / 2, Wi = W / 2;
     const size_t total = (size_t)nimg * Hi * Wi * c8;
     for (size_t q = blockIdx.x * (size_t)blockDim.x + threadIdx.x; q < total; q += (size_t)gridDim.x * blockDim.x) {
@@ -376,8 +378,9 @@ __device__ __forceinline__ uint4 relu_mask8(const float* v, const uint4 y) {
 // The head's backward pass, one sweep over d1b (d) and gout: per-block partial sums of its
 // gradients, part[b][c] = sum gout * d1b[:, c] (c < 32), part[b][32] = sum gout, over the pixels of
 // block b (fixed order), and dz = gout * wh through the last layer's ReLU.
-__global__ void k_head_bwd(const float* __restrict__ gout, const float* __restrict__ wh, const bf16* __restrict__ d,
+__global__ void k_head_bwd(const float* gout, const float* wh, const bf16* d,
                            bf16* __restrict__ dz, float* __restrict__ part, size_t total) {
+    after_previous();
     __shared__ float red[kNT / 32][kHead + 1];
     __shared__ float w[kHead];
     if (threadIdx.x < kHead) w[threadIdx.x] = wh[threadIdx.x];
@@ -423,8 +426,9 @@ __global__ void k_head_bwd(const float* __restrict__ gout, const float* __restri
 // dz = g through the layer's ReLU (y > 0), eight channels a thread; g = the channel slice
 // [g_c0, g_c0 + c) of a tensor with g_cs channels, plus (optionally) 0.25 * gp at the parent cell
 // of a half-size tensor (pool backward).  H and W are the image's, c a multiple of 8.
-__global__ void k_relu_bwd(const bf16* __restrict__ g, int g_cs, int g_c0, const bf16* __restrict__ gp,
-                           const bf16* __restrict__ y, bf16* __restrict__ dz, int nimg, int H, int W, int c) {
+__global__ void k_relu_bwd(const bf16* g, int g_cs, int g_c0, const bf16* gp,
+                           const bf16* y, bf16* __restrict__ dz, int nimg, int H, int W, int c) {
+    after_previous();
     const int c8 = c / 8;
     const size_t total = (size_t)nimg * H * W * c8;
     for (size_t q = blockIdx.x * (size_t)blockDim.x + threadIdx.x; q < total; q += (size_t)gridDim.x * blockDim.x) {
@@ -459,8 +463,9 @@ __global__ void k_relu_bwd(const bf16* __restrict__ g, int g_cs, int g_c0, const
 
 // Upsampling backward and the layer's ReLU: dz[n, Y, X, c] = the sum of the 4 children of g
 // (channel slice [g_c0, g_c0 + c) of a tensor with g_cs channels), rounded to BF16, where y > 0.
-__global__ void k_up_relu_bwd(const bf16* __restrict__ g, int g_cs, int g_c0, const bf16* __restrict__ y,
+__global__ void k_up_relu_bwd(const bf16* g, int g_cs, int g_c0, const bf16* y,
                               bf16* __restrict__ dz, int nimg, int Ho, int Wo, int c) {
+    after_previous();
     const int c8 = c / 8, W = 2 * Wo;
     const size_t total = (size_t)nimg * Ho * Wo * c8;
     for (size_t q = blockIdx.x * (size_t)blockDim.x + threadIdx.x; q < total; q += (size_t)gridDim.x * blockDim.x) {
@@ -490,9 +495,10 @@ __global__ void k_up_relu_bwd(const bf16* __restrict__ g, int g_cs, int g_c0, co
 // grad[k] = sum over chunks of part[chunk][k], for k < n, and the same of a second set (bpart, nb
 // values to bgrad, may be empty): 8 threads per value take every 8th chunk, then add up in a
 // fixed order.  Block: 32 values x 8 threads.
-__global__ void __launch_bounds__(256) k_sum_parts(const float* __restrict__ part, int nchunk, size_t n,
-                                                   float* __restrict__ grad, const float* __restrict__ bpart, size_t nb,
+__global__ void __launch_bounds__(256) k_sum_parts(const float* part, int nchunk, size_t n,
+                                                   float* __restrict__ grad, const float* bpart, size_t nb,
                                                    float* __restrict__ bgrad) {
+    after_previous();
     __shared__ float red[8][33];
     const int x = threadIdx.x & 31, y = threadIdx.x >> 5;
     const size_t blocks = (n + 31) / 32;
@@ -514,15 +520,16 @@ __global__ void __launch_bounds__(256) k_sum_parts(const float* __restrict__ par
 }
 int sum_parts(const float* part, int nchunk, size_t n, float* grad, const float* bpart, size_t nb, float* bgrad,
               cudaStream_t s) {
-    k_sum_parts<<<(unsigned)((n + 31) / 32 + (nb + 31) / 32), 256, 0, s>>>(part, nchunk, n, grad, bpart, nb, bgrad);
-    LICA_CUDA_TRY(cudaGetLastError());
+    LICA_CUDA_TRY(launch_next(k_sum_parts, (unsigned)((n + 31) / 32 + (nb + 31) / 32), 256, 0, s, part, nchunk, n, grad, bpart,
+                              nb, bgrad));
     lica_count_launches(1);
     return LICA_OK;
 }
 
 // Adam (FP32 master weights).
-__global__ void k_adam(float* __restrict__ w, const float* __restrict__ g, float* __restrict__ m,
+__global__ void k_adam(float* __restrict__ w, const float* g, float* __restrict__ m,
                        float* __restrict__ v, size_t n, float lr, float b1, float b2, float eps, float c1, float c2) {
+    after_previous();
     for (size_t k = blockIdx.x * (size_t)blockDim.x + threadIdx.x; k < n; k += (size_t)gridDim.x * blockDim.x) {
         const float gk = g[k];
         const float mk = b1 * m[k] + (1.f - b1) * gk;
@@ -550,8 +557,9 @@ __global__ void k_pack(const float* __restrict__ w, bf16* __restrict__ wb, bf16*
 
 // FP64 pressure operator of the solver: out = s - d*u (x periodic, bottom Neumann, top
 // p = 0 on the face), the oracle's apply, for nimg images.
-__global__ void k_apply_op(const double* __restrict__ u, const double* __restrict__ bx, const double* __restrict__ by,
+__global__ void k_apply_op(const double* u, const double* bx, const double* by,
                            double* __restrict__ out, int nimg, int ny, int nx, double cx, double cy) {
+    after_previous();
     const size_t npix = (size_t)nx * ny, total = npix * nimg;
     for (size_t q = blockIdx.x * (size_t)blockDim.x + threadIdx.x; q < total; q += (size_t)gridDim.x * blockDim.x) {
         const size_t img = q / npix, k = q - img * npix;
@@ -605,8 +613,9 @@ __global__ void k_part_sum(const double* __restrict__ part, double* __restrict__
 }
 
 // dL/dout = -2 (A r) sigma h^2 rho / (nimg ||f||^2), ||f||^2 = sigma^2 npix.
-__global__ void k_gout(const double* __restrict__ ar, const double* __restrict__ sigma, const double* __restrict__ rho,
+__global__ void k_gout(const double* ar, const double* sigma, const double* rho,
                        double hsq, float* __restrict__ gout, int npix, int nimg) {
+    after_previous();
     const size_t total = (size_t)npix * nimg;
     for (size_t p = blockIdx.x * (size_t)blockDim.x + threadIdx.x; p < total; p += (size_t)gridDim.x * blockDim.x) {
         const double sg = sigma[p / npix];
@@ -636,9 +645,10 @@ __global__ void k_energy(const double* __restrict__ ae, const double* __restrict
 }
 
 // dL/dout of L = mean_images num/den: -2 (A e) sigma h^2 rho / (nimg den).
-__global__ void k_gout_energy(const double* __restrict__ ae, const double* __restrict__ den,
-                              const double* __restrict__ sigma, const double* __restrict__ rho, double hsq,
+__global__ void k_gout_energy(const double* ae, const double* den,
+                              const double* sigma, const double* rho, double hsq,
                               float* __restrict__ gout, int npix, int nimg) {
+    after_previous();
     const size_t total = (size_t)npix * nimg;
     for (size_t p = blockIdx.x * (size_t)blockDim.x + threadIdx.x; p < total; p += (size_t)gridDim.x * blockDim.x) {
         const size_t img = p / npix;
@@ -646,15 +656,17 @@ __global__ void k_gout_energy(const double* __restrict__ ae, const double* __res
     }
 }
 
-__global__ void k_sub(double* __restrict__ a, const double* __restrict__ b, size_t n) {
+__global__ void k_sub(double* __restrict__ a, const double* b, size_t n) {
+    after_previous();
     for (size_t k = blockIdx.x * (size_t)blockDim.x + threadIdx.x; k < n; k += (size_t)gridDim.x * blockDim.x)
         a[k] -= b[k];
 }
 
 // gout from a given dL/dx0 (the gradient check): gout = gx0 * sigma * h^2 * rho
-__global__ void k_gout_from_gx(const double* __restrict__ gx, const double* __restrict__ sigma,
-                               const double* __restrict__ rho, double hsq, float* __restrict__ gout, int npix,
+__global__ void k_gout_from_gx(const double* gx, const double* sigma,
+                               const double* rho, double hsq, float* __restrict__ gout, int npix,
                                int nimg) {
+    after_previous();
     const size_t total = (size_t)npix * nimg;
     for (size_t p = blockIdx.x * (size_t)blockDim.x + threadIdx.x; p < total; p += (size_t)gridDim.x * blockDim.x)
         gout[p] = (float)(gx[p] * sigma[p / npix] * hsq * rho[p]);
@@ -752,8 +764,7 @@ int conv_layer(lica_unet* u, int l, const bf16* x0, const bf16* x1, bf16* out, c
 
 template <typename K, typename... A>
 int launch(size_t n, cudaStream_t s, K kernel, A... args) {
-    kernel<<<grid_for(n), kNT, 0, s>>>(args...);
-    LICA_CUDA_TRY(cudaGetLastError());
+    LICA_CUDA_TRY(launch_next(kernel, grid_for(n), kNT, 0, s, args...));
     lica_count_launches(1);
     return LICA_OK;
 }
@@ -766,8 +777,8 @@ int forward(lica_unet* u, const double* rho, const double* f, double hsq, double
     const int npix = u->h * u->w;
     int st;
     k_rms_part<<<dim3(kRmsParts, u->n), kNT, 0, s>>>(f, u->rms_part, npix);
-    k_rms_final<<<u->n, kNT, 0, s>>>(u->rms_part, u->sigma, npix);
     LICA_CUDA_TRY(cudaGetLastError());
+    LICA_CUDA_TRY(launch_next(k_rms_final, u->n, kNT, 0, s, u->rms_part, u->sigma, npix));
     lica_count_launches(2);
     if ((st = launch(level_pixels(u, 0), s, k_input, rho, f, (const double*)u->sigma, u->x16, npix, u->n))) return st;
     const int h = u->h, w = u->w, n = u->n;
@@ -865,8 +876,8 @@ int layer_wgrad(lica_unet* u, int l, const bf16* x0, const bf16* x1, cudaStream_
     m1 = m0;
     if (L.cin1 && (st = act_map(&m1, x1, L.cin1, W, H, u->n, P.cblk, kTileW, kTileH + 2))) return st;
     const int chunks = wgrad_chunks(u, l);
-    k_wgrad3x3<<<dim3(chunks, ctot / P.cblk), kWgThreads, 1024 + P.nstages * P.stage + kWgBehind, s>>>(mdz, m0, m1, P);
-    LICA_CUDA_TRY(cudaGetLastError());
+    LICA_CUDA_TRY(launch_next(k_wgrad3x3, dim3(chunks, ctot / P.cblk), kWgThreads, 1024 + P.nstages * P.stage + kWgBehind, s,
+                              mdz, m0, m1, P));
     lica_count_launches(1);
     return sum_parts(u->part, chunks, (size_t)L.cout * 9 * ctot, u->grad + u->woff[l], u->bpart, (size_t)L.cout,
                      u->grad + u->boff[l], s);
@@ -906,8 +917,7 @@ int backward(lica_unet* u, cudaStream_t s) {
     int st;
     // head and the ReLU of L9
     const int hb = grid_for(p0);
-    k_head_bwd<<<hb, kNT, 0, s>>>(u->gout, u->param + u->hoff, u->y[9], u->dz, u->hpart, p0);
-    LICA_CUDA_TRY(cudaGetLastError());
+    LICA_CUDA_TRY(launch_next(k_head_bwd, hb, kNT, 0, s, u->gout, u->param + u->hoff, u->y[9], u->dz, u->hpart, p0));
     lica_count_launches(1);
     if ((st = sum_parts(u->hpart, hb, (size_t)(kHead + 1), u->grad + u->hoff, nullptr, 0, nullptr, s))) return st;
     // L9 (input d1a)

@@ -32,6 +32,7 @@
 #include <cuda.h>
 #include <cuda_bf16.h>
 
+#include "chain.cuh"
 #include "tc_sm100.cuh"
 
 namespace lica {
@@ -211,6 +212,8 @@ __global__ void __launch_bounds__(kConvThreads, 1)
             tc::prefetch_tmap(&tm_w1);
         }
     }
+    // before the tensor memory is taken: the kernel before may not have taken its own yet
+    after_previous();
     if (warp == 0) tc::tmem_alloc(tmem_slot, (uint32_t)(2 * P.tmem_cols));
     tc::tc_fence_before();
     __syncthreads();

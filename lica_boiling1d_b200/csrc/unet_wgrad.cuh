@@ -75,6 +75,7 @@ __global__ void __launch_bounds__(kWgThreads, 1)
         tc::mbar_init(&done, 1);
         tc::fence_barrier_init();
     }
+    after_previous();  // before the tensor memory is taken
     if (warp == 0) tc::tmem_alloc(&tmem_slot, 512);
     tc::tc_fence_before();
     __syncthreads();
