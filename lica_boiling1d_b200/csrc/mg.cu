@@ -1811,14 +1811,19 @@ __global__ void __launch_bounds__(128) k_yline_half(double* __restrict__ u, cons
 // warps redo every row's division with the plain operator while the back substitution runs, and
 // the column is redone serially where one does not agree.  With one thread per column, which waits
 // for seven loads and two divisions a row, a half-sweep of 256 x 256 cells took 49 us on average
-// over the levels; so it takes 4.9.  Columns whose seven arrays do not fit a CTA's shared memory keep k_yline_half.
+// over the levels; so it takes 4.8.  Columns whose seven arrays do not fit a CTA's shared memory keep k_yline_half.
 constexpr int kYlThreads = 128;
 constexpr int kYlArrays = 7;
+// What a half-sweep's neighbours hold: u, zero, or u + P uc.  A half-sweep reads its neighbours alone and
+// writes its own columns in full, and so does the next one, so the first of a smoothing can take the
+// iterate from zero or from the coarse correction without either being stored: no launch that adds
+// the correction, no clearing (256 x 256 cells: a solve 11.27 -> 10.98 ms).
+constexpr int kFromIterate = 0, kFromZero = 1, kFromCoarse = 2;
 __host__ __device__ inline int yl_pitch(int ny) { return (ny + 7) & ~7; }
 __global__ void __launch_bounds__(kYlThreads)
     k_yline_column(double* u, const double* f, const double* __restrict__ ax,
                    const double* __restrict__ ay, const double* __restrict__ yc, const double* __restrict__ yd,
-                   const double* __restrict__ yi, int nx, int ny, int parity) {
+                   const double* __restrict__ yi, int nx, int ny, int parity, int from, const double* uc) {
     extern __shared__ double ysm[];
     const int np = yl_pitch(ny), tid = threadIdx.x;
     double *rhs = ysm, *as = ysm + np, *den = ysm + 2 * np, *inv = ysm + 3 * np, *c = ysm + 4 * np, *e = ysm + 5 * np,
@@ -1842,9 +1847,18 @@ __global__ void __launch_bounds__(kYlThreads)
     after_previous<false>();
     for (int j = tid; j < ny; j += kYlThreads) {  // the thread's own rows of e and x
         const size_t k = (size_t)j * nx;
-        double r = f[k + i];
-        r -= e[j] * u[k + im];
-        r -= x[j] * u[k + ip];
+        double r = f[k + i], uw = 0.0, ue = 0.0;
+        if (from != kFromZero) {
+            uw = u[k + im];
+            ue = u[k + ip];
+        }
+        if (from == kFromCoarse) {
+            const size_t kc = (size_t)(j >> 1) * (nx >> 1);
+            uw += uc[kc + (im >> 1)];
+            ue += uc[kc + (ip >> 1)];
+        }
+        r -= e[j] * uw;
+        r -= x[j] * ue;
         rhs[j] = r;
     }
     __syncthreads();
@@ -2432,15 +2446,17 @@ int vcycle(lica_mg* m, cudaStream_t s) {
 // The y-line V-cycle (FP64), z = M r on m->r / m->z; the oracle's vcycle_outer with
 // coarse_solve and vcycle_inner.
 size_t yl_smem(int ny) { return sizeof(double) * kYlArrays * (size_t)yl_pitch(ny); }
-int yl_smooth(lica_mg* m, int l, double* u, const double* f, int nsw, bool reverse, cudaStream_t s) {
+// from: what the smoothing starts from (a level without yc has it in u already).
+int yl_smooth(lica_mg* m, int l, double* u, const double* f, int nsw, bool reverse, int from, cudaStream_t s) {
     const LevelBuf& L = m->lv[l];
     const int cols = L.nx / 2;
+    const double* uc = from == kFromCoarse ? (const double*)m->lv[l + 1].u : nullptr;
     for (int q = 0; q < nsw; ++q)
         for (int c = 0; c < 2; ++c) {
             const int parity = reverse ? 1 - c : c;
             if (L.yc)
                 LICA_CUDA_TRY(launch_next(k_yline_column, cols, kYlThreads, yl_smem(L.ny), s, u, f, L.ax64, L.ay64, L.yc,
-                                          L.yd, L.yi, L.nx, L.ny, parity));
+                                          L.yd, L.yi, L.nx, L.ny, parity, q + c ? kFromIterate : from, uc));
             else
                 k_yline_half<<<(cols + 127) / 128, 128, 0, s>>>(u, f, L.ax64, L.ay64, m->ycp, m->ydp, L.nx, L.ny,
                                                                parity);
@@ -2461,6 +2477,7 @@ int yl_restrict(lica_mg* m, int l, const double* u, const double* f, cudaStream_
 
 int yl_prolong(lica_mg* m, int l, double* u, cudaStream_t s) {
     const LevelBuf& L = m->lv[l];
+    if (L.yc) return LICA_OK;  // the first half-sweep of the smoothing that follows adds it
     const dim3 blk(32, 8), grid((L.nx + 31) / 32, (L.ny + 7) / 8);
     LICA_CUDA_TRY(launch_next(k_prolong_add, grid, blk, 0, s, u, (const double*)m->lv[l + 1].u, L.nx, L.ny));
     lica_count_launches(1);
@@ -2474,13 +2491,14 @@ int yl_dense(lica_mg* m, cudaStream_t s) {
     return LICA_OK;
 }
 
-int yl_inner(lica_mg* m, int l, cudaStream_t s) {
+int yl_inner(lica_mg* m, int l, int from, cudaStream_t s) {
     if (l == m->bottom) return yl_dense(m, s);
     double* u = (double*)m->lv[l].u;
     const double* f = (const double*)m->lv[l].f;
     int st;
-    if ((st = yl_smooth(m, l, u, f, m->o.nu1, false, s)) || (st = yl_restrict(m, l, u, f, s)) ||
-        (st = yl_inner(m, l + 1, s)) || (st = yl_prolong(m, l, u, s)) || (st = yl_smooth(m, l, u, f, m->o.nu2, true, s)))
+    if ((st = yl_smooth(m, l, u, f, m->o.nu1, false, from, s)) || (st = yl_restrict(m, l, u, f, s)) ||
+        (st = yl_inner(m, l + 1, kFromZero, s)) || (st = yl_prolong(m, l, u, s)) ||
+        (st = yl_smooth(m, l, u, f, m->o.nu2, true, kFromCoarse, s)))
         return st;
     return LICA_OK;
 }
@@ -2488,13 +2506,13 @@ int yl_inner(lica_mg* m, int l, cudaStream_t s) {
 int vcycle_yline(lica_mg* m, cudaStream_t s) {
     const int lc = m->nouter - 1;
     int st;
-    LICA_CUDA_TRY(cudaMemsetAsync(m->z, 0, sizeof(double) * (size_t)m->nx * m->ny, s));
+    if (!m->lv[0].yc) LICA_CUDA_TRY(cudaMemsetAsync(m->z, 0, sizeof(double) * (size_t)m->nx * m->ny, s));
     {
         ProfScope ps(m, LICA_MG_DOWN, s);
         for (int l = 0; l < lc; ++l) {
             double* u = l == 0 ? (double*)m->z : (double*)m->lv[l].u;
             const double* f = l == 0 ? (const double*)m->r : (const double*)m->lv[l].f;
-            if ((st = yl_smooth(m, l, u, f, m->o.nu1, false, s)) || (st = yl_restrict(m, l, u, f, s))) return st;
+            if ((st = yl_smooth(m, l, u, f, m->o.nu1, false, kFromZero, s)) || (st = yl_restrict(m, l, u, f, s))) return st;
         }
     }
     {
@@ -2504,7 +2522,7 @@ int vcycle_yline(lica_mg* m, cudaStream_t s) {
             if ((st = yl_dense(m, s))) return st;
         } else {
             for (int c = 0; c < m->o.ncoarse; ++c)
-                if ((st = yl_inner(m, lc, s))) return st;
+                if ((st = yl_inner(m, lc, c ? kFromIterate : kFromZero, s))) return st;
         }
     }
     {
@@ -2512,7 +2530,7 @@ int vcycle_yline(lica_mg* m, cudaStream_t s) {
         for (int l = lc - 1; l >= 0; --l) {
             double* u = l == 0 ? (double*)m->z : (double*)m->lv[l].u;
             const double* f = l == 0 ? (const double*)m->r : (const double*)m->lv[l].f;
-            if ((st = yl_prolong(m, l, u, s)) || (st = yl_smooth(m, l, u, f, m->o.nu2, true, s))) return st;
+            if ((st = yl_prolong(m, l, u, s)) || (st = yl_smooth(m, l, u, f, m->o.nu2, true, kFromCoarse, s))) return st;
         }
     }
     const size_t n0 = (size_t)m->nx * m->ny;

@@ -30,3 +30,26 @@ def test_yline_columns_bitwise(nx, ny, nlevels):
     mg.precond(z, t(fs), t(bxs), t(bys))
     mg.close()
     np.testing.assert_array_equal(z.cpu().numpy(), ref)
+
+
+# a smoothing's first half-sweep from zero, from the coarse correction and from the iterate: the second
+# coarse cycle starts from the first's result; one, two and three sweeps
+@pytest.mark.parametrize("nx,ny,nu", [(64, 64, 1), (32, 96, 2), (96, 64, 3)])
+def test_yline_start_of_smoothing(nx, ny, nu):
+    import torch
+    from lica_boiling1d_b200 import poisson as PP
+    rng = np.random.default_rng(nx + nu)
+    rho = np.where(rng.random((ny, nx)) < 0.2, 1.0, 40.0)
+    bx = 1.0 / (0.5 * (rho + np.roll(rho, 1, axis=1)))
+    by = np.ones((ny + 1, nx))
+    by[1:ny] = 1.0 / (0.5 * (rho[1:] + rho[:-1]))
+    by[0], by[ny] = 1.0 / rho[0], 1.0 / rho[ny - 1]
+    f = rng.standard_normal((ny, nx))
+    ref = O.mg_precond(f, bx, by, 1.0 / nx, 1.0 / ny, nlevels=2, nu1=nu, nu2=nu, ncoarse=2, sym=13)
+    mg = PP.MultigridPoisson(nx, ny, 1.0 / nx, 1.0 / ny, nlevels=2, nu1=nu, nu2=nu, ncoarse=2, smoother="yline")
+    t = lambda a: torch.from_numpy(np.ascontiguousarray(a)).cuda()  # noqa: E731
+    z = torch.full((ny, nx), float("nan"), dtype=torch.float64, device="cuda")
+    for _ in range(2):
+        mg.precond(z, t(f), t(bx), t(by))
+    mg.close()
+    np.testing.assert_array_equal(z.cpu().numpy(), ref)
