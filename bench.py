@@ -254,7 +254,7 @@ def column_roofline(state_bytes, ms_per_step, kernel):
             "frac": achieved / peak, "peak_source": src, "traffic": None,
             "alg_bytes_per_step": alg,
             "note": "latency-bound, not bandwidth-bound: one CTA per column walks the step's phases in order "
-                    "(three Thomas sweeps per substep on one thread, band lists, the TEMP_EXTP iterations); "
+                    "(three Thomas sweeps per substep on one warp, band lists, the TEMP_EXTP iterations); "
                     "the per-phase cycle profile is the lica_gpu_column_profile_device record"}
 
 

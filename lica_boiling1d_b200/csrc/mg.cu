@@ -16,7 +16,8 @@
 //                level 0 the r.z partial of the CG update
 //   * The levels below 64x64 run in one CTA with everything in shared memory
 //     (k_cta): remaining outer levels, the coarsest outer level solved in FP64 by inner
-//     V-cycles that end in a dense elimination; levels <= 8x8 run in warp 0 alone.
+//     V-cycles that end in a dense elimination; each level has a group of warps as wide as it
+//     is.  A system of at most 4096 cells is solved whole by one CTA (k_small_solve).
 //   * CG vector updates are fused with the stencil they need (k_pupdate: p = z + beta p
 //     and p.Ap; k_xupdate: x += alpha p and the true residual f - A x with its norm).
 //     Grid-wide sums use a deterministic last-block reduction, which also computes the
@@ -27,7 +28,7 @@
 //     one graph node per level, so it is off by default.
 //   * With use_graph the whole solve is one CUDA graph: set-up kernels followed by a
 //     conditional WHILE node whose body is one PCG iteration; the last block of
-//     k_xupdate sets the loop condition.
+//     k_xupdate sets the loop condition.  The kernels are launched as a chain (chain.cuh).
 //   * Every kernel follows the operation order of the oracle and the library is built
 //     with -fmad=false, so a preconditioner application is bit-identical to the CPU
 //     restatement in FP64 and in FP32; only the dot products differ (summation order).
