@@ -2067,6 +2067,230 @@ __global__ void __launch_bounds__(64) k_dense_solve(const double* __restrict__ l
     for (int k = threadIdx.x; k < n; k += blockDim.x) u[k] = b[k];
 }
 
+// The y-line cycle from level l0 down, with everything in one CTA's shared memory: the outer levels
+// l0 .. lc - 1 with the ncoarse inner cycles of lc, or, where l0 > lc, an inner cycle from l0.  The
+// arithmetic is the grid kernels' (k_yline_column, k_resid_restrict, k_dense_solve), one thread to a
+// column's chain.  Bound: the chains, about 60 cycles a row, and four barriers a half-sweep.  As
+// launches of their own these levels' half-sweeps are 1312 of a 256 x 256 solve's 2296, each a launch
+// and its loads: 10.91 ms, 10.17 so.  Levels of up to 2048 cells that fit with those below them; a
+// larger one has more rows than one CTA's threads take in a few passes.
+constexpr int kYcThreads = 256, kYcCells = 2048;
+constexpr size_t kYcSmem = 200 * 1024;
+struct YlCoarse {
+    int l0, lc, bottom, ncoarse, nu1, nu2;
+    unsigned off_rhs, off_e;   // in doubles, like lv[].off
+    const double* f;
+    double* u;
+    const double* lu;
+    struct {
+        int nx, ny;
+        unsigned off;
+        const double *ax, *ay, *yc, *yd, *yi;
+    } lv[kMaxLevels];
+};
+struct YlLevel {   // one level's arrays in shared memory
+    double *u, *f, *ax, *c, *d, *i, *ay;
+    int nx, ny;
+};
+__device__ __forceinline__ YlLevel yl_level(const YlCoarse& P, int l) {
+    extern __shared__ double ysm[];
+    YlLevel L;
+    L.nx = P.lv[l].nx;
+    L.ny = P.lv[l].ny;
+    const int n = L.nx * L.ny;
+    L.u = ysm + P.lv[l].off;
+    L.f = L.u + n;
+    L.ax = L.f + n;
+    L.c = L.ax + n;
+    L.d = L.c + n;
+    L.i = L.d + n;
+    L.ay = L.i + n;
+    return L;
+}
+inline size_t yl_level_doubles(int nx, int ny) { return (size_t)7 * nx * ny + nx; }
+
+__device__ __noinline__ void yc_smooth(const YlCoarse& P, int l, int nsw, bool reverse, int from) {
+    extern __shared__ double ysm[];
+    const YlLevel L = yl_level(P, l);
+    const double* uc = from == kFromCoarse ? yl_level(P, l + 1).u : nullptr;
+    double *rhs = ysm + P.off_rhs, *e = ysm + P.off_e;
+    const int nx = L.nx, ny = L.ny, cols = nx / 2, n = cols * ny, tid = threadIdx.x;
+    const int helpers = (cols + 31) & ~31;   // the first thread that has no column
+    for (int h = 0; h < 2 * nsw; ++h) {
+        const int parity = reverse ? 1 - (h & 1) : (h & 1);
+        const int start = h ? kFromIterate : from;
+        for (int t = tid; t < n; t += kYcThreads) {
+            const int j = t / cols, i = 2 * (t - j * cols) + parity, k = j * nx;
+            const int ip = (i + 1 == nx) ? 0 : i + 1, im = (i == 0) ? nx - 1 : i - 1;
+            double r = L.f[k + i], uw = 0.0, ue = 0.0;
+            if (start != kFromZero) {
+                uw = L.u[k + im];
+                ue = L.u[k + ip];
+            }
+            if (start == kFromCoarse) {
+                const int kc = (j >> 1) * (nx >> 1);
+                uw += uc[kc + (im >> 1)];
+                ue += uc[kc + (ip >> 1)];
+            }
+            r -= L.ax[k + i] * uw;
+            r -= L.ax[k + ip] * ue;
+            rhs[t] = r;
+        }
+        __syncthreads();
+        const int i = 2 * tid + parity;
+        if (tid < cols) {
+            double p = 0.0;
+#pragma unroll 1
+            for (int j = 0; j < ny; j += 4) {
+                double R[4], A[4], D[4], I[4];
+#pragma unroll
+                for (int q = 0; q < 4; ++q) {
+                    const int jj = min(j + q, ny - 1), k = jj * nx + i;
+                    R[q] = rhs[jj * cols + tid];
+                    A[q] = L.ay[k];
+                    D[q] = L.d[k];
+                    I[q] = L.i[k];
+                }
+#pragma unroll
+                for (int q = 0; q < 4; ++q) {
+                    const double t = R[q] - A[q] * p;
+                    const double w = t * I[q];
+                    p = __fma_rn(__fma_rn(-D[q], w, t), I[q], w);
+                    if (j + q < ny) e[(j + q) * cols + tid] = p;
+                }
+            }
+        }
+        __syncthreads();
+        bool bad = false;
+        if (tid < cols) {
+            double x = 0.0;
+#pragma unroll 1
+            for (int j = ny - 1; j >= 0; j -= 4) {
+                double C[4], E[4];
+#pragma unroll
+                for (int q = 0; q < 4; ++q) {
+                    const int jj = max(j - q, 0);
+                    E[q] = e[jj * cols + tid];
+                    C[q] = L.c[jj * nx + i];
+                }
+#pragma unroll
+                for (int q = 0; q < 4; ++q) {
+                    x = E[q] - C[q] * x;
+                    if (j - q >= 0) L.u[(j - q) * nx + i] = x;
+                }
+            }
+        } else if (tid >= helpers) {
+            for (int t = tid - helpers; t < n; t += kYcThreads - helpers) {
+                const int j = t / cols, k = j * nx + 2 * (t - j * cols) + parity;
+                bad |= !(e[t] == (rhs[t] - L.ay[k] * (j > 0 ? e[t - cols] : 0.0)) / L.d[k]);
+            }
+        }
+        if (__syncthreads_or(bad)) {   // as k_yline_column: the columns redone with the plain operator
+            if (tid < cols) {
+                double p = 0.0;
+                for (int j = 0; j < ny; ++j) {
+                    p = (rhs[j * cols + tid] - L.ay[j * nx + i] * p) / L.d[j * nx + i];
+                    e[j * cols + tid] = p;
+                }
+                L.u[(ny - 1) * nx + i] = p;
+                for (int j = ny - 2; j >= 0; --j) {
+                    p = e[j * cols + tid] - L.c[j * nx + i] * p;
+                    L.u[j * nx + i] = p;
+                }
+            }
+            __syncthreads();
+        }
+    }
+}
+
+__device__ __noinline__ void yc_restrict(const YlCoarse& P, int l) {
+    const YlLevel L = yl_level(P, l), C = yl_level(P, l + 1);
+    const int nx = L.nx, ny = L.ny;
+    for (int t = threadIdx.x; t < C.nx * C.ny; t += kYcThreads) {
+        const int J = t / C.nx, I = t - J * C.nx;
+        double r[2][2];
+#pragma unroll
+        for (int b = 0; b < 2; ++b) {
+#pragma unroll
+            for (int a = 0; a < 2; ++a) {
+                const int i = 2 * I + a, j = 2 * J + b, k = j * nx;
+                const int ip = (i + 1 == nx) ? 0 : i + 1, im = (i == 0) ? nx - 1 : i - 1;
+                const double aw = L.ax[k + i], ae = L.ax[k + ip], as = L.ay[k + i], an = L.ay[k + nx + i];
+                const double us = (j > 0) ? L.u[k - nx + i] : 0.0;
+                const double un = (j < ny - 1) ? L.u[k + nx + i] : 0.0;
+                double sm = aw * L.u[k + im];
+                sm += ae * L.u[k + ip];
+                sm += as * us;
+                sm += an * un;
+                double d = aw;
+                d += ae;
+                d += as;
+                d += an;
+                r[b][a] = L.f[k + i] - (sm - d * L.u[k + i]);
+            }
+        }
+        C.f[t] = 0.25 * ((r[0][0] + r[0][1]) + (r[1][0] + r[1][1]));
+    }
+    __syncthreads();
+}
+
+__device__ __noinline__ void yc_inner(const YlCoarse& P, int from_level, int from) {
+    for (int l = from_level; l < P.bottom; ++l) {
+        yc_smooth(P, l, P.nu1, false, l == from_level ? from : kFromZero);
+        yc_restrict(P, l);
+    }
+    {
+        const YlLevel B = yl_level(P, P.bottom);
+        const int n = B.nx * B.ny;
+        double* b = B.u;
+        for (int k = threadIdx.x; k < n; k += kYcThreads) b[k] = B.f[k];
+        __syncthreads();
+        for (int k = 0; k + 1 < n; ++k) {
+            const double bk = b[k];
+            for (int i = k + 1 + threadIdx.x; i < n; i += kYcThreads) b[i] -= P.lu[i * n + k] * bk;
+            __syncthreads();
+        }
+        if (threadIdx.x == 0)
+            for (int i = n - 1; i >= 0; --i) {
+                double sm = b[i];
+                for (int j = i + 1; j < n; ++j) sm -= P.lu[i * n + j] * b[j];
+                b[i] = sm / P.lu[i * n + i];
+            }
+        __syncthreads();
+    }
+    for (int l = P.bottom - 1; l >= from_level; --l) yc_smooth(P, l, P.nu2, true, kFromCoarse);
+}
+
+__global__ void __launch_bounds__(kYcThreads, 1) k_yline_coarse(const __grid_constant__ YlCoarse P) {
+    for (int l = P.l0; l < P.bottom; ++l) {
+        const YlLevel L = yl_level(P, l);
+        const int n = L.nx * L.ny;
+        for (int t = threadIdx.x; t < n; t += kYcThreads) {
+            L.ax[t] = P.lv[l].ax[t];
+            L.c[t] = P.lv[l].yc[t];
+            L.d[t] = P.lv[l].yd[t];
+            L.i[t] = P.lv[l].yi[t];
+        }
+        for (int t = threadIdx.x; t < n + L.nx; t += kYcThreads) L.ay[t] = P.lv[l].ay[t];
+    }
+    after_previous<false>();
+    const YlLevel T = yl_level(P, P.l0);
+    const int n0 = T.nx * T.ny;
+    for (int t = threadIdx.x; t < n0; t += kYcThreads) T.f[t] = P.f[t];
+    __syncthreads();
+    if (P.l0 > P.lc) {
+        yc_inner(P, P.l0, kFromZero);
+    } else {
+        for (int l = P.l0; l < P.lc; ++l) {
+            yc_smooth(P, l, P.nu1, false, kFromZero);
+            yc_restrict(P, l);
+        }
+        for (int c = 0; c < (P.lc == P.bottom ? 1 : P.ncoarse); ++c) yc_inner(P, P.lc, c ? kFromIterate : kFromZero);
+        for (int l = P.lc - 1; l >= P.l0; --l) yc_smooth(P, l, P.nu2, true, kFromCoarse);
+    }
+    for (int t = threadIdx.x; t < n0; t += kYcThreads) P.u[t] = T.u[t];
+}
+
 // r.z of the level-0 preconditioner application and the CG beta (the part of k_up's
 // level-0 epilogue the y-line cycle needs).
 __global__ void __launch_bounds__(256) k_rz(const double* r, const double* z, size_t n, State* st,
@@ -2130,6 +2354,8 @@ struct lica_mg {
     bool yline = false;  // y-line zebra relaxation on every level (lica_mg_options.smoother = 1)
     double *ycp = nullptr, *ydp = nullptr;  // k_yline_half's Thomas scratch (level-0 size), where it is used
     double* ylines = nullptr;               // the levels' yc, yd, yi
+    int ylc = 0;                            // k_yline_coarse's first level, or 0
+    size_t ylc_smem = 0;
     std::vector<LevelBuf> lv;  // outer levels then inner levels
     size_t cta_smem = 0;
     CtaParams cp{};
@@ -2492,8 +2718,51 @@ int yl_dense(lica_mg* m, cudaStream_t s) {
     return LICA_OK;
 }
 
+// The levels of k_yline_coarse: the first that fits with all below it.
+size_t yl_coarse_layout(const lica_mg* m, int l0, YlCoarse* P) {
+    size_t off = 0, own = 0;
+    for (int l = l0; l <= m->bottom; ++l) {
+        const LevelBuf& L = m->lv[l];
+        if (P) {
+            P->lv[l].nx = L.nx;
+            P->lv[l].ny = L.ny;
+            P->lv[l].off = (unsigned)off;
+            P->lv[l].ax = L.ax64;
+            P->lv[l].ay = L.ay64;
+            P->lv[l].yc = L.yc;
+            P->lv[l].yd = L.yd;
+            P->lv[l].yi = L.yi;
+        }
+        off += yl_level_doubles(L.nx, L.ny);
+        own = std::max(own, (size_t)(L.nx / 2) * L.ny);
+    }
+    if (P) {
+        P->off_rhs = (unsigned)off;
+        P->off_e = (unsigned)(off + own);
+    }
+    return sizeof(double) * (off + 2 * own);
+}
+
+int yl_coarse(lica_mg* m, cudaStream_t s) {
+    YlCoarse P{};
+    P.l0 = m->ylc;
+    P.lc = m->nouter - 1;
+    P.bottom = m->bottom;
+    P.ncoarse = m->o.ncoarse;
+    P.nu1 = m->o.nu1;
+    P.nu2 = m->o.nu2;
+    P.f = (const double*)m->lv[m->ylc].f;
+    P.u = (double*)m->lv[m->ylc].u;
+    P.lu = m->dense_lu;
+    yl_coarse_layout(m, m->ylc, &P);
+    LICA_CUDA_TRY(launch_next(k_yline_coarse, 1, kYcThreads, m->ylc_smem, s, P));
+    lica_count_launches(1);
+    return LICA_OK;
+}
+
 int yl_inner(lica_mg* m, int l, int from, cudaStream_t s) {
     if (l == m->bottom) return yl_dense(m, s);
+    if (l == m->ylc && l > m->nouter - 1) return yl_coarse(m, s);
     double* u = (double*)m->lv[l].u;
     const double* f = (const double*)m->lv[l].f;
     int st;
@@ -2506,11 +2775,13 @@ int yl_inner(lica_mg* m, int l, int from, cudaStream_t s) {
 
 int vcycle_yline(lica_mg* m, cudaStream_t s) {
     const int lc = m->nouter - 1;
+    const bool one = m->ylc && m->ylc <= lc;   // from there down in one CTA
+    const int last = one ? m->ylc : lc;
     int st;
     if (!m->lv[0].yc) LICA_CUDA_TRY(cudaMemsetAsync(m->z, 0, sizeof(double) * (size_t)m->nx * m->ny, s));
     {
         ProfScope ps(m, LICA_MG_DOWN, s);
-        for (int l = 0; l < lc; ++l) {
+        for (int l = 0; l < last; ++l) {
             double* u = l == 0 ? (double*)m->z : (double*)m->lv[l].u;
             const double* f = l == 0 ? (const double*)m->r : (const double*)m->lv[l].f;
             if ((st = yl_smooth(m, l, u, f, m->o.nu1, false, kFromZero, s)) || (st = yl_restrict(m, l, u, f, s))) return st;
@@ -2519,7 +2790,9 @@ int vcycle_yline(lica_mg* m, cudaStream_t s) {
     {
         ProfScope ps(m, LICA_MG_CTA, s);
         if (lc == 0) return LICA_BAD_ARG;
-        if (lc == m->bottom) {
+        if (one) {
+            if ((st = yl_coarse(m, s))) return st;
+        } else if (lc == m->bottom) {
             if ((st = yl_dense(m, s))) return st;
         } else {
             for (int c = 0; c < m->o.ncoarse; ++c)
@@ -2528,7 +2801,7 @@ int vcycle_yline(lica_mg* m, cudaStream_t s) {
     }
     {
         ProfScope ps(m, LICA_MG_UP, s);
-        for (int l = lc - 1; l >= 0; --l) {
+        for (int l = last - 1; l >= 0; --l) {
             double* u = l == 0 ? (double*)m->z : (double*)m->lv[l].u;
             const double* f = l == 0 ? (const double*)m->r : (const double*)m->lv[l].f;
             if ((st = yl_prolong(m, l, u, s)) || (st = yl_smooth(m, l, u, f, m->o.nu2, true, kFromCoarse, s))) return st;
@@ -3080,6 +3353,18 @@ int lica_mg_create(lica_mg** out, int32_t nx, int32_t ny, double hx, double hy, 
                 }
                 lines += n;
             }
+        }
+        for (int l = m->bottom - 1; l >= 1; --l) {
+            const LevelBuf& L = m->lv[l];
+            const size_t bytes = yl_coarse_layout(m, l, nullptr);
+            if (!L.yc || L.nx > kYcThreads || L.nx * L.ny > kYcCells || bytes > std::min(kYcSmem, (size_t)most)) break;
+            m->ylc = l;
+            m->ylc_smem = bytes;
+        }
+        if (m->ylc &&
+            cudaFuncSetAttribute(k_yline_coarse, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kYcSmem) != cudaSuccess) {
+            lica_set_last_error("cudaFuncSetAttribute(k_yline_coarse)", "failed", __FILE__, __LINE__);
+            return fail(LICA_ERR_CUDA);
         }
         if (!m->lv[0].yc) {
             TRY_ALLOC(m->ycp, sizeof(double) * n0);

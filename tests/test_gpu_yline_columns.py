@@ -53,3 +53,20 @@ def test_yline_start_of_smoothing(nx, ny, nu):
         mg.precond(z, t(f), t(bx), t(by))
     mg.close()
     np.testing.assert_array_equal(z.cpu().numpy(), ref)
+
+
+# where the levels of the one-CTA kernel begin: above the coarsest outer level, at it, inside the inner
+# cycle (its coarsest outer level too large), and odd row counts below it
+@pytest.mark.parametrize("nx,ny,nlevels,ncoarse", [(128, 64, 5, 2), (64, 64, 2, 1), (96, 128, 2, 2), (32, 160, 4, 1)])
+def test_yline_coarse_levels(nx, ny, nlevels, ncoarse):
+    import torch
+    from lica_boiling1d_b200 import poisson as PP
+    rng = np.random.default_rng(nx * ny + nlevels)
+    bx, by, f = rng.uniform(0.1, 40.0, (ny, nx)), rng.uniform(0.1, 40.0, (ny + 1, nx)), rng.standard_normal((ny, nx))
+    ref = O.mg_precond(f, bx, by, 1.0 / nx, 0.2 / ny, nlevels=nlevels, ncoarse=ncoarse, sym=13)
+    mg = PP.MultigridPoisson(nx, ny, 1.0 / nx, 0.2 / ny, nlevels=nlevels, ncoarse=ncoarse, smoother="yline")
+    t = lambda a: torch.from_numpy(np.ascontiguousarray(a)).cuda()  # noqa: E731
+    z = torch.empty((ny, nx), dtype=torch.float64, device="cuda")
+    mg.precond(z, t(f), t(bx), t(by))
+    mg.close()
+    np.testing.assert_array_equal(z.cpu().numpy(), ref)
