@@ -783,7 +783,10 @@ constexpr size_t xupdate_smem() { return sizeof(double) * 5 * PAREA; }
 //
 // Every level is stored colour-split: cell (i, j) of colour c = (i + j) & 1 sits in X_c at
 // [j * half + (i >> 1)], half = nx / 2, for X = u, f, ax (west faces), ay (south faces,
-// rows 0..ny) and 1/d.  A red (black) half-sweep then reads and writes consecutive words
+// rows 0..ny) and 1/d.  Where nx is odd, which only the bottom level can be (coarsening ends there),
+// half = (nx + 1) / 2: every cell then has an entry of its own, one colour's last entry of a row being
+// unused; only the restriction, the prolongation and the dense solve touch that level.
+// A red (black) half-sweep then reads and writes consecutive words
 // across a warp, and the four children of coarse cell (I, J) are the entries I of rows
 // 2J and 2J+1 of both colours.  u has a zero ghost row below row 0 and above row ny-1,
 // so the wall neighbours need no branch.  Work items are walked with an incremental
@@ -800,7 +803,7 @@ struct CtaParams {
     int lcta, lc, bottom;
     int nu1, nu2, ncoarse;
     unsigned off_dense, off_rhs;
-    const void* image; // the weights of every level and the bottom elimination as they lie in shared memory,
+    const void* image; // the weights of every level but the bottom, and its elimination, as they lie in shared memory,
     unsigned image_bytes;  // from its start (k_cta_image)
     const void* f_in;  // f of level lcta (T)
     void* u_out;       // u of level lcta (T)
@@ -1198,7 +1201,7 @@ __device__ __forceinline__ void zero_ghosts(const CtaParams& P, unsigned char* s
     }
 }
 
-// The weights of every level lie in global memory as they do in shared memory (k_cta_image, once
+// The weights of the swept levels lie in global memory as they do in shared memory (k_cta_image, once
 // per solve), so staging them is one bulk copy under an mbarrier while the threads stage f: as
 // element copies of each level's arrays it took 7.2 k of a V-cycle's 43 k cycles on one SM.
 // With the sweeps' weights in registers, groups of warps as wide as their level, one copy of the
@@ -1288,7 +1291,8 @@ __global__ void __launch_bounds__(NT_CTA, 1) k_cta(const __grid_constant__ CtaPa
     }
 }
 
-// The weights of level l (row-major AX, AY, DINV) into the image at the level's offsets.
+// The weights of level l (row-major AX, AY, DINV; above the bottom, so L.half = nx / 2) into the image
+// at the level's offsets.
 template <typename E>
 __global__ void k_cta_image(const E* ax, const E* ay, const E* di, unsigned char* __restrict__ image,
                             const CtaLevel L) {
@@ -1418,7 +1422,7 @@ __global__ void __launch_bounds__(NT_CTA, 1) k_small_solve(const __grid_constant
         }
     }
     __syncthreads();
-    for (int l = 0; l <= P.bottom; ++l) {
+    for (int l = 0; l < P.bottom; ++l) {   // the bottom is not swept
         const SL<double> S = make_sl<double>(P.lv, sm, l);
         for (int q = t; q < S.nx * S.ny; q += NT_CTA) {
             const int c = q >= S.ny * S.h, k = q - c * S.ny * S.h, j = k / S.h, m = k - j * S.h, o = (j + c) & 1;
@@ -2875,7 +2879,7 @@ int setup_beta(lica_mg* m, const double* bx, const double* by, cudaStream_t s) {
     }
     // the single-CTA kernel's weights as it holds them (the y-line cycle has none)
     if (!m->yline)
-        for (int l = m->lcta; l <= m->bottom; ++l) {
+        for (int l = m->lcta; l < m->bottom; ++l) {
             const LevelBuf& L = m->lv[l];
             const int blocks = blocks_for((size_t)L.nx * (L.ny + 1));
             if (l < m->nouter - 1 && is_mixed(m))
@@ -3224,11 +3228,12 @@ int lica_mg_create(lica_mg** out, int32_t nx, int32_t ny, double hx, double hy, 
     const size_t tsz = mixed ? sizeof(float) : sizeof(double);
     // single-CTA levels: from the first level >= 1 whose remaining hierarchy fits in
     // shared memory and has <= 32*32 cells, or that cannot be tiled
-    // per level: u (two colours, each (ny+2) x nx/2 with zero ghost rows), f, ax, 1/d
-    // (ny x nx/2 each) and ay ((ny+1) x nx/2), 16-byte aligned arrays
+    // per level: u (two colours, each (ny+2) x half with zero ghost rows), f, ax, 1/d
+    // (ny x half each) and ay ((ny+1) x half), 16-byte aligned arrays; the bottom level's weights
+    // only where its elimination is made from them (k_small_solve: factor)
     auto level_arrays = [&](int l, CtaLevel& C, auto&& take, bool weights) {
         const size_t e = (l < m->nouter - 1) ? tsz : sizeof(double);
-        const size_t h = (size_t)m->lv[l].nx / 2, ny = m->lv[l].ny;
+        const size_t h = ((size_t)m->lv[l].nx + 1) / 2, ny = m->lv[l].ny;
         for (int c = 0; c < 2; ++c) {
             if (weights) {
                 C.off_ax[c] = take(e * ny * h);
@@ -3240,12 +3245,12 @@ int lica_mg_create(lica_mg** out, int32_t nx, int32_t ny, double hx, double hy, 
             }
         }
     };
-    auto cta_bytes = [&](int from) {
+    auto cta_bytes = [&](int from, bool factor) {
         size_t off = 0;
         auto take = [&](size_t bytes) { size_t r = off; off = (off + bytes + 15) & ~(size_t)15; return (unsigned)r; };
         CtaLevel C{};
         for (int l = from; l <= m->bottom; ++l) {
-            level_arrays(l, C, take, true);
+            if (l < m->bottom || factor) level_arrays(l, C, take, true);
             level_arrays(l, C, take, false);
         }
         const size_t nb = (size_t)m->lv[m->bottom].nx * m->lv[m->bottom].ny;
@@ -3257,9 +3262,9 @@ int lica_mg_create(lica_mg** out, int32_t nx, int32_t ny, double hx, double hy, 
     for (int l = 1; l < m->nouter; ++l) {
         const bool tileable = m->lv[l].nx % 16 == 0 && m->lv[l].ny % 16 == 0;
         const size_t n = (size_t)m->lv[l].nx * m->lv[l].ny;
-        if (!tileable || (n <= 32 * 32 && cta_bytes(l) <= 226 * 1024)) { lcta = l; break; }
+        if (!tileable || (n <= 32 * 32 && cta_bytes(l, false) <= 226 * 1024)) { lcta = l; break; }
     }
-    if (cta_bytes(lcta) > 227 * 1024) {
+    if (cta_bytes(lcta, false) > 227 * 1024) {
         delete m;
         lica_set_last_error("lica_mg_create", "coarse levels do not fit in shared memory; use more levels",
                             __FILE__, __LINE__);
@@ -3277,22 +3282,22 @@ int lica_mg_create(lica_mg** out, int32_t nx, int32_t ny, double hx, double hy, 
         m->yline = o.smoother == 1;
     }
     // shared-memory layout of the single-CTA kernels, from their first level
-    auto cta_layout = [&](CtaParams& P, int from) {
+    auto cta_layout = [&](CtaParams& P, int from, bool factor) {
         std::memset(&P, 0, sizeof(P));
         P.lcta = from; P.lc = m->nouter - 1; P.bottom = m->bottom;
         P.nu1 = o.nu1; P.nu2 = o.nu2; P.ncoarse = o.ncoarse;
         size_t off = 0;
         auto take = [&](size_t bytes) { size_t r = off; off = (off + bytes + 15) & ~(size_t)15; return (unsigned)r; };
         const size_t nb = (size_t)m->lv[m->bottom].nx * m->lv[m->bottom].ny;
-        // the image first: every level's weights and the bottom elimination
-        for (int l = from; l <= m->bottom; ++l) level_arrays(l, P.lv[l], take, true);
+        // the image first: the swept levels' weights and the bottom elimination
+        for (int l = from; l < m->bottom + (factor ? 1 : 0); ++l) level_arrays(l, P.lv[l], take, true);
         P.off_dense = take(sizeof(double) * nb * nb);
         P.image_bytes = (unsigned)off;
         int warps = NT_CTA / 32;
         for (int l = from; l <= m->bottom; ++l) {
             CtaLevel& C = P.lv[l];
             level_arrays(l, C, take, false);
-            C.nx = m->lv[l].nx; C.ny = m->lv[l].ny; C.half = m->lv[l].nx / 2;
+            C.nx = m->lv[l].nx; C.ny = m->lv[l].ny; C.half = (m->lv[l].nx + 1) / 2;
             auto mag = [](unsigned c) { return c > 1 ? (unsigned)((1ull << 32) / c + 1) : 0u; };
             C.mag_h = mag((unsigned)C.half);
             C.mag_nx = mag((unsigned)C.nx);
@@ -3303,10 +3308,10 @@ int lica_mg_create(lica_mg** out, int32_t nx, int32_t ny, double hx, double hy, 
         return off;
     };
     CtaParams& P = m->cp;
-    m->cta_smem = cta_layout(P, lcta);
-    if (!mixed && o.smoother == 0 && (size_t)nx * ny <= (size_t)kSmallOwn * NT_CTA && cta_bytes(0) <= 224 * 1024) {
+    m->cta_smem = cta_layout(P, lcta, false);
+    if (!mixed && o.smoother == 0 && (size_t)nx * ny <= (size_t)kSmallOwn * NT_CTA && cta_bytes(0, true) <= 224 * 1024) {
         m->small = true;
-        m->small_smem = cta_layout(m->small_cp, 0);
+        m->small_smem = cta_layout(m->small_cp, 0, true);
     }
 
     auto fail = [&](int code) { lica_mg_destroy(m); return code; };
