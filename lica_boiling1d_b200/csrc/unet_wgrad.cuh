@@ -10,25 +10,32 @@
 // pixels per 32 channels) and three boxes of x of 18 x 8 pixels, one per dx, zero-filled outside
 // the image.  8 pixels of an image row are one swizzle atom, so 16 pixels of the contraction are
 // two atoms, and the three dy are the same box started 0, 1 or 2 atoms further: one MMA of
-// N = 3 * 32 covers them (the operand's N blocks lie one atom apart, as its K blocks do).  The
-// 9 * 32 columns of all taps stay in tensor memory over the CTA's tiles, and each CTA writes
-// one partial sum, added over the CTAs by k_sum_parts in a fixed order.
-//   warp 4: TMA producer; warp 5: MMA issuer (24 instructions of 128 x 96 x 16 a tile);
-//   warps 0-3: the bias gradient from the dz tiles in shared memory (first channel block only),
-//   then the epilogue.
+// N = 3 * 32 covers them (the operand's N blocks lie one atom apart, as its K blocks do).
+// The tensor core does not round its running sum to nearest, so a sum left there over many tiles
+// drifts in proportion to their number: 1.1e-5 of layer 8's weights for 64 images of 64 x 64,
+// 3.6e-4 for 1024, against 2.3e-7 and 3.7e-6 of FP32 sums over 2048 pixels on the CUDA cores.  It
+// therefore holds one tile at a time, an accumulator for each dx, and the epilogue warps add it to
+// running sums in their registers (4.7e-8 and 3.1e-7).  Tensor memory has room for five such
+// accumulators: the next tile waits only for the first of this one to be read.  Each CTA writes one
+// partial sum, added over the CTAs by k_sum_parts in a fixed order.
+//   warps 0-11: four for each dy, a lane for each output channel, 3 * 32 running sums a lane;
+//   warp 12: TMA producer; warp 13: MMA issuer (24 instructions of 128 x 96 x 16 a tile);
+//   warps 14-15: the bias gradient from the dz tiles in shared memory (first channel block only).
 // Fewer than 128 output channels leave rows of D unused: the instruction reads what lies behind
 // the dz boxes for them (other boxes, and kWgBehind bytes kept after the last stage), and they are
 // not written.
-// Bound: the MMAs, 24 x about 90 cycles a tile and channel block (the narrow N and the unused
-// rows cost up to 4x the useful products at 32 channels).  Four images of 256 x 256, all ten
-// layers: CUDA-core sums over 32 x 32 blocks 8.40 ms, 0.29 ms so.
+// Bound: the MMA warp, 24 x 60 cycles of issue and two waits a tile and channel block (the narrow
+// N and the unused rows cost up to 4x the useful products at 32 channels).  Four images of 256 x
+// 256, all ten layers: CUDA-core sums over 32 x 32 blocks 8.40 ms, 0.32 ms so; with the sums left
+// in the tensor core over all tiles 0.29 ms.
 #pragma once
 #include "unet_conv.cuh"
 
 namespace lica {
 namespace unet {
 
-constexpr int kWgThreads = 192;
+constexpr int kWgThreads = 512;
+constexpr int kWgRing = 5;              // accumulators in tensor memory: 5 * 96 columns
 constexpr int kWgMaxStages = 6;
 constexpr int kWgDzBox = kTileM * 64;   // bytes of a dz box: 128 pixels x 32 channels
 constexpr int kWgBehind = 4 * kWgDzBox; // room behind the last stage for the unused rows' reads
@@ -56,22 +63,48 @@ __device__ __forceinline__ uint64_t mn_desc(uint32_t addr, uint32_t row_bytes, u
     return d;
 }
 
+// tc::mbar_wait_warp without the suspend-time hint.  The MMA warp waits twice a tile on barriers that
+// are mostly ready, and a try_wait with the hint takes 700 to 900 cycles even then, 130 without it.
+__device__ __forceinline__ bool wait_warp(uint64_t* bar, uint32_t parity, int lane) {
+    int ok = 1;
+    if (lane == 0) {
+        auto ready = [&] {
+            uint32_t r;
+            asm volatile(
+                "{\n\t.reg .pred p;\n\t"
+                "mbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2;\n\t"
+                "selp.u32 %0, 1, 0, p;\n\t}"
+                : "=r"(r)
+                : "r"(tc::smem_u32(bar)), "r"(parity)
+                : "memory");
+            return r != 0;
+        };
+        if (!ready()) {
+            const uint64_t t0 = tc::global_ns();
+            while (ok && !ready()) ok = tc::global_ns() - t0 <= tc::kWaitNs;
+        }
+    }
+    return __shfl_sync(0xffffffffu, ok, 0) != 0;
+}
+
 __global__ void __launch_bounds__(kWgThreads, 1)
     k_wgrad3x3(const __grid_constant__ CUtensorMap tm_dz, const __grid_constant__ CUtensorMap tm_x0,
                const __grid_constant__ CUtensorMap tm_x1, const WgradParams P) {
     extern __shared__ __align__(16) unsigned char smem_raw[];
     unsigned char* base = reinterpret_cast<unsigned char*>(((uintptr_t)smem_raw + 1023) & ~(uintptr_t)1023);
-    __shared__ uint64_t full[kWgMaxStages], empty[kWgMaxStages], done;
+    __shared__ uint64_t full[kWgMaxStages], empty[kWgMaxStages], sums_full[2], drained, done;
     __shared__ uint32_t tmem_slot;
-    __shared__ float sbias[4][128];
+    __shared__ float sbias[128];
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
     const int NS = P.nstages, nco = P.cout / 32;
     const bool bias = blockIdx.y == 0;
     if (threadIdx.x == 0) {
         for (int s = 0; s < NS; ++s) {
             tc::mbar_init(&full[s], 1);
-            tc::mbar_init(&empty[s], bias ? 5 : 1);   // the MMAs, and the four warps that sum dz
+            tc::mbar_init(&empty[s], bias ? 3 : 1);   // the MMAs, and the two warps that sum dz
         }
+        for (int b = 0; b < 2; ++b) tc::mbar_init(&sums_full[b], 1);
+        tc::mbar_init(&drained, 3 * nco);             // the warps that have output channels
         tc::mbar_init(&done, 1);
         tc::fence_barrier_init();
     }
@@ -86,14 +119,14 @@ __global__ void __launch_bounds__(kWgThreads, 1)
     const int dz_bytes = nco * kWgDzBox, xbox = kHaloRows * row;
     const int ncol = 3 * P.cblk;                       // columns of one dx
 
-    if (warp == 4) {
+    if (warp == 12) {
         int s = 0;
         uint32_t ph = 0;
         const void* tmx = ci0 < P.c0 ? (const void*)&tm_x0 : (const void*)&tm_x1;
         const int cx = ci0 < P.c0 ? ci0 : ci0 - P.c0;
         int g = 0;
         for (int t = blockIdx.x; t < P.tiles; t += gridDim.x, ++g) {
-            if (g >= NS && !tc::mbar_wait_warp(&empty[s], ph ^ 1u, lane)) {
+            if (g >= NS && !wait_warp(&empty[s], ph ^ 1u, lane)) {
                 if (lane == 0) atomicExch(P.err, 1);
                 break;
             }
@@ -112,28 +145,37 @@ __global__ void __launch_bounds__(kWgThreads, 1)
                 ph ^= 1u;
             }
         }
-    } else if (warp == 5) {
+    } else if (warp == 13) {
         // both operands M-/N-major: bits 15 and 16
         const uint32_t idesc = tc::idesc_bf16_f32(128, (uint32_t)ncol) | (1u << 15) | (1u << 16);
         const uint32_t atom = 8u * (uint32_t)row;
         int s = 0;
         uint32_t ph = 0;
-        for (int t = blockIdx.x; t < P.tiles; t += gridDim.x) {
-            if (!tc::mbar_wait_warp(&full[s], ph, lane)) {
-                if (lane == 0) atomicExch(P.err, 1);
-                break;
-            }
+        bool ok = true;
+        int slot = 0;     // the tile's first accumulator
+        for (int t = blockIdx.x, i = 0; t < P.tiles; t += gridDim.x, ++i) {
+            // the third accumulator was the first of the tile before; the others' last contents were
+            // read by the same warps before that
+            ok = wait_warp(&full[s], ph, lane) && (i == 0 || wait_warp(&drained, (unsigned)(i - 1) & 1u, lane));
+            if (!ok) break;
+            tc::tc_fence_after();
             const uint32_t st = tc::smem_u32(base + s * P.stage);
             const uint64_t a0 = mn_desc(st, 64, (uint32_t)kWgDzBox, 512);
             const uint64_t b0 = mn_desc(st + (uint32_t)dz_bytes, (uint32_t)row, atom, atom);
+            uint32_t acc[3];
+#pragma unroll
+            for (int dx = 0; dx < 3; ++dx) {
+                acc[dx] = tmem + (uint32_t)(slot * ncol);
+                slot = slot + 1 == kWgRing ? 0 : slot + 1;
+            }
             if (tc::elect_one()) {
 #pragma unroll 1
                 for (int k = 0; k < kTileM / 16; ++k)
 #pragma unroll
                     for (int dx = 0; dx < 3; ++dx)
-                        tc::mma_bf16(tmem + (uint32_t)(dx * ncol), a0 + (uint32_t)(k * 1024 / 16),
-                                     b0 + (uint32_t)(dx * xbox) / 16u + (uint32_t)k * (2u * atom / 16u), idesc,
-                                     t != (int)blockIdx.x || k != 0);
+                        tc::mma_bf16(acc[dx], a0 + (uint32_t)(k * 1024 / 16),
+                                     b0 + (uint32_t)(dx * xbox) / 16u + (uint32_t)k * (2u * atom / 16u), idesc, k != 0);
+                tc::mma_commit(&sums_full[i & 1]);
                 tc::mma_commit(&empty[s]);
             }
             __syncwarp();
@@ -144,37 +186,45 @@ __global__ void __launch_bounds__(kWgThreads, 1)
         }
         if (tc::elect_one()) tc::mma_commit(&done);
         __syncwarp();
-    } else {
+        if (!wait_warp(&done, 0, lane) || !ok)
+            if (lane == 0) atomicExch(P.err, 1);
+    } else if (warp >= 14) {
         if (bias) {
-            // thread = 8 channels (one 16-byte chunk of 4) of every 32-channel box, pixels p, p + 32, ...
+            // lane = 8 channels (one 16-byte chunk of 4) of every 32-channel box, pixels p, p + 8, ... of the
+            // warp's half of the tile, whose sum is formed by itself, then added
             float acc[4][8];
 #pragma unroll
             for (int b = 0; b < 4; ++b)
 #pragma unroll
                 for (int q = 0; q < 8; ++q) acc[b][q] = 0.f;
-            const int chunk = threadIdx.x & 3, p0 = threadIdx.x >> 2;
+            const int chunk = lane & 3, p0 = (warp - 14) * (kTileM / 2) + (lane >> 2);
             int s = 0;
             uint32_t ph = 0;
             for (int t = blockIdx.x; t < P.tiles; t += gridDim.x) {
-                if (!tc::mbar_wait_warp(&full[s], ph, lane)) {
+                if (!wait_warp(&full[s], ph, lane)) {
                     if (lane == 0) atomicExch(P.err, 1);
                     break;
                 }
                 const unsigned char* st = base + s * P.stage;
 #pragma unroll
                 for (int b = 0; b < 4; ++b)
-                    if (b < nco)
-                        for (int p = p0; p < kTileM; p += 32) {
+                    if (b < nco) {
+                        float v[8] = {0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f};
+#pragma unroll 4
+                        for (int p = p0; p < p0 + kTileM / 2; p += 8) {
                             // the 64-byte swizzle: address bits 4-5 exclusive-or bits 7-8
-                            const uint4 v = *reinterpret_cast<const uint4*>(st + b * kWgDzBox + p * 64 +
+                            const uint4 w = *reinterpret_cast<const uint4*>(st + b * kWgDzBox + p * 64 +
                                                                             ((chunk ^ ((p >> 1) & 3)) << 4));
-                            const uint32_t u[4] = {v.x, v.y, v.z, v.w};
+                            const uint32_t u[4] = {w.x, w.y, w.z, w.w};
 #pragma unroll
                             for (int q = 0; q < 4; ++q) {
-                                acc[b][2 * q] += __uint_as_float(u[q] << 16);
-                                acc[b][2 * q + 1] += __uint_as_float(u[q] & 0xffff0000u);
+                                v[2 * q] += __uint_as_float(u[q] << 16);
+                                v[2 * q + 1] += __uint_as_float(u[q] & 0xffff0000u);
                             }
                         }
+#pragma unroll
+                        for (int q = 0; q < 8; ++q) acc[b][q] += v[q];
+                    }
                 __syncwarp();
                 if (lane == 0) tc::mbar_arrive(&empty[s]);
                 if (++s == NS) {
@@ -182,42 +232,75 @@ __global__ void __launch_bounds__(kWgThreads, 1)
                     ph ^= 1u;
                 }
             }
-            // over the 8 pixels groups of a warp (lanes of one chunk are 4 apart), then the warps
+            // over the 8 pixel groups (lanes of one chunk are 4 apart), then the two halves
 #pragma unroll
             for (int b = 0; b < 4; ++b)
                 if (b < nco)
 #pragma unroll
-                    for (int q = 0; q < 8; ++q) {
-                        float v = acc[b][q];
-                        for (int o = 16; o >= 4; o >>= 1) v += __shfl_xor_sync(0xffffffffu, v, o);
-                        if (lane < 4) sbias[warp][32 * b + 8 * chunk + q] = v;
-                    }
-            asm volatile("bar.sync 1, 128;" ::: "memory");
-            if ((int)threadIdx.x < P.cout)
-                P.bpart[(size_t)blockIdx.x * P.cout + threadIdx.x] =
-                    (sbias[0][threadIdx.x] + sbias[1][threadIdx.x]) + (sbias[2][threadIdx.x] + sbias[3][threadIdx.x]);
-        }
-        if (!tc::mbar_wait_warp(&done, 0, lane)) {
-            if (lane == 0) atomicExch(P.err, 1);
-        } else if (32 * warp < P.cout) {
-            tc::tc_fence_after();
-            const int co = 32 * warp + lane;
-            float* dst = P.part + ((size_t)blockIdx.x * P.cout + co) * 9 * P.ctot + ci0;
-            const uint32_t taddr = tmem + ((uint32_t)(32 * warp) << 16);
-            for (int dx = 0; dx < 3; ++dx)
-                for (int dy = 0; dy < 3; ++dy) {
-                    float* d = dst + (3 * dy + dx) * P.ctot;
-                    for (int c = 0; c < P.cblk; c += 16) {
-                        float v[16];
-                        tc::tmem_ld16(taddr + (uint32_t)(dx * ncol + dy * P.cblk + c), v);
+                    for (int q = 0; q < 8; ++q)
+                        for (int o = 16; o >= 4; o >>= 1) acc[b][q] += __shfl_xor_sync(0xffffffffu, acc[b][q], o);
+            if (warp == 15 && lane < 4)
 #pragma unroll
-                        for (int q = 0; q < 4; ++q)
-                            *reinterpret_cast<float4*>(d + c + 4 * q) =
-                                make_float4(v[4 * q], v[4 * q + 1], v[4 * q + 2], v[4 * q + 3]);
-                    }
-                }
+                for (int b = 0; b < 4; ++b)
+#pragma unroll
+                    for (int q = 0; q < 8; ++q) sbias[32 * b + 8 * chunk + q] = acc[b][q];
+            asm volatile("bar.sync 1, 64;" ::: "memory");
+            if (warp == 14 && lane < 4)
+#pragma unroll
+                for (int b = 0; b < 4; ++b)
+                    if (b < nco)
+#pragma unroll
+                        for (int q = 0; q < 8; ++q) {
+                            const int c = 32 * b + 8 * chunk + q;
+                            P.bpart[(size_t)blockIdx.x * P.cout + c] = acc[b][q] + sbias[c];
+                        }
         }
-        tc::tc_fence_before();
+    } else if (32 * (warp & 3) < P.cout) {
+        const int dy = warp >> 2;
+        const uint32_t taddr = tmem + ((uint32_t)(32 * (warp & 3)) << 16) + (uint32_t)(dy * P.cblk);
+        float acc[3][32];
+#pragma unroll
+        for (int dx = 0; dx < 3; ++dx)
+#pragma unroll
+            for (int q = 0; q < 32; ++q) acc[dx][q] = 0.f;
+        int slot = 0;
+        bool ok = true;
+        for (int t = blockIdx.x, i = 0; t < P.tiles; t += gridDim.x, ++i) {
+            if (!(ok = wait_warp(&sums_full[i & 1], (unsigned)(i >> 1) & 1u, lane))) {
+                if (lane == 0) atomicExch(P.err, 1);
+                break;
+            }
+            tc::tc_fence_after();
+#pragma unroll
+            for (int dx = 0; dx < 3; ++dx) {
+                const uint32_t at = taddr + (uint32_t)(slot * ncol);
+                slot = slot + 1 == kWgRing ? 0 : slot + 1;
+#pragma unroll
+                for (int c = 0; c < 32; c += 16)
+                    if (c < P.cblk) {
+                        float v[16];
+                        tc::tmem_ld16(at + (uint32_t)c, v);
+#pragma unroll
+                        for (int q = 0; q < 16; ++q) acc[dx][c + q] += v[q];
+                    }
+                if (dx == 0) {
+                    tc::tc_fence_before();
+                    __syncwarp();
+                    if (lane == 0) tc::mbar_arrive(&drained);
+                }
+            }
+        }
+        if (ok) {
+            const int co = 32 * (warp & 3) + lane;
+            float* dst = P.part + ((size_t)blockIdx.x * P.cout + co) * 9 * P.ctot + ci0;
+#pragma unroll
+            for (int dx = 0; dx < 3; ++dx)
+#pragma unroll
+                for (int q = 0; q < 32; q += 4)
+                    if (q < P.cblk)
+                        *reinterpret_cast<float4*>(dst + (3 * dy + dx) * P.ctot + q) =
+                            make_float4(acc[dx][q], acc[dx][q + 1], acc[dx][q + 2], acc[dx][q + 3]);
+        }
     }
     __syncwarp();
     tc::tc_fence_before();
