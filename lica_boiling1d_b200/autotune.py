@@ -8,30 +8,34 @@ per SM, a few long ones wide CTAs that finish each column sooner.
 
 ``tune(batch)`` times one warm-up step and ``trial_steps`` steps of each shape on a copy of
 the batch's device state (the batch itself does not advance), keeps the fastest, and
-caches the choice per GPU and batch shape: in memory, and in a JSON file
+caches the choice per GPU, kernel generation and batch shape: in memory, and in a JSON file
 (``$LICA_TUNE_CACHE``, default ``~/.cache/lica_b200/column_tune.json``) so a later process
-on the same GPU model skips the trial.  ``ColumnBatch.steps(threads=0)`` calls it.
+on the same GPU model skips the trial.  A choice timed on an earlier generation of the step
+kernel is not taken.  ``ColumnBatch.steps(threads=0)`` calls it.
 """
 import json
 import os
 import threading
 
-# (threads, tri_cap): tri_cap has no effect any more; cache entries of the shapes that had one
-# (tri_cap 0) are still read
+# (threads, tri_cap); tri_cap, once -1 or 0, has no effect any more
 SHAPES = ((32, -1), (64, -1), (128, -1), (256, -1))
+# Raised when a change of the step kernel moves the fastest widths.  1: the tridiagonal arrays in
+# shared memory or not, 5 columns of 64 threads per SM (its entries name no generation); 2: all
+# columns through shared memory of a fixed size, 4 of 64 or 2 of 128 threads per SM.
+GENERATION = 2
 
 
 def _name(shape):
-    return f"{shape[0]}/{'smem' if shape[1] < 0 else 'scratch'}"
+    return f"{shape[0]} threads"
 
 
 def _shape(entry):
-    """A cache entry's shape, or None if it is not one of SHAPES."""
+    """A cache entry's shape, or None if its width is none of SHAPES'."""
     try:
         sh = (int(entry["threads"]), int(entry.get("tri_cap", -1)))
     except (KeyError, TypeError, ValueError):
         return None
-    return sh if sh in SHAPES or (sh[0], -1 - sh[1]) in SHAPES else None
+    return sh if sh[0] in {w for w, _ in SHAPES} and sh[1] in (-1, 0) else None
 
 
 _lock = threading.Lock()
@@ -55,6 +59,10 @@ def batch_key(batch):
     n = np.asarray(batch.n)
     q = np.percentile(n, [25, 50, 75]).astype(int).tolist()
     return f"ncol={batch.ncol},cells={int(n.sum())},nmax={int(n.max())},q={q[0]}/{q[1]}/{q[2]}"
+
+
+def cache_key(gpu, batch):
+    return f"{gpu}|kernel={GENERATION}|{batch_key(batch)}"
 
 
 def _load():
@@ -82,7 +90,7 @@ def tune(batch, trial_steps=2, force=False):
     ms per step} of the trial, or None when the choice came from the cache)."""
     import torch
     dev = batch.arrays["w"].device
-    key = f"{_gpu_name(dev)}|{batch_key(batch)}"
+    key = cache_key(_gpu_name(dev), batch)
     with _lock:
         if not force:
             if key in _memo:
