@@ -20,6 +20,32 @@ using namespace lica::unet;
 
 namespace {
 
+// Shared-memory limits of the tensor-core kernels, set once for each device (they are the device's),
+// and the SMs of the current one.
+constexpr int kMaxDevices = 64;
+constexpr int kConvSmemMax = 227 * 1024, kWgSmemMax = 220 * 1024;
+cudaError_t device_setup(int& sms) {
+    struct Device {
+        std::once_flag once;
+        cudaError_t err = cudaSuccess;
+        int sms = 1;
+    };
+    static Device devices[kMaxDevices];
+    int dev = 0;
+    const cudaError_t e = cudaGetDevice(&dev);
+    if (e != cudaSuccess) return e;
+    if (dev >= kMaxDevices) return cudaErrorInvalidDevice;
+    Device& d = devices[dev];
+    std::call_once(d.once, [&d, dev] {
+        d.err = cudaFuncSetAttribute(k_conv3x3_tcp, cudaFuncAttributeMaxDynamicSharedMemorySize, kConvSmemMax);
+        if (d.err == cudaSuccess)
+            d.err = cudaFuncSetAttribute(k_wgrad3x3, cudaFuncAttributeMaxDynamicSharedMemorySize, kWgSmemMax);
+        if (d.err == cudaSuccess) d.err = cudaDeviceGetAttribute(&d.sms, cudaDevAttrMultiProcessorCount, dev);
+    });
+    sms = d.sms;
+    return d.err;
+}
+
 PFN_cuTensorMapEncodeTiled_v12000 encode_fn() {
     static PFN_cuTensorMapEncodeTiled_v12000 fn = nullptr;
     static std::once_flag once;
@@ -90,8 +116,6 @@ int tmem_columns(int cout) {
 
 bool aligned16(const void* p) { return ((uintptr_t)p & 15u) == 0; }
 
-constexpr int kConvSmemMax = 227 * 1024;
-
 }  // namespace
 
 namespace lica {
@@ -128,16 +152,8 @@ int conv3x3(const __nv_bfloat16* x0, int c0, const __nv_bfloat16* x1, int c1, co
                             __LINE__);
         return LICA_BAD_ARG;
     }
-    static std::once_flag attr_once;
-    static cudaError_t attr_err = cudaSuccess;
-    static int num_sms = 148;
-    std::call_once(attr_once, [] {
-        attr_err = cudaFuncSetAttribute(k_conv3x3_tcp, cudaFuncAttributeMaxDynamicSharedMemorySize, kConvSmemMax);
-        int dev = 0;
-        if (attr_err == cudaSuccess) attr_err = cudaGetDevice(&dev);
-        if (attr_err == cudaSuccess) attr_err = cudaDeviceGetAttribute(&num_sms, cudaDevAttrMultiProcessorCount, dev);
-    });
-    LICA_CUDA_TRY(attr_err);
+    int num_sms = 0;
+    LICA_CUDA_TRY(device_setup(num_sms));
     ConvParams P{};
     P.n = n; P.h = h; P.w = wd; P.tw = tw; P.th = th;
     P.nsrc = c1 > 0 ? 2 : 1;
@@ -807,11 +823,11 @@ int forward(lica_unet* u, const double* rho, const double* f, double hsq, double
 
 // CTAs along the pixels for a layer's weight gradient: one per SM over the blocks of input
 // channels, at most one per pixel tile.
-int wgrad_chunks(const lica_unet* u, int l) {
+int wgrad_chunks(const lica_unet* u, int l, int sms) {
     const LayerDef& L = kNet[l];
     const int blocks = (L.cin0 + L.cin1) / (L.cin0 % 32 ? 16 : 32);
     const int tiles = (int)(level_pixels(u, L.level) / kTileM);
-    return std::max(1, std::min(tiles, 148 / blocks));
+    return std::max(1, std::min(tiles, sms / blocks));
 }
 
 int alloc_training(lica_unet* u) {
@@ -831,9 +847,11 @@ int alloc_training(lica_unet* u) {
     if ((st = dev_alloc(&u->gcat1, p1 * 192))) return st;
     // weight-gradient partials: the largest layer's chunks x weights
     size_t pe = 0, be = 0;
+    int sms = 0;
+    LICA_CUDA_TRY(device_setup(sms));
     for (int l = 0; l < kLayers; ++l) {
         const LayerDef& L = kNet[l];
-        const size_t chunks = (size_t)wgrad_chunks(u, l);
+        const size_t chunks = (size_t)wgrad_chunks(u, l, sms);
         pe = std::max(pe, chunks * L.cout * 9 * (L.cin0 + L.cin1));
         be = std::max(be, chunks * L.cout);
     }
@@ -849,13 +867,6 @@ int alloc_training(lica_unet* u) {
 int layer_wgrad(lica_unet* u, int l, const bf16* x0, const bf16* x1, cudaStream_t s) {
     const LayerDef& L = kNet[l];
     const int H = u->h >> L.level, W = u->w >> L.level, ctot = L.cin0 + L.cin1;
-    static std::once_flag attr_once;
-    static cudaError_t attr_err = cudaSuccess;
-    constexpr int kSmem = 220 * 1024;
-    std::call_once(attr_once, [] {
-        attr_err = cudaFuncSetAttribute(k_wgrad3x3, cudaFuncAttributeMaxDynamicSharedMemorySize, kSmem);
-    });
-    LICA_CUDA_TRY(attr_err);
     WgradParams P{};
     P.h = H;
     P.w = W;
@@ -865,7 +876,7 @@ int layer_wgrad(lica_unet* u, int l, const bf16* x0, const bf16* x1, cudaStream_
     P.cblk = L.cin0 % 32 ? 16 : 32;
     P.c0 = L.cin0;
     P.stage = (L.cout / 32) * kWgDzBox + (3 * kHaloRows * 2 * P.cblk + 1023) / 1024 * 1024;
-    P.nstages = std::min(kWgMaxStages, (kSmem - 1024 - kWgBehind) / P.stage);
+    P.nstages = std::min(kWgMaxStages, (kWgSmemMax - 1024 - kWgBehind) / P.stage);
     P.part = u->part;
     P.bpart = u->bpart;
     P.err = u->err;
@@ -875,7 +886,9 @@ int layer_wgrad(lica_unet* u, int l, const bf16* x0, const bf16* x1, cudaStream_
     if ((st = act_map(&m0, x0, L.cin0, W, H, u->n, P.cblk, kTileW, kTileH + 2))) return st;
     m1 = m0;
     if (L.cin1 && (st = act_map(&m1, x1, L.cin1, W, H, u->n, P.cblk, kTileW, kTileH + 2))) return st;
-    const int chunks = wgrad_chunks(u, l);
+    int sms = 0;
+    LICA_CUDA_TRY(device_setup(sms));
+    const int chunks = wgrad_chunks(u, l, sms);
     LICA_CUDA_TRY(launch_next(k_wgrad3x3, dim3(chunks, ctot / P.cblk), kWgThreads, 1024 + P.nstages * P.stage + kWgBehind, s,
                               mdz, m0, m1, P));
     lica_count_launches(1);
