@@ -1,11 +1,10 @@
 // Correctly rounded FP64 reciprocals, quotients and square roots without a branch.
 //
-// `a / b`, `1.0 / b` and `sqrt` carry a test for extreme operands and a call behind it, so two
-// independent divisions of one thread do not overlap: measured on a B200, 64 cycles for 1/b,
-// 115 for a/b, and 123 for two independent 1/b.  These forms are straight-line FMA chains
-// that do overlap, and the test for extreme operands (`ordinary`) is apart, to be made once
-// for a group of divisions; where it fails the caller takes the plain operator.  The results
-// are the IEEE quotients bit for bit.
+// Two independent divisions of one thread do not overlap when they are written with the
+// operators: measured on a B200, 64 cycles for 1/b, 115 for a/b, and 123 for two independent 1/b.
+// These forms are straight-line FMA chains that do overlap, and the test for extreme operands
+// (`ordinary`) is apart, to be made once for a group of divisions; where it fails the caller
+// takes the plain operator.  The results are the IEEE quotients bit for bit.
 //
 // Method: the reciprocal by a cubic step from the hardware's 20-bit seed, to within a unit
 // in the last place, then Markstein's correction, whose result is the correctly rounded 1/b
@@ -50,7 +49,8 @@ __device__ __forceinline__ double quot(double a, double b, double y) {
     return __fma_rn(__fma_rn(-b, q, a), y, q);
 }
 
-// sqrt(x), x ordinary; ok is cleared where the result is not the correctly rounded root
+// sqrt(x), x in range (the test of the rounding needs nothing of the mantissa); ok is cleared where
+// the result is not the correctly rounded root
 __device__ __forceinline__ double root(double x, bool& ok) {
     double y;
     asm("rsqrt.approx.ftz.f64 %0, %1;" : "=d"(y) : "d"(x));
