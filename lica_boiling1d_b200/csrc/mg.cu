@@ -1311,8 +1311,8 @@ __global__ void k_cta_image(const E* ax, const E* ay, const E* di, unsigned char
 // ------------------------------------------------------------------------------------
 // Whole solves of small systems (FP64, red-black smoothing): level 0 and its hierarchy in one
 // CTA's shared memory, the CG vectors in registers, set-up, V-cycles and CG in one launch.  Such
-// a solve is launches and gaps otherwise: 64 x 64 cells took 588 us as 17 set-up launches and 12
-// rounds of 5 kernels, most of them a few blocks; so it takes 430 us.  The V-cycle is the
+// a solve is launches and gaps otherwise: 64 x 64 cells took 637 us as 17 set-up launches and 12
+// rounds of 5 kernels, most of them a few blocks; so it takes 471 us.  The V-cycle is the
 // single-CTA kernel's (s_outer from level 0), bit-identical to the grid kernels'; the sums of the
 // CG are added in this CTA's order.  The rule: the hierarchy fits a CTA's shared memory, and
 // level 0 has at most kSmallOwn cells a thread (4096 cells, 213 KB).
@@ -1822,7 +1822,7 @@ constexpr int kYlArrays = 7;
 // What a half-sweep's neighbours hold: u, zero, or u + P uc.  A half-sweep reads its neighbours alone and
 // writes its own columns in full, and so does the next one, so the first of a smoothing can take the
 // iterate from zero or from the coarse correction without either being stored: no launch that adds
-// the correction, no clearing (256 x 256 cells: a solve 11.27 -> 10.98 ms).
+// the correction or clears (256 x 256 cells: a solve 11.27 -> 10.98 ms).
 constexpr int kFromIterate = 0, kFromZero = 1, kFromCoarse = 2;
 __host__ __device__ inline int yl_pitch(int ny) { return (ny + 7) & ~7; }
 __global__ void __launch_bounds__(kYlThreads)
@@ -2003,7 +2003,7 @@ __global__ void __launch_bounds__(kYlThreads)
 
 // Residual r = f - (s - d u) of the four children of coarse cell (I, J) and their 2x2
 // average, fc = (r00 + r01) + (r10 + r11) times 1/4 in the oracle's order; the coarse iterate
-// starts from zero.
+// starts from zero, stored for levels that k_yline_half sweeps (the others start from kFromZero).
 __global__ void k_resid_restrict(const double* u, const double* f, const double* __restrict__ ax,
                                  const double* __restrict__ ay, double* __restrict__ fc, double* __restrict__ uc, int nx,
                                  int ny) {
